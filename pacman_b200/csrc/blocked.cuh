@@ -436,20 +436,20 @@ struct CholWaveCache {             // one wave of the large-patch engine
 };
 struct SmallRange {                // one launch of the register kernel
   size_t first = 0;                // offset into the cached patch list
-  int count = 0, nmax = 0;
+  int count = 0, nclass = 0;       // patches and their size class
   size_t fac_off = 0;              // offset (doubles) of its factors
 };
 struct FactorCache {
   int basis = -1;
   std::vector<CholWaveCache> waves;
   DevMem small_list;               // patch ids of the small launches
-  DevMem small_fac;                // their L^{-1} blocks and pivots
+  DevMem small_fac;                // their L and U factors
   std::vector<SmallRange> ranges;
   std::vector<int> redo_small, redo_big;  // re-solved by the FP64 LU every execute
   int64_t patches = 0;
 };
-// Bytes of the kept factors of one register-kernel patch of size class N.
-inline size_t small_fac_doubles(int N) { return size_t(N) * N + N; }
+// Doubles of the kept factors of one register-kernel patch of size class N.
+inline size_t small_fac_doubles(int N) { return size_t(N) * N; }
 
 // Forward sweep L y = r from kept factors (an execute that reuses them).
 void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, cudaStream_t st);

@@ -43,15 +43,24 @@ struct PatchArgs {
   int *act_out;           // forward: active axes, K x 3, or null
   const double *h;        // adjoint: weighted upstream gradient per (patch, target)
   double *g_out;          // adjoint: result per (patch, source)
-  // Register kernel (small.cu): 0 factor, 1 factor and store the eliminated
-  // blocks at fac (N * N doubles per list entry), 2 load them instead of
-  // assembling and factoring.
+  // Register kernel (small.cu).  Polynomial block per list entry, from
+  // launch_small_poly: 4 * kMaxF doubles and 8 ints.
+  double *pbeta;
+  int *pact;
+  double *pred;  // their moments, kRedVals doubles
+  // 0 factor, 1 factor and store the factors at fac (N * N doubles per list
+  // entry), 2 load them instead of assembling and factoring.
   double *fac;
   int fac_mode;
 };
 
-// Register-resident Cholesky of the patches with n <= 64 (small.cu); the
-// list must hold patches of one size class (n <= 32 or 32 < n <= 64).
-void launch_small_chol(const PatchArgs &a, const int *plist, int np, int nmax, cudaStream_t st);
+// Register-resident LU of the patches with n <= kSmallMax (small.cu).  The
+// list of launch_small_lu holds patches of one size class N = small_class(n);
+// launch_small_poly must have run on the same list (pbeta, pact, status).
+constexpr int kSmallMax = 64;
+int small_class(int n);
+void launch_small_poly(const PatchArgs &a, const int *plist, int np, bool adj, cudaStream_t st);
+void launch_small_lu(const PatchArgs &a, const int *plist, int np, int N, bool adj,
+                     cudaStream_t st);
 
 }  // namespace pacman_b200

@@ -102,11 +102,11 @@ __device__ inline void gram_from_moments(const double *red, double G[4][4]) {
 // Active polynomial terms of a patch (SerialFillQ's condition loop,
 // serial_ops.hpp:108-139): S[0..pv) are monomial ids (0 = constant, a + 1 =
 // axis a), R is the Cholesky factor of the centred Gram matrix restricted to
-// S.  mn / mx are the coordinate ranges used to pick the axis to drop.
-// Returns 1 if an axis was dropped.
-__device__ inline int poly_axes(const double *red, int dim, const double *shift,
-                                const double *mn, const double *mx, int S[4], int &pv_out,
-                                double R[4][4]) {
+// S.  ranges(mn, mx) gives the coordinate ranges, called only where an axis
+// has to be dropped.  Returns 1 if an axis was dropped.
+template <typename Ranges>
+__device__ inline int poly_axes(const double *red, int dim, const double *shift, Ranges &&ranges,
+                                int S[4], int &pv_out, double R[4][4]) {
   double G[4][4];
   gram_from_moments(red, G);
   bool active[3] = {dim > 0, dim > 1, dim > 2};
@@ -144,6 +144,8 @@ __device__ inline int poly_axes(const double *red, int dim, const double *shift,
     }
     if (!(cond > kCondMax)) break;
     // SerialDeactivateOneAxis (serial_ops.hpp:28-57).
+    double mn[3], mx[3];
+    ranges(mn, mx);
     double best = 1.7976931348623157e308;
     int bi = 0;
     for (int a = 0; a < dim; ++a) {
@@ -167,6 +169,18 @@ __device__ inline int poly_axes(const double *red, int dim, const double *shift,
   return dropped;
 }
 
+// The same with the ranges at hand: mn[0..2], mx[0..2].
+__device__ inline int poly_axes(const double *red, int dim, const double *shift,
+                                const double *mn, const double *mx, int S[4], int &pv_out,
+                                double R[4][4]) {
+  return poly_axes(red, dim, shift, [&](double *lo, double *hi) {
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = mn[d];
+      hi[d] = mx[d];
+    }
+  }, S, pv_out, R);
+}
+
 // Solves (R^T R) x = rhs for the pv active terms.
 __device__ inline void gram_solve(const double R[4][4], int pv, const double *rhs, double *x) {
   double z[4];
@@ -182,18 +196,11 @@ __device__ inline void gram_solve(const double R[4][4], int pv, const double *rh
   }
 }
 
-// Polynomial block of one patch from the reduced moments (one thread).
-// red: moments as above, [10 + 4f + c] = sum q_c b_f, [10+4F .. +6] = min
-// x,y,z, max x,y,z.  Writes beta[4 x F] (uncentred basis, zero for dropped
-// axes), act[0..2] (active axis ids, -1 terminated) and returns the dropped
-// flag.
-__device__ inline int poly_block(const double *red, int F, int dim, const double *shift,
-                                 double *beta, int *act) {
-  const double *mn = red + 10 + 4 * F;
-  const double *mx = mn + 3;
-  int S[4], pv;
-  double R[4][4];
-  const int dropped = poly_axes(red, dim, shift, mn, mx, S, pv, R);
+// Least-squares coefficients for the active terms S with their factor R
+// (uncentred basis, zero for dropped axes) and act[0..2] (active axis ids, -1
+// terminated).
+__device__ inline void poly_fit(const double *red, int F, const double *shift, const int S[4],
+                                int pv, const double R[4][4], double *beta, int *act) {
   int na = 0;
   for (int i = 1; i < pv; ++i) act[na++] = S[i] - 1;
   for (int a = na; a < 3; ++a) act[a] = -1;
@@ -208,6 +215,21 @@ __device__ inline int poly_block(const double *red, int F, int dim, const double
     for (int i = 1; i < pv; ++i) beta[4 * f + i] = bp[i];
     for (int i = pv; i < 4; ++i) beta[4 * f + i] = 0.0;
   }
+}
+
+// Polynomial block of one patch from the reduced moments (one thread).
+// red: moments as above, [10 + 4f + c] = sum q_c b_f, [10+4F .. +6] = min
+// x,y,z, max x,y,z.  Writes beta[4 x F] (uncentred basis, zero for dropped
+// axes), act[0..2] (active axis ids, -1 terminated) and returns the dropped
+// flag.
+__device__ inline int poly_block(const double *red, int F, int dim, const double *shift,
+                                 double *beta, int *act) {
+  const double *mn = red + 10 + 4 * F;
+  const double *mx = mn + 3;
+  int S[4], pv;
+  double R[4][4];
+  const int dropped = poly_axes(red, dim, shift, mn, mx, S, pv, R);
+  poly_fit(red, F, shift, S, pv, R, beta, act);
   return dropped;
 }
 }  // namespace pacman_b200

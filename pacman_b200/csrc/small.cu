@@ -1,389 +1,598 @@
-// Register-resident Cholesky solver for the small patches (n <= 64) of the
-// B200 RBF-PUM transfer, precision "mixed".
+// Register-resident solver for the small patches (n <= 64) of the B200
+// RBF-PUM transfer: both precisions of the forward transfer and the adjoint.
 //
 // Per patch (src/rbf_pum/solver/solver.hpp:180-286): A = phi(|x_i - x_j|),
-// the polynomial block (serial_ops.hpp:108-139) and alpha = A^{-1}(b - Q beta),
-// local = E alpha + V beta.  A team of (N/4)^2 threads holds the N x N matrix
-// (N = 32 or 64, zero padded with an identity block) as 4 x 4 register blocks
-// and eliminates it as L D L^T with the identity carried along (Gauss-Jordan
-// on [A | I]): slot (i, s) holds A[i][s] until pivot s and L^{-1}[i][s]
-// afterwards; one team barrier per pivot.  Then alpha = L^{-T} D^{-1} L^{-1} r
-// by two team reductions.  The polynomial block (moments, condition test,
-// least squares; poly.cuh) runs meanwhile on a separate warp.  For a plan
-// that keeps its factorisations the eliminated blocks are stored after the
-// elimination (fac_mode 1) and later loaded in place of assembly and
-// elimination (fac_mode 2): N * N doubles per patch, thread-block order.
+// the polynomial block (serial_ops.hpp:108-139), alpha = A^{-1}(b - Q beta)
+// by unpivoted LU (the elimination order of the reference, here on the
+// symmetric positive definite A) and local = E alpha + V beta.
+//
+// k_small_moments and k_small_fit do the polynomial block of every listed
+// patch beforehand: a warp sums one patch's moments, then a thread per patch
+// does the condition test and the least squares.
+//
+// k_small_lu is one block of N / 32 warps per patch with one matrix row per
+// thread, in registers.  Pivot p: every thread holds a[i][p]; the column was
+// published to shared memory (a[p][j] = a[j][p] by symmetry), so row i needs
+// only its own multiplier a[i][p] / a[p][p] and broadcast reads of the
+// column.  Column p + 1 is updated and published before the rest of the row,
+// so that the barrier's and the reciprocal's latency overlaps the remaining
+// multiply-adds, and the right-hand sides ride along.  The pivot loop is
+// unrolled by kBlk columns; a finished group of columns (multipliers below
+// the diagonal, U on and above it) goes to shared memory and the row shifts
+// down by kBlk registers, which keeps the code small and every register index
+// static.  U x = y is then solved row-locally with shuffles inside each warp.
+//
+// What bounds it: latency and issue, not the FP64 pipe.  A pivot is a chain
+// of about 300 cycles (column read, reciprocal, multiplier, update, publish,
+// barrier) and a row takes 2 N registers, so 8 to 16 warps share an SM; the
+// FP64 pipe is 34% busy and an instruction issues in 42% of the cycles (ncu,
+// class 48, 4 fields).  Size classes in steps of 8 keep the registers and the
+// unused columns few.  500,000 uniform points, Wendland C4, 4 fields (54,500
+// patches): all small-patch launches 2.1 ms, against 8.6 ms for a 256-thread
+// team per patch on the padded 64 x 64 block with the explicit L^{-1}; 200,000
+// points, C6, 1 field, FP64: 0.77 ms against 4.5 ms for the shared-memory LU.
+#include <type_traits>
+
 #include "patch.cuh"
 
 namespace pacman_b200 {
 
 namespace {
 
-template <int N>
-struct SmallCfg {
-  static constexpr int kG = N / 4;                      // 4 x 4 blocks per side
-  static constexpr int kTeam = kG * kG;                 // threads per patch
-  static constexpr int kTeams = 256 / kTeam;            // patches per CTA
-  static constexpr int kThreads = kTeams * kTeam + 32;  // + the polynomial warp
-  static constexpr int kTPT = N / 16;                   // threads per target (evaluation)
-};
+constexpr int kMomWarps = 4;          // patches per block of k_small_moments
+constexpr int kMomLd = kSmallMax + 1; // column stride: odd, one bank per column
 
-template <int N>
-struct SmallShared {
-  double x[N], y[N], z[N];
-  double b[kMaxF][N];  // values, then the residual r
-  double w[kMaxF][N];  // D^{-1} L^{-1} r, then alpha
-  double cv[2][N];     // the published pivot vector, double buffered
-  double part[N / 4][N];
-  double d[N];         // pivots of L D L^T
+// Moments of the patch's centred monomials (poly.cuh: red layout up to the
+// coordinate ranges), a warp per patch and a lane per value: every value is a
+// sum over the points of a product of two of the columns 1, q_x, q_y, q_z,
+// b_f, in point order.
+__global__ void __launch_bounds__(kMomWarps * 32)
+    k_small_moments(PatchArgs a, const int *__restrict__ plist, int np, int Fm) {
+  __shared__ double tab[kMomWarps][4 + kMaxF][kMomLd];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.x * kMomWarps + warp;
+  if (e >= np) return;
+  const int k = plist[e];
+  const int64_t s0 = a.soff[k];
+  const int n = int(a.soff[k + 1] - s0);
+  const double4 c = a.centers[k];
+  double(*col)[kMomLd] = tab[warp];
+  for (int i = lane; i < n; i += 32) {
+    const int id = a.sidx[s0 + i];
+    const double4 p = a.src[id];
+    col[0][i] = 1.0;
+    col[1][i] = p.x - c.x;
+    col[2][i] = p.y - c.y;
+    col[3][i] = p.z - c.z;
+    for (int f = 0; f < Fm; ++f) col[4 + f][i] = a.vals[int64_t(id) * a.F + f];
+  }
+  __syncwarp();
+  const int nred = 10 + 4 * Fm;
+  for (int id = lane; id < nred; id += 32) {
+    int u = id, v = 0;
+    if (id >= 10) {
+      u = (id - 10) & 3;
+      v = 4 + ((id - 10) >> 2);
+    } else if (id >= 4) {
+      u = id < 7 ? 1 : (id < 9 ? 2 : 3);
+      v = id < 7 ? id - 3 : (id < 9 ? id - 5 : 3);
+    }
+    const double *cu = col[u], *cv = col[v];
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < n; ++i) s = __fma_rn(cu[i], cv[i], s);
+    a.pred[int64_t(e) * kRedVals + id] = s;
+  }
+}
+
+// Polynomial block of a patch per thread: the condition test and the least
+// squares are serial chains of a few thousand dependent FP64 operations, so a
+// warp works on 32 patches side by side.  adj: beta receives the 4 x 4 factor
+// R, act its terms S and their count.
+__global__ void __launch_bounds__(32)
+    k_small_fit(PatchArgs a, const int *__restrict__ plist, int np, int adj) {
+  const int e = blockIdx.x * 32 + threadIdx.x;
+  if (e >= np) return;
+  const int k = plist[e];
+  const double4 c = a.centers[k];
+  const double shift[3] = {c.x, c.y, c.z};
+  double *beta = a.pbeta + int64_t(e) * 4 * kMaxF;
+  int *act = a.pact + int64_t(e) * 8;
+  const int Fm = adj ? 0 : a.F;
   double red[kRedVals];
-  double beta[4 * kMaxF];
-  int64_t s0, t0;
-  int k, n, m, flag;
-  int act[3];
+  for (int v = 0; v < 10 + 4 * Fm; ++v) red[v] = a.pred[int64_t(e) * kRedVals + v];
+  // Coordinate ranges: only a failed condition test reads them.
+  auto ranges = [&](double *mn, double *mx) {
+    for (int d = 0; d < 3; ++d) {
+      mn[d] = INFINITY;
+      mx[d] = -INFINITY;
+    }
+    for (int64_t i = a.soff[k]; i < a.soff[k + 1]; ++i) {
+      const double4 p = a.src[a.sidx[i]];
+      mn[0] = fmin(mn[0], p.x);
+      mn[1] = fmin(mn[1], p.y);
+      mn[2] = fmin(mn[2], p.z);
+      mx[0] = fmax(mx[0], p.x);
+      mx[1] = fmax(mx[1], p.y);
+      mx[2] = fmax(mx[2], p.z);
+    }
+  };
+  int S[4] = {0, 0, 0, 0}, pv;
+  double R[4][4];
+  const int dropped = poly_axes(red, a.dim, shift, ranges, S, pv, R);
+  if (adj) {
+    for (int i = 0; i < 4; ++i) {
+      act[i] = S[i];
+      for (int j = 0; j < 4; ++j) beta[4 * i + j] = R[i][j];
+    }
+    act[4] = pv;
+  } else {
+    poly_fit(red, a.F, shift, S, pv, R, beta, act);
+    if (a.alpha_out != nullptr) {
+      double *bo = a.beta_out + int64_t(k) * 4 * kMaxF;
+      for (int v = 0; v < 4 * kMaxF; ++v) bo[v] = v < 4 * a.F ? beta[v] : 0.0;
+      for (int d = 0; d < 3; ++d) a.act_out[int64_t(k) * 3 + d] = act[d];
+    }
+  }
+  a.status[k] = dropped ? kStatusDropped : 0;
+}
+
+// 1 / d: the hardware's approximation r refined to r (1 + e + e^2), e = 1 - d r
+// (the series of the reciprocal), without branches so that it overlaps other
+// work.  Quotients formed with it are corrected (quot below).
+__device__ __forceinline__ double recip(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  double e = __fma_rn(-d, r, 1.0);
+  e = __fma_rn(e, e, e);
+  return __fma_rn(r, e, r);
+}
+
+// a / d from r ~ 1 / d: one residual correction (Markstein, IBM J. Res. Dev.
+// 34(1), 1990), exact where a = d.
+__device__ __forceinline__ double quot(double a, double d, double r) {
+  const double q = a * r;
+  return __fma_rn(__fma_rn(-q, d, a), r, q);
+}
+
+// sqrt(x) for x >= 0 without branches: the hardware's 1 / sqrt(x) and one
+// Goldschmidt step for g ~ sqrt(x), h ~ 1 / (2 sqrt(x)), then the residual
+// correction g + (x - g g) h (Markstein, IBM J. Res. Dev. 34(1), 1990).  Zero
+// and what the approximation flushes give zero, overflowed squares pass.
+__device__ __forceinline__ double root(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  double g = x * y, h = 0.5 * y;
+  const double e = __fma_rn(-g, h, 0.5);
+  g = __fma_rn(g, e, g);
+  h = __fma_rn(h, e, h);
+  g = __fma_rn(__fma_rn(-g, g, x), h, g);
+  g = x < 1e-290 ? 0.0 : g;
+  return x > 1e290 ? x : g;
+}
+
+// phi at squared distance d2 (common.cuh: wendland with its mask, r >= 0).
+template <int B>
+__device__ __forceinline__ double phi_at(double d2, double rinv) {
+  const double p = root(d2) * rinv;
+  const double q = 1.0 - p, q2 = q * q;
+  double v;
+  if (B == kWendlandC0) {
+    v = q2;
+  } else if (B == kWendlandC2) {
+    v = (q2 * q2) * fma(4.0, p, 1.0);
+  } else if (B == kWendlandC4) {
+    v = (q2 * q2 * q2) * fma(35.0, p * p, fma(18.0, p, 3.0));
+  } else if (B == kWendlandC6) {
+    const double q4 = q2 * q2, p2 = p * p;
+    v = (q4 * q4) * (fma(32.0, p2 * p, 25.0 * p2) + fma(8.0, p, 1.0));
+  } else {
+    const double q4 = q2 * q2, p2 = p * p;
+    double t = fma(1287.0, p2 * p2, 1350.0 * p2 * p);
+    t = fma(630.0, p2, t);
+    v = (q4 * q4 * q2) * (t + fma(150.0, p, 15.0));
+  }
+  return p >= 1.0 ? 0.0 : v;
+}
+
+// Calls fn(basis constant) with the basis as a compile-time constant, so that
+// the loops inside hold no switch.
+template <typename Fn>
+__device__ __forceinline__ void with_basis(int basis, Fn &&fn) {
+  switch (basis) {
+  case kWendlandC0: fn(std::integral_constant<int, kWendlandC0>{}); break;
+  case kWendlandC2: fn(std::integral_constant<int, kWendlandC2>{}); break;
+  case kWendlandC4: fn(std::integral_constant<int, kWendlandC4>{}); break;
+  case kWendlandC6: fn(std::integral_constant<int, kWendlandC6>{}); break;
+  default: fn(std::integral_constant<int, kWendlandC8>{}); break;
+  }
+}
+
+template <int N, int KF, bool ADJ>
+struct SmallCfg {
+  static constexpr int kT = N <= 32 ? 32 : 64;  // threads
+  static constexpr int kLd = N + 2;             // row stride: 16-byte rows, spread over the banks
+  static constexpr int kBlk = 16;               // pivots per unrolled group
+  // Resident blocks per SM the registers are shared out for.  A row takes 2 N
+  // registers; four, three or two warps per scheduler leave 128, 168 or 255.
+  static constexpr int kMinBlocks = 
+      N <= 32 ? 16 : (N <= 40 ? 8 : (N <= 48 || (KF == 1 ? N <= 56 || !ADJ : N <= 56 && !ADJ) ? 5 : 4));
 };
 
-__device__ __forceinline__ void team_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
-}
-
-// One reduced value of the polynomial pass: moments of the centred monomials
-// q = [1, x - c] (ids 0..9), q * b_f (ids 10..nred-1), then min x,y,z and
-// max x,y,z.  The points are summed in order.
-template <int N>
-__device__ double small_moment(const SmallShared<N> &S, int id, int nred, const double *shift) {
-  const int n = S.n;
-  if (id < nred) {
-    int i0, i1 = 0, f = -1;
-    if (id < 4) {
-      i0 = id;
-    } else if (id < 10) {
-      const int pr[6][2] = {{1, 1}, {1, 2}, {1, 3}, {2, 2}, {2, 3}, {3, 3}};
-      i0 = pr[id - 4][0];
-      i1 = pr[id - 4][1];
-    } else {
-      f = (id - 10) >> 2;
-      i0 = (id - 10) & 3;
-    }
-    double v = 0.0;
-    for (int i = 0; i < n; ++i) {
-      const double q[4] = {1.0, S.x[i] - shift[0], S.y[i] - shift[1], S.z[i] - shift[2]};
-      const double w = (f >= 0) ? S.b[f][i] : (id < 4 ? 1.0 : q[i1]);
-      v += q[i0] * w;
-    }
-    return v;
-  }
-  const int d = (id - nred) % 3;
-  const bool is_max = id - nred >= 3;
-  const double *x = d == 0 ? S.x : (d == 1 ? S.y : S.z);
-  double v = x[0];
-  for (int i = 1; i < n; ++i) v = is_max ? fmax(v, x[i]) : fmin(v, x[i]);
-  return v;
-}
-
-// The polynomial block as a real call: its local arrays and spills stay out
-// of the register allocation of the elimination.
-__device__ __noinline__ int poly_block_call(const double *red, int F, int dim, const double *shift,
-                                            double *beta, int *act) {
-  return poly_block(red, F, dim, shift, beta, act);
-}
-
-template <int N>
-__global__ void __launch_bounds__(SmallCfg<N>::kThreads)
-    k_small_chol(PatchArgs a, const int *__restrict__ plist, int np) {
-  using C = SmallCfg<N>;
-  __shared__ SmallShared<N> sh[C::kTeams];
-  const int tid = threadIdx.x;
+template <int N, int KF, bool ADJ>
+__global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>::kMinBlocks)
+    k_small_lu(PatchArgs a, const int *__restrict__ plist) {
+  using C = SmallCfg<N, KF, ADJ>;
+  constexpr int T = C::kT, LD = C::kLd, BLK = C::kBlk;
+  __shared__ __align__(16) double As[N * LD];
+  __shared__ __align__(16) double col[2][T + BLK];
+  __shared__ double xs[T], ys[T], zs[T];
+  __shared__ double rp[2][KF];
+  __shared__ double al[KF][T];
+  __shared__ int flag_s;
+  const int e = blockIdx.x;
+  const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
+  const int k = plist[e];
+  const int64_t s0 = a.soff[k];
+  const int n = int(a.soff[k + 1] - s0);
+  const int64_t t0 = a.toff[k];
+  const int m = int(a.toff[k + 1] - t0);
   const int F = a.F;
-  const int nred = 10 + 4 * F;
-  const bool poly_warp = tid >= C::kTeams * C::kTeam;
-  const int team = poly_warp ? 0 : tid / C::kTeam;
-  const int lt = tid % C::kTeam;
-  SmallShared<N> &S = sh[team];
-  const int e = blockIdx.x * C::kTeams + team;
-  const bool live = !poly_warp && e < np;
+  const double *beta = a.pbeta + int64_t(e) * 4 * kMaxF;
+  const int *act = a.pact + int64_t(e) * 8;
+  const bool load = a.fac_mode == 2;
+  if (i == 0) flag_s = 0;
 
-  // Gather the patch (TeamFillB, team_ops.hpp:113-121), zero padded to N.
-  if (!poly_warp) {
-    int k = 0, n = 0, m = 0;
-    int64_t s0 = 0, t0 = 0;
-    if (live) {
-      k = plist[e];
-      s0 = a.soff[k];
-      n = int(a.soff[k + 1] - s0);
-      t0 = a.toff[k];
-      m = int(a.toff[k + 1] - t0);
-    }
-    if (lt == 0) {
-      S.k = k;
-      S.n = n;
-      S.m = m;
-      S.s0 = s0;
-      S.t0 = t0;
-      S.flag = 0;
-    }
-    if (lt < 4 * kMaxF) S.beta[lt] = 0.0;
-    for (int i = lt; i < N; i += C::kTeam) {
-      double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
-      int id = 0;
-      if (i < n) {
-        id = a.sidx[s0 + i];
-        p = a.src[id];
-      }
-      S.x[i] = p.x;
-      S.y[i] = p.y;
-      S.z[i] = p.z;
-      for (int f = 0; f < F; ++f) S.b[f][i] = i < n ? a.vals[int64_t(id) * F + f] : 0.0;
+  // Gather the patch (TeamFillB, team_ops.hpp:113-121) and form the residual
+  // b - Q beta (serial_ops.hpp:149-185).
+  double r[KF];
+#pragma unroll
+  for (int f = 0; f < KF; ++f) r[f] = 0.0;
+  double4 x = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (i < n) {
+    const int id = a.sidx[s0 + i];
+    x = a.src[id];
+    if (!ADJ) {
+      const double pc[3] = {x.x, x.y, x.z};
+#pragma unroll
+      for (int f = 0; f < KF; ++f)
+        if (f < F) {
+          double t = beta[4 * f];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const int ax = act[j];
+            if (ax >= 0) t = __fma_rn(ax == 0 ? pc[0] : (ax == 1 ? pc[1] : pc[2]), beta[4 * f + 1 + j], t);
+          }
+          r[f] = a.vals[int64_t(id) * F + f] - t;
+        }
     }
   }
+  xs[i] = x.x;
+  ys[i] = x.y;
+  zs[i] = x.z;
   __syncthreads();
 
-  if (poly_warp) {
-    // Moments, condition test and least squares of every live patch.
-    const int lane = tid & 31;
-    for (int t = 0; t < C::kTeams; ++t) {
-      SmallShared<N> &P = sh[t];
-      if (P.n == 0) continue;
-      const double4 c = a.centers[P.k];
-      const double shift[3] = {c.x, c.y, c.z};
-      for (int id = lane; id < nred + 6; id += 32) P.red[id] = small_moment(P, id, nred, shift);
-    }
-    __syncwarp();
-    if (lane < C::kTeams && sh[lane].n > 0) {
-      SmallShared<N> &P = sh[lane];
-      const double4 c = a.centers[P.k];
-      const double shift[3] = {c.x, c.y, c.z};
-      int act[3];
-      const int dropped = poly_block_call(P.red, F, a.dim, shift, P.beta, act);
-      for (int d = 0; d < 3; ++d) P.act[d] = act[d];
-      if (dropped) atomicOr(&P.flag, kStatusDropped);
+  if (ADJ && i < n) {
+    // Right-hand sides E^T h, E_ij = phi(|y_i - x_j|).
+    with_basis(a.basis, [&](auto B) {
+      for (int t = 0; t < m; ++t) {
+        const double4 y = a.tgt[a.tidx[t0 + t]];
+        const double ph = phi_at<B>(sqdist3(y.x, y.y, y.z, x.x, x.y, x.z), a.rinv);
+#pragma unroll
+        for (int f = 0; f < KF; ++f)
+          if (f < F) r[f] = __fma_rn(ph, a.h[(t0 + t) * F + f], r[f]);
+      }
+    });
+  }
+
+  bool bad = false;
+  if (!load) {
+    // Assembly (TeamFillA, team_ops.hpp:35-52): thread i evaluates the pairs
+    // (i, i + d mod n), d <= n / 2, which covers every pair of the symmetric
+    // matrix with equal work per thread.
+    if (i < n) {
+      with_basis(a.basis, [&](auto B) {
+        int j = i;
+        for (int d = 0; d <= n / 2; ++d) {
+          const double v = phi_at<B>(sqdist3(x.x, x.y, x.z, xs[j], ys[j], zs[j]), a.rinv);
+          As[i * LD + j] = v;
+          As[j * LD + i] = v;
+          if (++j == n) j = 0;
+        }
+      });
     }
     __syncthreads();
-    return;
-  }
-
-  // Assembly (TeamFillA, team_ops.hpp:35-52) and elimination in registers,
-  // or the eliminated blocks of an earlier execute (fac_mode 2).
-  const int n = S.n;
-  const int bi = lt / C::kG, bs = lt % C::kG;
-  const int bar = 1 + team;
-  double *facp = (a.fac_mode != 0 && live) ? a.fac + size_t(e) * N * N + size_t(lt) * 16 : nullptr;
-  double v[4][4];
-  const bool load = a.fac_mode == 2;
-  if (load && facp) {
+    double row[N];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const double2 lo = *reinterpret_cast<const double2 *>(facp + 4 * r);
-      const double2 hi = *reinterpret_cast<const double2 *>(facp + 4 * r + 2);
-      v[r][0] = lo.x;
-      v[r][1] = lo.y;
-      v[r][2] = hi.x;
-      v[r][3] = hi.y;
+    for (int j = 0; j < N; j += 2) {
+      double2 v = make_double2(0.0, 0.0);
+      if (i < n && j < n) v = *reinterpret_cast<const double2 *>(&As[i * LD + j]);
+      row[j] = v.x;
+      row[j + 1] = j + 1 < n ? v.y : 0.0;
+    }
+    col[0][i] = row[0];
+    if (i == 0) {
+#pragma unroll
+      for (int f = 0; f < KF; ++f) rp[0][f] = r[f];
+    }
+#pragma unroll 1
+    for (int pb = 0; pb < n; pb += BLK) {
+#pragma unroll
+      for (int q = 0; q < BLK; ++q) {
+        const int p = pb + q;
+        if (p < n) {
+          __syncthreads();
+          const double *cp = &col[q & 1][pb];  // this column from row pb on
+          const double d = cp[q];
+          bad |= !(d > 0.0);
+          double mi = quot(row[q], d, recip(d));
+          if (i <= p) mi = 0.0;
+          else row[q] = mi;
+          if (q + 1 < N) {
+            row[q + 1] = __fma_rn(-mi, cp[q + 1], row[q + 1]);
+            col[(q + 1) & 1][i] = row[q + 1];
+          }
+#pragma unroll
+          for (int f = 0; f < KF; ++f) r[f] = __fma_rn(-mi, rp[q & 1][f], r[f]);
+          if (i == p + 1) {
+#pragma unroll
+            for (int f = 0; f < KF; ++f) rp[(q + 1) & 1][f] = r[f];
+          }
+          // The rest of the row, in groups of eight columns up to n.
+#pragma unroll
+          for (int g = 0; g < N / 8; ++g) {
+            if (8 * g + 7 >= q + 2 && pb + 8 * g < n) {
+#pragma unroll
+              for (int j = 8 * g; j < 8 * g + 8; ++j)
+                if (j >= q + 2) row[j] = __fma_rn(-mi, cp[j], row[j]);
+            }
+          }
+        }
+      }
+      if (i < N) {
+#pragma unroll
+        for (int q = 0; q < BLK; q += 2)
+          if (N % BLK == 0 || pb + q < N)
+            *reinterpret_cast<double2 *>(&As[i * LD + pb + q]) = make_double2(row[q], row[q + 1]);
+      }
+      if constexpr (N > BLK) {
+#pragma unroll
+        for (int j = 0; j + BLK < N; ++j) row[j] = row[j + BLK];
+      }
+    }
+    __syncthreads();
+    if (a.fac_mode == 1) {
+      double *facp = a.fac + size_t(e) * N * N;
+      for (int v = i; v < N * N / 2; v += T) {
+        const int rr = v / (N / 2), cc = 2 * (v % (N / 2));
+        if (rr < n && cc < n)
+          *reinterpret_cast<double2 *>(facp + rr * N + cc) =
+              *reinterpret_cast<const double2 *>(&As[rr * LD + cc]);
+      }
     }
   } else {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int i = 4 * bi + r, s = 4 * bs + b;
-        double val = 0.0;
-        if (s <= i) {
-          if (!load && i < n && s < n)
-            val = wendland<double>(
-                a.basis, __dsqrt_rn(sqdist3(S.x[i], S.y[i], S.z[i], S.x[s], S.y[s], S.z[s])),
-                a.rinv);
-          else
-            val = (i == s) ? 1.0 : 0.0;
-        }
-        v[r][b] = val;
-      }
-  }
-  bool bad = false;
-  for (int p = 0; p < (load ? 0 : n); ++p) {
-    double *c = S.cv[p & 1];
-    const int pb = p >> 2, pr = p & 3;
-    if (bi == pb) {  // row p: L^{-1}[p][s] for s < p, the pivot at s = p
-#pragma unroll
-      for (int b = 0; b < 4; ++b)
-        if (4 * bs + b <= p) {
-          double x = v[0][b];
-          if (pr == 1) x = v[1][b];
-          if (pr == 2) x = v[2][b];
-          if (pr == 3) x = v[3][b];
-          c[4 * bs + b] = x;
-        }
+    // Kept factors of an earlier execute; the forward substitution, which
+    // the elimination does on the way, is done from them.
+    const double *facp = a.fac + size_t(e) * N * N;
+    for (int v = i; v < N * N / 2; v += T) {
+      const int rr = v / (N / 2), cc = 2 * (v % (N / 2));
+      if (rr < n && cc < n)
+        *reinterpret_cast<double2 *>(&As[rr * LD + cc]) =
+            *reinterpret_cast<const double2 *>(facp + rr * N + cc);
     }
-    if (bs == pb) {  // column p below the pivot
+    __syncthreads();
+    const int n0 = n < 32 ? n : 32;
+    const double *ar = As + (i < n ? i : 0) * LD;
+    if (warp == 0) {
+      for (int p = 0; p < n0; ++p) {
+        const double l = (lane > p && i < n) ? ar[p] : 0.0;
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (4 * bi + r > p) {
-          double x = v[r][0];
-          if (pr == 1) x = v[r][1];
-          if (pr == 2) x = v[r][2];
-          if (pr == 3) x = v[r][3];
-          c[4 * bi + r] = x;
-        }
-    }
-    team_sync(bar, C::kTeam);
-    const double piv = c[p];
-    bad |= !(piv > 0.0);
-    const double inv = 1.0 / piv;
-    double cs[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) cs[b] = c[4 * bs + b];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int i = 4 * bi + r;
-      if (i > p) {
-        const double mlt = c[i] * inv;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int s = 4 * bs + b;
-          if (s == p) v[r][b] = -mlt;
-          else if (s <= i) v[r][b] = __fma_rn(-mlt, cs[b], v[r][b]);
-        }
+        for (int f = 0; f < KF; ++f)
+          r[f] = __fma_rn(-l, __shfl_sync(0xffffffffu, r[f], p), r[f]);
       }
     }
-  }
-  if (a.fac_mode == 1 && facp) {
+    if (T > 32) {
+      if (warp == 0) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      *reinterpret_cast<double2 *>(facp + 4 * r) = make_double2(v[r][0], v[r][1]);
-      *reinterpret_cast<double2 *>(facp + 4 * r + 2) = make_double2(v[r][2], v[r][3]);
-    }
-  }
-  if (bi == bs) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) S.d[4 * bi + r] = v[r][r];
-  }
-  __syncthreads();  // the polynomial warp is done: beta and act are final
-
-  // Residual r = b - Q beta (serial_ops.hpp:149-185).
-  for (int e2 = lt; e2 < N * F; e2 += C::kTeam) {
-    const int i = e2 % N, f = e2 / N;
-    double r = 0.0;
-    if (i < n) {
-      const double pc[3] = {S.x[i], S.y[i], S.z[i]};
-      double t = S.beta[4 * f];
-      for (int j = 0; j < 3; ++j)
-        if (S.act[j] >= 0) t = __fma_rn(pc[S.act[j]], S.beta[4 * f + 1 + j], t);
-      r = S.b[f][i] - t;
-    }
-    S.b[f][i] = r;
-  }
-  team_sync(bar, C::kTeam);
-  // alpha = L^{-T} D^{-1} L^{-1} r, L^{-1}[i][s] = slot (i, s) for s < i, 1 at s = i.
-  for (int f = 0; f < F; ++f) {
-    double pr4[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int i = 4 * bi + r;
-      double s = 0.0;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int sc = 4 * bs + b;
-        const double y = sc < i ? v[r][b] : (sc == i ? 1.0 : 0.0);
-        s = __fma_rn(y, S.b[f][sc], s);
+        for (int f = 0; f < KF; ++f) al[f][i] = r[f];
       }
-      pr4[r] = s;
-    }
+      __syncthreads();
+      if (warp == 1) {
+        if (i < n) {
+          for (int p = 0; p < 32; ++p) {
+            const double l = ar[p];
 #pragma unroll
-    for (int o = C::kG / 2; o > 0; o >>= 1)
+            for (int f = 0; f < KF; ++f) r[f] = __fma_rn(-l, al[f][p], r[f]);
+          }
+        }
+        for (int p = 32; p < n; ++p) {
+          const double l = (i > p && i < n) ? ar[p] : 0.0;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) pr4[r] += __shfl_xor_sync(0xffffffffu, pr4[r], o);
-    if (bs == 0) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) S.w[f][4 * bi + r] = pr4[r] / S.d[4 * bi + r];
-    }
-    team_sync(bar, C::kTeam);
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int sc = 4 * bs + b;
-      double s = 0.0;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int i = 4 * bi + r;
-        const double y = sc < i ? v[r][b] : (sc == i ? 1.0 : 0.0);
-        s = __fma_rn(y, S.w[f][i], s);
+          for (int f = 0; f < KF; ++f)
+            r[f] = __fma_rn(-l, __shfl_sync(0xffffffffu, r[f], p - 32), r[f]);
+        }
       }
-      S.part[bi][sc] = s;
+      __syncthreads();
     }
-    team_sync(bar, C::kTeam);
-    if (lt < N) {
-      double s = 0.0;
-      for (int q = 0; q < C::kG; ++q) s += S.part[q][lt];
-      S.w[f][lt] = s;
-    }
-    team_sync(bar, C::kTeam);
-  }
-  if (a.alpha_out != nullptr && live) {  // teams past the end of the list hold no patch
-    for (int e2 = lt; e2 < n * F; e2 += C::kTeam) {
-      const int j = e2 / F, f = e2 % F;
-      a.alpha_out[(S.s0 + j) * F + f] = S.w[f][j];
-    }
-    if (lt < 4 * kMaxF) a.beta_out[int64_t(S.k) * 4 * kMaxF + lt] = S.beta[lt];
-    if (lt < 3) a.act_out[int64_t(S.k) * 3 + lt] = S.act[lt];
   }
 
-  // local = E alpha + V beta (solver.hpp:270-273): kTPT threads per target,
-  // 16 sources each.
-  const int m = S.m;
-  const int sub = lt % C::kTPT;
+  // U alpha = y: each warp its own rows from the last, the second warp's
+  // results through shared memory.
+  {
+    const double *ar = As + (i < n ? i : 0) * LD;
+    const double dg = i < n ? ar[i] : 1.0;
+    const double inv = recip(dg);
+    if (T > 32) {
+      if (warp == 1) {
+        for (int j = n - 1; j >= 32; --j) {
+          const double u = (i < j) ? ar[j] : 0.0;
+#pragma unroll
+          for (int f = 0; f < KF; ++f) {
+            const double xj = __shfl_sync(0xffffffffu, quot(r[f], dg, inv), j - 32);
+            if (i == j) r[f] = xj;
+            else r[f] = __fma_rn(-u, xj, r[f]);
+          }
+        }
+#pragma unroll
+        for (int f = 0; f < KF; ++f) al[f][i] = r[f];
+      }
+      __syncthreads();
+      if (warp == 0) {
+        for (int j = 32; j < n; ++j) {
+          const double u = ar[j];
+#pragma unroll
+          for (int f = 0; f < KF; ++f) r[f] = __fma_rn(-u, al[f][j], r[f]);
+        }
+      }
+    }
+    if (warp == 0) {
+      for (int j = (n < 32 ? n : 32) - 1; j >= 0; --j) {
+        const double u = (i < j) ? ar[j] : 0.0;
+#pragma unroll
+        for (int f = 0; f < KF; ++f) {
+          const double xj = __shfl_sync(0xffffffffu, quot(r[f], dg, inv), j);
+          if (i == j) r[f] = xj;
+          else r[f] = __fma_rn(-u, xj, r[f]);
+        }
+      }
+#pragma unroll
+      for (int f = 0; f < KF; ++f) al[f][i] = r[f];
+    }
+    __syncthreads();
+  }
+
   bool nonfinite = false;
-  for (int i = lt / C::kTPT; i < ((m + C::kTeam / C::kTPT - 1) / (C::kTeam / C::kTPT)) *
-                                     (C::kTeam / C::kTPT);
-       i += C::kTeam / C::kTPT) {
-    double acc[kMaxF];
-#pragma unroll
-    for (int f = 0; f < kMaxF; ++f) acc[f] = 0.0;
-    double4 y = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (i < m) {
-      y = a.tgt[a.tidx[S.t0 + i]];
-      const int j1 = min(n, 16 * sub + 16);
-      for (int j = 16 * sub; j < j1; ++j) {
-        const double ph = wendland<double>(
-            a.basis, __dsqrt_rn(sqdist3(y.x, y.y, y.z, S.x[j], S.y[j], S.z[j])), a.rinv);
-#pragma unroll
-        for (int f = 0; f < kMaxF; ++f)
-          if (f < F) acc[f] = __fma_rn(ph, S.w[f][j], acc[f]);
+  if (ADJ) {
+    // g = z - Q' G'^{-1} (Q'^T z - V'^T h), centred monomials q' = [1, x - c]:
+    // the sums by one thread per (field, monomial), points in order.
+    __shared__ double corr[4 * KF];
+    const double4 c = a.centers[k];
+    if (i < 4 * KF && (i >> 2) < F) {
+      const int f = i >> 2, ax = i & 3;
+      const double cc = ax == 1 ? c.x : (ax == 2 ? c.y : c.z);
+      const double *xc = ax == 1 ? xs : (ax == 2 ? ys : zs);
+      double u = 0.0, v = 0.0;
+      for (int j = 0; j < n; ++j) u += (ax == 0 ? 1.0 : xc[j] - cc) * al[f][j];
+      for (int t = 0; t < m; ++t) {
+        const double4 y = a.tgt[a.tidx[t0 + t]];
+        const double yc = ax == 1 ? y.x : (ax == 2 ? y.y : y.z);
+        v += (ax == 0 ? 1.0 : yc - cc) * a.h[(t0 + t) * F + f];
       }
+      corr[4 * f + ax] = u - v;
     }
+    __syncthreads();
+    if (i < F) {
+      double R[4][4], rhs[4] = {0, 0, 0, 0}, sol[4] = {0, 0, 0, 0};
+      const int pv = act[4];
+      for (int q = 0; q < 4; ++q)
+        for (int j = 0; j < 4; ++j) R[q][j] = beta[4 * q + j];
+      for (int q = 0; q < pv; ++q) rhs[q] = corr[4 * i + act[q]];
+      gram_solve(R, pv, rhs, sol);
+      for (int q = 0; q < 4; ++q) corr[4 * i + q] = 0.0;
+      for (int q = 0; q < pv; ++q) corr[4 * i + act[q]] = sol[q];
+    }
+    __syncthreads();
+    if (i < n) {
+      const double q[3] = {x.x - c.x, x.y - c.y, x.z - c.z};
 #pragma unroll
-    for (int o = C::kTPT / 2; o > 0; o >>= 1)
+      for (int f = 0; f < KF; ++f)
+        if (f < F) {
+          double g = al[f][i];
+          g -= corr[4 * f];
 #pragma unroll
-      for (int f = 0; f < kMaxF; ++f)
-        if (f < F) acc[f] += __shfl_xor_sync(0xffffffffu, acc[f], o);
-    if (i < m && sub == 0) {
-      const double yc[3] = {y.x, y.y, y.z};
-      for (int f = 0; f < F; ++f) {
-        double vb = S.beta[4 * f];
-        for (int d = 0; d < 3; ++d)
-          if (S.act[d] >= 0) vb = __fma_rn(yc[S.act[d]], S.beta[4 * f + 1 + d], vb);
-        const double out = acc[f] + vb;
-        nonfinite |= !isfinite(out);
-        a.local[(S.t0 + i) * F + f] = out;
+          for (int d = 0; d < 3; ++d) g -= q[d] * corr[4 * f + 1 + d];
+          nonfinite |= !isfinite(g);
+          a.g_out[(s0 + i) * F + f] = g;
+        }
+    }
+  } else {
+    if (a.alpha_out != nullptr && i < n) {
+#pragma unroll
+      for (int f = 0; f < KF; ++f)
+        if (f < F) a.alpha_out[(s0 + i) * F + f] = al[f][i];
+    }
+    // local = E alpha + V beta (solver.hpp:270-273), a thread per target, two
+    // sources at a time with a sum each.
+    with_basis(a.basis, [&](auto B) {
+      for (int t = i; t < m; t += T) {
+        const double4 y = a.tgt[a.tidx[t0 + t]];
+        double acc[KF], odd[KF];
+#pragma unroll
+        for (int f = 0; f < KF; ++f) acc[f] = odd[f] = 0.0;
+        auto at = [&](int j, double *sum) {
+          const double ph = phi_at<B>(sqdist3(y.x, y.y, y.z, xs[j], ys[j], zs[j]), a.rinv);
+#pragma unroll
+          for (int f = 0; f < KF; ++f) sum[f] = __fma_rn(ph, al[f][j], sum[f]);
+        };
+        int j = 0;
+        for (; j + 1 < n; j += 2) {
+          at(j, acc);
+          at(j + 1, odd);
+        }
+        if (j < n) at(j, acc);
+#pragma unroll
+        for (int f = 0; f < KF; ++f) acc[f] += odd[f];
+        const double yc[3] = {y.x, y.y, y.z};
+#pragma unroll
+        for (int f = 0; f < KF; ++f)
+          if (f < F) {
+            double vb = beta[4 * f];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+              const int ax = act[j];
+              if (ax >= 0) vb = __fma_rn(ax == 0 ? yc[0] : (ax == 1 ? yc[1] : yc[2]), beta[4 * f + 1 + j], vb);
+            }
+            const double out = acc[f] + vb;
+            nonfinite |= !isfinite(out);
+            a.local[(t0 + t) * F + f] = out;
+          }
       }
-    }
+    });
   }
-  if (nonfinite) atomicOr(&S.flag, kStatusNonFinite);
-  if (lt == 0 && bad) atomicOr(&S.flag, kStatusBreakdown);
-  team_sync(bar, C::kTeam);
-  if (lt == 0 && live) a.status[S.k] = S.flag;
+  if (nonfinite) atomicOr(&flag_s, kStatusNonFinite);
+  if (bad && i == 0) atomicOr(&flag_s, kStatusBreakdown);
+  __syncthreads();
+  if (i == 0 && flag_s) a.status[k] |= flag_s;
+}
+
+template <int N, bool ADJ>
+void launch_n(const PatchArgs &a, const int *plist, int np, cudaStream_t st) {
+  const int T = SmallCfg<N, 1, ADJ>::kT;
+  if (a.F == 1) k_small_lu<N, 1, ADJ><<<np, T, 0, st>>>(a, plist);
+  else if (a.F <= 4) k_small_lu<N, 4, ADJ><<<np, T, 0, st>>>(a, plist);
+  else k_small_lu<N, 8, ADJ><<<np, T, 0, st>>>(a, plist);
+  note_launch();
+  PB_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
-void launch_small_chol(const PatchArgs &a, const int *plist, int np, int nmax, cudaStream_t st) {
+int small_class(int n) { return n <= 32 ? 32 : (n + 7) / 8 * 8; }
+
+void launch_small_poly(const PatchArgs &a, const int *plist, int np, bool adj, cudaStream_t st) {
   if (np == 0) return;
-  if (nmax <= 32) {
-    using C = SmallCfg<32>;
-    k_small_chol<32><<<(np + C::kTeams - 1) / C::kTeams, C::kThreads, 0, st>>>(a, plist, np);
-  } else {
-    using C = SmallCfg<64>;
-    k_small_chol<64><<<(np + C::kTeams - 1) / C::kTeams, C::kThreads, 0, st>>>(a, plist, np);
-  }
-  note_launch();
+  k_small_moments<<<(np + kMomWarps - 1) / kMomWarps, kMomWarps * 32, 0, st>>>(
+      a, plist, np, adj ? 0 : a.F);
+  k_small_fit<<<(np + 31) / 32, 32, 0, st>>>(a, plist, np, adj ? 1 : 0);
+  note_launch(2);
   PB_CUDA(cudaGetLastError());
+}
+
+void launch_small_lu(const PatchArgs &a, const int *plist, int np, int N, bool adj,
+                     cudaStream_t st) {
+  if (np == 0) return;
+  auto go = [&](auto A) {
+    constexpr bool kAdjoint = decltype(A)::value;
+    switch (N) {
+    case 32: launch_n<32, kAdjoint>(a, plist, np, st); break;
+    case 40: launch_n<40, kAdjoint>(a, plist, np, st); break;
+    case 48: launch_n<48, kAdjoint>(a, plist, np, st); break;
+    case 56: launch_n<56, kAdjoint>(a, plist, np, st); break;
+    default: launch_n<64, kAdjoint>(a, plist, np, st); break;
+    }
+  };
+  if (adj) go(std::true_type{});
+  else go(std::false_type{});
 }
 
 }  // namespace pacman_b200

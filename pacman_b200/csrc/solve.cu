@@ -354,89 +354,132 @@ static void launch(int mode, const PatchArgs &a, const int *plist, int np, int u
   PB_CUDA(cudaGetLastError());
 }
 
-// Runs one mode over a list of patches: buckets by size so the dynamic
-// shared memory follows the bucket's largest patch; patches too large for
-// shared memory use the global workspace.
-static void run_list(Plan &p, PatchArgs a, int mode, const std::vector<int> &patches,
-                     SolveReport &rep, cudaStream_t st, FactorCache *keep = nullptr) {
-  if (patches.empty()) return;
-  for (int k : patches) {
-    const double n = p.n_host[k], m = p.m_host[k];
-    rep.factor_flops += (mode == kLU ? 2.0 / 3.0 : 1.0 / 3.0) * n * n * n +
-                        2.0 * n * n * a.F + 2.0 * m * n * a.F;
+// Polynomial results of `count` register-kernel patches (launch_small_poly).
+struct PolyBuf {
+  DevMem beta, act, red;
+  void alloc(size_t count, cudaStream_t st, PatchArgs &a) {
+    red.alloc(sizeof(double) * kRedVals * count, st);
+    a.pred = red.as<double>();
+    beta.alloc(sizeof(double) * 4 * kMaxF * count, st);
+    act.alloc(sizeof(int) * 8 * count, st);
+    a.pbeta = beta.as<double>();
+    a.pact = act.as<int>();
   }
+};
+
+// One launch per size class over the register-kernel patches of a list whose
+// classes lie one after another.
+static void run_register_ranges(PatchArgs a, const std::vector<SmallRange> &ranges,
+                                const int *list, bool adj, double *fac, int fac_mode,
+                                cudaStream_t st) {
+  for (const SmallRange &r : ranges) {
+    PatchArgs b = a;
+    b.pbeta = a.pbeta + r.first * 4 * kMaxF;
+    b.pact = a.pact + r.first * 8;
+    b.fac = fac ? fac + r.fac_off : nullptr;
+    b.fac_mode = fac ? fac_mode : 0;
+    launch_small_lu(b, list + r.first, r.count, r.nclass, adj, st);
+  }
+}
+
+// Runs one mode over a list of patches: n <= kSmallMax in the register kernel,
+// by size class; the rest in k_patch_solve, in buckets of doubling size so
+// that the dynamic shared memory follows the bucket's largest patch, patches
+// too large for shared memory in a global workspace.  general: every patch in
+// k_patch_solve.
+static void run_list(Plan &p, PatchArgs a, int mode, const std::vector<int> &patches,
+                     SolveReport &rep, cudaStream_t st, FactorCache *keep = nullptr,
+                     bool general = false) {
+  if (patches.empty()) return;
   const int F = a.F;
   const size_t smem_cap = 200 * 1024;
-  std::vector<int> order(patches);
-  std::sort(order.begin(), order.end(),
-            [&](int x, int y) { return p.n_host[x] < p.n_host[y]; });
+  // Register-kernel classes, the largest first (the last blocks to start are
+  // then the shortest), then the rest by size.
+  std::vector<int> host_list, rest;
+  host_list.reserve(patches.size());
+  std::vector<SmallRange> ranges;
+  if (!general) {
+    constexpr int kClasses = (kSmallMax - 32) / 8 + 1;
+    std::vector<int> cls[kClasses];  // sizes 64, 56, 48, 40, 32
+    for (int k : patches) {
+      const int n = p.n_host[k];
+      if (n > kSmallMax) rest.push_back(k);
+      else cls[(kSmallMax - small_class(n)) / 8].push_back(k);
+    }
+    // A class that would not fill the GPU joins the next larger one: its own
+    // launch would only add the latency of one patch.
+    const size_t fill = size_t(5) * size_t(tuning_for_current_device().sms);
+    for (int c = 1; c < kClasses; ++c)
+      if (!cls[c].empty() && cls[c].size() < fill) {
+        int to = c - 1;
+        while (to > 0 && cls[to].empty()) --to;
+        if (cls[to].empty()) continue;
+        cls[to].insert(cls[to].end(), cls[c].begin(), cls[c].end());
+        cls[c].clear();
+      }
+    size_t tot = 0;
+    for (int ci = 0; ci < kClasses; ++ci) {
+      const std::vector<int> &c = cls[ci];
+      if (c.empty()) continue;
+      SmallRange sr;
+      sr.first = host_list.size();
+      sr.count = int(c.size());
+      sr.nclass = kSmallMax - 8 * ci;
+      sr.fac_off = tot;
+      tot += c.size() * small_fac_doubles(sr.nclass);
+      ranges.push_back(sr);
+      host_list.insert(host_list.end(), c.begin(), c.end());
+    }
+    if (keep) {
+      keep->ranges = ranges;
+      keep->small_fac.alloc(sizeof(double) * std::max<size_t>(tot, 2), st);
+    }
+  } else {
+    rest = patches;
+  }
+  const size_t nreg = host_list.size();
+  for (int k : patches) {
+    const double n = p.n_host[k], m = p.m_host[k];
+    rep.factor_flops += (mode == kLU ? 2.0 / 3.0 : 1.0 / 3.0) * n * n * n + 2.0 * n * n * F +
+                        2.0 * m * n * F;
+  }
+  std::sort(rest.begin(), rest.end(), [&](int x, int y) { return p.n_host[x] < p.n_host[y]; });
   std::vector<int> small, big;
-  for (int k : order) {
+  for (int k : rest) {
     if (smem_bytes(p.n_host[k], F, true) <= smem_cap) small.push_back(k);
     else big.push_back(k);
   }
-  // Small: buckets of doubling size, each launched with its own shared memory.
+  host_list.insert(host_list.end(), small.begin(), small.end());
+  host_list.insert(host_list.end(), big.begin(), big.end());
+  DevMem list;
+  list.alloc(sizeof(int) * host_list.size(), st);
+  HostArena::get().upload(host_list.data(), host_list.size(), list.p, st);
+  if (nreg) {
+    PolyBuf poly;
+    poly.alloc(nreg, st, a);
+    launch_small_poly(a, list.as<int>(), int(nreg), mode == kAdj, st);
+    run_register_ranges(a, ranges, list.as<int>(), mode == kAdj,
+                        keep ? keep->small_fac.as<double>() : nullptr, 1, st);
+  }
+  // Buckets of doubling size, each launched with its own shared memory.
   size_t pos = 0;
-  std::vector<std::pair<size_t, size_t>> ranges;
   while (pos < small.size()) {
     const int n0 = p.n_host[small[pos]];
     int cap = 32;
     while (cap < n0) cap *= 2;
     size_t end = pos;
-    while (end < small.size() && p.n_host[small[end]] <= cap &&
-           smem_bytes(p.n_host[small[end]], F, true) <= smem_cap)
-      ++end;
-    ranges.emplace_back(pos, end);
+    while (end < small.size() && p.n_host[small[end]] <= cap) ++end;
+    launch(mode, a, list.as<int>() + nreg + pos, int(end - pos), 0,
+           smem_bytes(p.n_host[small[end - 1]], F, true), st);
     pos = end;
-  }
-  std::vector<int> host_list(small);
-  host_list.insert(host_list.end(), big.begin(), big.end());
-  DevMem list;
-  list.alloc(sizeof(int) * host_list.size(), st);
-  HostArena::get().upload(host_list.data(), host_list.size(), list.p, st);
-  if (keep) {
-    // Kept factors of the register kernel: N * N doubles per patch of the
-    // launch's size class, in launch order.
-    size_t tot = 0;
-    keep->ranges.clear();
-    for (auto &r : ranges) {
-      int nmax = 0;
-      for (size_t i = r.first; i < r.second; ++i) nmax = std::max(nmax, p.n_host[small[i]]);
-      if (mode != kChol || nmax > 64) continue;
-      SmallRange sr;
-      sr.first = r.first;
-      sr.count = int(r.second - r.first);
-      sr.nmax = nmax;
-      sr.fac_off = tot;
-      tot += size_t(sr.count) * small_fac_doubles(nmax <= 32 ? 32 : 64);
-      keep->ranges.push_back(sr);
-    }
-    keep->small_fac.alloc(sizeof(double) * std::max<size_t>(tot, 2), st);
-  }
-  size_t ri = 0;
-  for (auto &r : ranges) {
-    int nmax = 0;
-    for (size_t i = r.first; i < r.second; ++i) nmax = std::max(nmax, p.n_host[small[i]]);
-    if (mode == kChol && nmax <= 64) {
-      PatchArgs b = a;
-      if (keep) {
-        b.fac = keep->small_fac.as<double>() + keep->ranges[ri++].fac_off;
-        b.fac_mode = 1;
-      }
-      launch_small_chol(b, list.as<int>() + r.first, int(r.second - r.first), nmax, st);
-    } else
-      launch(mode, a, list.as<int>() + r.first, int(r.second - r.first), 0,
-             smem_bytes(nmax, F, true), st);
   }
   if (!big.empty()) {
     std::vector<int64_t> offs(big.size());
     int64_t tot = 0;
-    int nmax = 0;
     for (size_t i = 0; i < big.size(); ++i) {
       offs[i] = tot;
       const int64_t n = p.n_host[big[i]];
       tot += n * (n + F);
-      nmax = std::max<int>(nmax, int(n));
     }
     DevMem goff, gA;
     goff.alloc(sizeof(int64_t) * big.size(), st);
@@ -445,20 +488,22 @@ static void run_list(Plan &p, PatchArgs a, int mode, const std::vector<int> &pat
     PatchArgs b = a;
     b.gA = gA.as<double>();
     b.gAoff = goff.as<int64_t>();
-    launch(mode, b, list.as<int>() + small.size(), int(big.size()), 1,
-           smem_bytes(nmax, F, false), st);
+    launch(mode, b, list.as<int>() + nreg + small.size(), int(big.size()), 1,
+           smem_bytes(p.n_host[big.back()], F, false), st);
   }
   if (keep) keep->small_list = std::move(list);  // freed with the plan's cache
 }
 
 // The register-kernel patches from kept factors.
 static void run_small_cached(const FactorCache &c, PatchArgs a, cudaStream_t st) {
-  for (const SmallRange &r : c.ranges) {
-    PatchArgs b = a;
-    b.fac = const_cast<double *>(c.small_fac.as<double>()) + r.fac_off;
-    b.fac_mode = 2;
-    launch_small_chol(b, c.small_list.as<int>() + r.first, r.count, r.nmax, st);
-  }
+  size_t nreg = 0;
+  for (const SmallRange &r : c.ranges) nreg += size_t(r.count);
+  if (nreg == 0) return;
+  PolyBuf poly;
+  poly.alloc(nreg, st, a);
+  launch_small_poly(a, c.small_list.as<int>(), int(nreg), false, st);
+  run_register_ranges(a, c.ranges, c.small_list.as<int>(), false,
+                      const_cast<double *>(c.small_fac.as<double>()), 2, st);
 }
 
 void solve_big(Plan &p, int basis, const double *vals, int F, bool lu,
@@ -578,7 +623,10 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;
     if (stat[k] & kStatusDropped) rep.dropped++;
-    if ((mode == kChol && (stat[k] & (kStatusBreakdown | kStatusNonFinite | kStatusTimeout))) ||
+    // Every patch of the mixed path, and the register-kernel patches of the
+    // FP64 path (the others are solved by the LU already).
+    const bool other = mode == kChol || p.n_host[k] <= std::min(nbig, kSmallMax);
+    if ((other && (stat[k] & (kStatusBreakdown | kStatusNonFinite | kStatusTimeout))) ||
         (cached && redo_mark[k]))
       (p.n_host[k] > nbig ? redo_big : redo_small).push_back(k);
   }
@@ -587,18 +635,25 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
     keep->redo_big = redo_big;
   }
   p.patch_status = stat;
-  for (int k : redo_small) p.patch_status[k] |= kStatusResolved;
-  for (int k : redo_big) p.patch_status[k] |= kStatusResolved;
+  if (chol) {
+    for (int k : redo_small) p.patch_status[k] |= kStatusResolved;
+    for (int k : redo_big) p.patch_status[k] |= kStatusResolved;
+  }
   rep.patches_fp64 = int64_t(small.size() + big.size());
   if (!redo_small.empty() || !redo_big.empty()) {
     PB_CUDA(cudaEventRecord(ev0, st));
-    run_list(p, a, kLU, redo_small, rep, st);
+    run_list(p, a, kLU, redo_small, rep, st, nullptr, true);
     solve_big(p, basis, vals_dev, F, true, redo_big, local_dev, p.status.as<int>(), rep, ex);
+    // FP64: the LU is that path's own algorithm, so its status words are the
+    // call's and nothing counts as a fallback.
+    if (!chol)
+      PB_CUDA(cudaMemcpyAsync(p.patch_status.data(), p.status.p, sizeof(int) * K,
+                              cudaMemcpyDeviceToHost, st));
     PB_CUDA(cudaEventRecord(ev1, st));
     PB_CUDA(host_sync(st));
     PB_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
     rep.ms_factor += ms;
-    rep.patches_fallback += int64_t(redo_small.size() + redo_big.size());
+    if (chol) rep.patches_fallback += int64_t(redo_small.size() + redo_big.size());
   }
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
@@ -648,10 +703,17 @@ void solve_adjoint(Plan &p, int basis, int F, const double *h, double *g_out, So
   ex.h = h;
   ex.g_out = g_out;
   solve_big(p, basis, nullptr, F, false, big, nullptr, p.status.as<int>(), rep, ex);
-  // The adjoint has no second path: a pipeline wait that gave up is an error.
+  // The tiled engine has no second path here: a pipeline wait that gave up is
+  // an error.  Register-kernel patches with a non-positive pivot go to the
+  // shared-memory Cholesky.
   std::vector<int> stat(K);
   PB_CUDA(cudaMemcpyAsync(stat.data(), p.status.p, sizeof(int) * K, cudaMemcpyDeviceToHost, st));
   PB_CUDA(host_sync(st));
+  std::vector<int> redo;
+  for (int k : small)
+    if (p.n_host[k] <= kSmallMax && (stat[k] & (kStatusBreakdown | kStatusNonFinite)))
+      redo.push_back(k);
+  run_list(p, a, kAdj, redo, rep, st, nullptr, true);
   for (int k = 0; k < K; ++k)
     if (stat[k] & kStatusTimeout)
       throw Error{PACMAN_B200_ERR_CUDA, "adjoint: a pipeline wait timed out in patch " +
