@@ -693,7 +693,7 @@ int pipeline_wait_limit() {
   return 1 << 22;
 }
 
-void solve_big(Plan &p, int basis, const double *vals, int F, bool lu,
+void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
                const std::vector<int> &patches, double *local, int *status, SolveReport &rep,
                const BigExtra &extra, FactorCache *keep) {
   if (patches.empty()) return;
@@ -729,7 +729,7 @@ void solve_big(Plan &p, int basis, const double *vals, int F, bool lu,
   a.g_out = extra.g_out;
   a.wait_limit = pipeline_wait_limit();
   const bool adjoint = extra.mode == kBigAdjoint;
-  if (adjoint) lu = false;
+  const bool lu = solver == BigSolver::kLU && !adjoint;
   if (!lu) chol_set_smem_attributes();
   // The Cholesky forward path evaluates local = E alpha + V beta from alpha
   // per (patch, source): alpha_out when saving, else a scratch array.
@@ -745,7 +745,7 @@ void solve_big(Plan &p, int basis, const double *vals, int F, bool lu,
   // The forward Cholesky of precision "mixed" runs its column updates on the
   // int8 tensor cores (k_col_step_ws); PACMAN_B200_INT8=0 keeps them in FP64.
   const char *i8env = std::getenv("PACMAN_B200_INT8");
-  const bool oz = !lu && !adjoint && !(i8env && std::atoi(i8env) == 0);
+  const bool oz = solver == BigSolver::kInt8Cholesky && !adjoint && !(i8env && std::atoi(i8env) == 0);
   if (oz) {
     // sigma bounds every |L[r][c]| <= sqrt(A_rr) = sqrt(phi(0)) (1 for the
     // identity padding), with margin for rounding and for d_1 <= 127.

@@ -304,12 +304,12 @@ __device__ __forceinline__ void warp_rows_trsm8_tc(double *rows, const double *s
     for (int q = 0; q < 4; ++q) acc[q] = rows[(rsel + 2 * q) * LDS + cb + col16];
 #pragma unroll 4
     for (int c = 0; c < 16; ++c) {
-      const double d = dinv[cb + c];
+      const double d = dinv[cb + c], ucc = sU[(cb + c) * LDS + cb + c];
       const double u = sU[(cb + c) * LDS + cb + col16];
       const bool own = col16 == c;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const double x = __shfl_sync(0xffffffffu, acc[q], half | c) * d;
+        const double x = quot(__shfl_sync(0xffffffffu, acc[q], half | c), ucc, d);
         acc[q] = own ? x : __fma_rn(-x, u, acc[q]);
       }
     }

@@ -1,5 +1,5 @@
 // Left-looking blocked Cholesky for the large patches of the B200 RBF-PUM
-// transfer (precision "mixed" and the adjoint).
+// transfer (both precisions and the adjoint).
 //
 // The reference factors each patch matrix with an unpivoted LU in one GPU
 // thread (src/rbf_pum/solver/solver.hpp:422-490, KokkosBatched
@@ -112,8 +112,10 @@ __device__ __forceinline__ void sync_all() { __syncthreads(); }
 // 8 h .. 8 h + 7 of row kb + i; column c's entries reach the other lanes by
 // shuffles.  A column-by-column right-looking Cholesky of the block: 1 / L_cc
 // = rsqrt(d_cc) (one operation on the chain of pivots instead of a square
-// root and a reciprocal), L_cc = d_cc / L_cc, L_ic = d_ic (1 / L_cc), d_ij -=
-// L_ic L_jc; dis[kb + c] = 1 / L_cc.  Written without branches (selects; lane
+// root and a reciprocal), L_cc = sqrt(d_cc) and L_ic = d_ic / L_cc from it,
+// each with one residual correction (plain products with 1 / L_cc gave local
+// values 20-50% further from the 64-bit reference on the shell patches), d_ij
+// -= L_ic L_jc; dis[kb + c] = 1 / L_cc.  Written without branches (selects; lane
 // c keeps 1 / L_cc and stores it after the loop) so that the sixteen unrolled
 // steps form one block the compiler can schedule across: FP64 operations
 // and shuffles each take ~25 cycles to complete on this GPU, and a step is a
@@ -131,9 +133,11 @@ __device__ __noinline__ bool warp_chol16(double *D, int ld, int kb, double *dis,
     const double piv = __shfl_sync(0xffffffffu, a[tc], c + 16 * hc);
     ok = ok && piv > 0.0;
     const double rs = rsqrt(piv);
-    const double sc = a[tc] * rs;
+    const double g = piv * rs;
+    const double lcc = __fma_rn(__fma_rn(-g, g, piv), 0.5 * rs, g);
+    const double sc = quot(a[tc], lcc, rs);
     const bool mine = h == hc;
-    a[tc] = mine ? (i == c ? piv * rs : (i > c ? sc : a[tc])) : a[tc];
+    a[tc] = mine ? (i == c ? lcc : (i > c ? sc : a[tc])) : a[tc];
     myrs = lane == c ? rs : myrs;
     const double oth = __shfl_xor_sync(0xffffffffu, a[tc], 16);
     const double lic = mine ? a[tc] : oth;  // L[i][c]
@@ -222,12 +226,12 @@ __device__ bool diag_tile_t(const double *g_in, int ld, double *rg, int rld, int
       for (int q = 0; q < 4; ++q) acc[q] = D[(r0 + rsel + 2 * q) * ld + kb + col16];
 #pragma unroll 4
       for (int c = 0; c < 16; ++c) {
-        const double d = dis[kb + c];
+        const double d = dis[kb + c], lcc = D[(kb + c) * ld + kb + c];
         const double l = D[(kb + col16) * ld + kb + c];  // L_kk[col16][c], used for col16 > c
         const bool own = col16 == c, below = col16 > c;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const double x = __shfl_sync(0xffffffffu, acc[q], half | c) * d;
+          const double x = quot(__shfl_sync(0xffffffffu, acc[q], half | c), lcc, d);
           acc[q] = own ? x : (below ? __fma_rn(-x, l, acc[q]) : acc[q]);
         }
       }

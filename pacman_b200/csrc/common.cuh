@@ -38,6 +38,24 @@ __device__ __forceinline__ double sqdist(const double4 &a, const double4 &b) {
   return sqdist3(a.x, a.y, a.z, b.x, b.y, b.z);
 }
 
+// 1 / d: the hardware's approximation r refined to r (1 + e + e^2), e = 1 - d r
+// (the series of the reciprocal), without branches so that it overlaps other
+// work.  Quotients formed with it are corrected (quot below).
+__device__ __forceinline__ double recip(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  double e = __fma_rn(-d, r, 1.0);
+  e = __fma_rn(e, e, e);
+  return __fma_rn(r, e, r);
+}
+
+// a / d from r ~ 1 / d: one residual correction (Markstein, IBM J. Res. Dev.
+// 34(1), 1990), exact where a = d.
+__device__ __forceinline__ double quot(double a, double d, double r) {
+  const double q = a * r;
+  return __fma_rn(__fma_rn(-q, d, a), r, q);
+}
+
 // Wendland C0..C8 (src/rbf_pum/solver/rbf_functions.hpp:22-150), branch-free
 // with the reference's support mask.  Powers are multiplication chains.
 template <typename T>

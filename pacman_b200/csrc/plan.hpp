@@ -288,6 +288,9 @@ void solve_patches(Plan &p, int basis, const double *vals_dev, int F, int precis
                    double *local_dev, SolveReport &rep, bool save_state = false,
                    bool keep_factors = false);
 
+// Factorisations of the blocked engine: unpivoted LU, Cholesky with FP64
+// updates, Cholesky with split-integer updates (forward only).
+enum class BigSolver { kLU, kCholesky, kInt8Cholesky };
 // Extra inputs / outputs of the blocked engine beyond the forward transfer.
 enum { kBigForward = 0, kBigForwardSave = 1, kBigAdjoint = 2 };
 struct BigExtra {

@@ -137,24 +137,6 @@ __global__ void __launch_bounds__(32)
   a.status[k] = dropped ? kStatusDropped : 0;
 }
 
-// 1 / d: the hardware's approximation r refined to r (1 + e + e^2), e = 1 - d r
-// (the series of the reciprocal), without branches so that it overlaps other
-// work.  Quotients formed with it are corrected (quot below).
-__device__ __forceinline__ double recip(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  double e = __fma_rn(-d, r, 1.0);
-  e = __fma_rn(e, e, e);
-  return __fma_rn(r, e, r);
-}
-
-// a / d from r ~ 1 / d: one residual correction (Markstein, IBM J. Res. Dev.
-// 34(1), 1990), exact where a = d.
-__device__ __forceinline__ double quot(double a, double d, double r) {
-  const double q = a * r;
-  return __fma_rn(__fma_rn(-q, d, a), r, q);
-}
-
 // sqrt(x) for x >= 0 without branches: the hardware's 1 / sqrt(x) and one
 // Goldschmidt step for g ~ sqrt(x), h ~ 1 / (2 sqrt(x)), then the residual
 // correction g + (x - g g) h (Markstein, IBM J. Res. Dev. 34(1), 1990).  Zero

@@ -506,20 +506,24 @@ static void run_small_cached(const FactorCache &c, PatchArgs a, cudaStream_t st)
                       const_cast<double *>(c.small_fac.as<double>()), 2, st);
 }
 
-void solve_big(Plan &p, int basis, const double *vals, int F, bool lu,
+void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
                const std::vector<int> &patches, double *local, int *status, SolveReport &rep,
                const BigExtra &extra, FactorCache *keep = nullptr);
 void solve_big_cached(Plan &p, FactorCache &c, int basis, const double *vals, int F,
                       double *local, int *status, SolveReport &rep, const BigExtra &extra);
 
-// Patches above this size use the blocked engine (blocked.cu): for the
-// Cholesky path the tuned value (64 by default; the register kernels of
-// small.cu take n <= 64), 128 for the LU and adjoint paths.
+// Patches above this size use the blocked engine (blocked.cu): for the mixed
+// path the tuned value, at most kSmallMax (the register kernel's largest
+// patch); 128 for the FP64 and adjoint paths, whose shared-memory kernel is as
+// fast up to there and takes one launch (250k refined points, 685 patches of
+// 65 to 128 sources: 46.7 ms a call with either line; 150k uniform points,
+// 154 such patches, gradients: 7.77 against 7.97 ms with 64).
 // PACMAN_B200_BIG_N overrides both.
 static int big_threshold(int mode) {
   const char *e = std::getenv("PACMAN_B200_BIG_N");
   if (e) return std::max(1, std::atoi(e));
-  return mode == kChol ? std::min(64, std::max(1, tuning_for_current_device().big_n_chol)) : 128;
+  if (mode != kChol) return 128;
+  return std::min(kSmallMax, std::max(1, tuning_for_current_device().big_n_chol));
 }
 
 static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F, int precision,
@@ -572,6 +576,14 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   a.F = F;
   a.dim = p.dim;
   a.basis = basis;
+  // FP64: the reference's LU for the patches of the register kernel and the
+  // shared-memory kernel, the Cholesky with FP64 updates for the tiled ones (A
+  // is symmetric positive definite: half of the LU's work, and the evaluation
+  // rows need no elimination).  250k refined points: 82 -> 42 ms a call.
+  // Relative error against a 64-bit reference, LU -> Cholesky: 120k refined
+  // points C2 4.4e-16 -> 5.1e-16, C4 5.6e-15 -> 7.1e-15; 300k shell points C2
+  // 5.8e-15 -> 4.4e-15, C4 2.5e-13 -> 2.8e-13.  A patch that is not positive
+  // definite in FP64 is solved again by the LU below.
   const int mode = precision == PACMAN_B200_FP64 ? kLU : kChol;
   const int nbig = big_threshold(mode);
   std::vector<int> small, big;
@@ -598,8 +610,8 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
     solve_big_cached(p, *p.fcache, basis, vals_dev, F, local_dev, p.status.as<int>(), rep, ex);
     for (const SmallRange &r : cached->ranges) rep.factors_reused += r.count;
   } else {
-    solve_big(p, basis, vals_dev, F, mode == kLU, big, local_dev, p.status.as<int>(), rep, ex,
-              keep);
+    solve_big(p, basis, vals_dev, F, chol ? BigSolver::kInt8Cholesky : BigSolver::kCholesky, big,
+              local_dev, p.status.as<int>(), rep, ex, keep);
     PB_CUDA(cudaStreamWaitEvent(ss, rep.tail_event, 0));
     run_list(p, a, mode, small, rep, ss, keep);
   }
@@ -623,9 +635,9 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;
     if (stat[k] & kStatusDropped) rep.dropped++;
-    // Every patch of the mixed path, and the register-kernel patches of the
-    // FP64 path (the others are solved by the LU already).
-    const bool other = mode == kChol || p.n_host[k] <= std::min(nbig, kSmallMax);
+    // Every patch that the LU has not solved already (k_patch_solve takes
+    // kSmallMax < n <= nbig of the FP64 path).
+    const bool other = mode == kChol || p.n_host[k] <= kSmallMax || p.n_host[k] > nbig;
     if ((other && (stat[k] & (kStatusBreakdown | kStatusNonFinite | kStatusTimeout))) ||
         (cached && redo_mark[k]))
       (p.n_host[k] > nbig ? redo_big : redo_small).push_back(k);
@@ -643,7 +655,8 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   if (!redo_small.empty() || !redo_big.empty()) {
     PB_CUDA(cudaEventRecord(ev0, st));
     run_list(p, a, kLU, redo_small, rep, st, nullptr, true);
-    solve_big(p, basis, vals_dev, F, true, redo_big, local_dev, p.status.as<int>(), rep, ex);
+    solve_big(p, basis, vals_dev, F, BigSolver::kLU, redo_big, local_dev, p.status.as<int>(), rep,
+              ex);
     // FP64: the LU is that path's own algorithm, so its status words are the
     // call's and nothing counts as a fallback.
     if (!chol)
@@ -702,7 +715,7 @@ void solve_adjoint(Plan &p, int basis, int F, const double *h, double *g_out, So
   ex.mode = kBigAdjoint;
   ex.h = h;
   ex.g_out = g_out;
-  solve_big(p, basis, nullptr, F, false, big, nullptr, p.status.as<int>(), rep, ex);
+  solve_big(p, basis, nullptr, F, BigSolver::kCholesky, big, nullptr, p.status.as<int>(), rep, ex);
   // The tiled engine has no second path here: a pipeline wait that gave up is
   // an error.  Register-kernel patches with a non-positive pivot go to the
   // shared-memory Cholesky.
