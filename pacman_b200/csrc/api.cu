@@ -187,7 +187,7 @@ int create_plan(int32_t dim, const double *src, int64_t n, const double *tgt, in
     if (o.stream) {
       p.stream = static_cast<cudaStream_t>(o.stream);
     } else {
-      PB_CUDA(cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking));
+      p.stream = take_stream(ds.dev);
       p.own_stream = true;
     }
     if (n > 0) {
@@ -391,13 +391,15 @@ struct PlanHandle {
 // streams live until release(), after the plans are gone.
 struct GeometryWorkers {
   std::vector<cudaStream_t> streams;
+  int device = 0;
   int run(const pacman_b200_problem *qs, int32_t count, const pacman_b200_options &o, int dev,
           std::vector<PlanHandle> &plans) {
     int nt = 8;
     if (const char *e = std::getenv("PACMAN_B200_BATCH_THREADS")) nt = std::atoi(e);
     nt = std::max(1, std::min<int>(nt, count));
     streams.assign(size_t(nt), nullptr);
-    for (auto &s : streams) PB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    device = dev;
+    for (auto &s : streams) s = take_stream(dev);
     std::atomic<int> next{0};
     std::atomic<bool> stop{false};
     std::vector<int> rcs(size_t(count), 0);
@@ -426,11 +428,7 @@ struct GeometryWorkers {
     return 0;
   }
   void release() {
-    for (auto s : streams) {
-      if (!s) continue;
-      cudaStreamSynchronize(s);
-      cudaStreamDestroy(s);
-    }
+    for (auto s : streams) give_stream(s, device);
     streams.clear();
   }
   ~GeometryWorkers() { release(); }
@@ -578,7 +576,7 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     DeviceScope ds(o.device);
     o.device = ds.dev;
     if (!o.stream) {
-      PB_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+      own = take_stream(ds.dev);
       o.stream = own;
     }
     cudaStream_t st = static_cast<cudaStream_t>(o.stream);
@@ -600,7 +598,7 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       cudaEventDestroy(e2);
-      if (own) cudaStreamDestroy(own);
+      give_stream(own, ds.dev);
       return rc;
     }
     PB_CUDA(cudaEventRecord(e1, st));
@@ -678,16 +676,10 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     cudaEventDestroy(e2);
     plans.clear();
     gw.release();
-    if (own) {
-      cudaStreamSynchronize(own);
-      cudaStreamDestroy(own);
-      own = nullptr;
-    }
+    give_stream(own, ds.dev);
+    own = nullptr;
   } catch (const Error &e) {
-    if (own) {
-      cudaStreamSynchronize(own);
-      cudaStreamDestroy(own);
-    }
+    give_stream(own, o.device);
     return fail(e.code, e.msg);
   }
   return 0;
@@ -780,10 +772,7 @@ void pacman_b200_plan_destroy(pacman_b200_plan *plan) {
   cudaStream_t st = plan->p.stream;
   const bool own = plan->p.own_stream;
   delete plan;  // frees device buffers stream-ordered on st
-  if (own) {
-    cudaStreamSynchronize(st);
-    cudaStreamDestroy(st);
-  }
+  if (own) give_stream(st, dev);
   if (prev >= 0 && prev != dev) cudaSetDevice(prev);
   cudaGetLastError();
 }
@@ -898,14 +887,16 @@ int pacman_b200_fe_interpolate(int32_t dim, int32_t method, const double *src, i
   if (opts) o = *opts;
   if (m == 0) return 0;
   cudaStream_t own = nullptr;
+  int own_device = 0;
   try {
     DeviceScope ds(o.device);
     tune_pool(ds.dev);
     HostArena::get().reset();
     cudaStream_t st = static_cast<cudaStream_t>(o.stream);
     if (!st) {
-      PB_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+      own = take_stream(ds.dev);
       st = own;
+      own_device = ds.dev;
     }
     {
       InBuf s, v, t;
@@ -931,15 +922,10 @@ int pacman_b200_fe_interpolate(int32_t dim, int32_t method, const double *src, i
                                 st));
       PB_CUDA(host_sync(st));
     }
-    if (own) {
-      cudaStreamDestroy(own);
-      own = nullptr;
-    }
+    give_stream(own, own_device);
+    own = nullptr;
   } catch (const Error &e) {
-    if (own) {
-      cudaStreamSynchronize(own);
-      cudaStreamDestroy(own);
-    }
+    give_stream(own, own_device);
     return fail(e.code, e.msg);
   }
   return 0;
@@ -966,14 +952,16 @@ int pacman_b200_mls_interpolate(int32_t dim, const double *src, int64_t n, const
   if (opts) o = *opts;
   if (m == 0) return 0;
   cudaStream_t own = nullptr;
+  int own_device = 0;
   try {
     DeviceScope ds(o.device);
     tune_pool(ds.dev);
     HostArena::get().reset();
     cudaStream_t st = static_cast<cudaStream_t>(o.stream);
     if (!st) {
-      PB_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+      own = take_stream(ds.dev);
       st = own;
+      own_device = ds.dev;
     }
     {
       InBuf s, v, t;
@@ -993,15 +981,10 @@ int pacman_b200_mls_interpolate(int32_t dim, const double *src, int64_t n, const
                                 st));
       PB_CUDA(host_sync(st));
     }
-    if (own) {
-      cudaStreamDestroy(own);
-      own = nullptr;
-    }
+    give_stream(own, own_device);
+    own = nullptr;
   } catch (const Error &e) {
-    if (own) {
-      cudaStreamSynchronize(own);
-      cudaStreamDestroy(own);
-    }
+    give_stream(own, own_device);
     return fail(e.code, e.msg);
   }
   return 0;

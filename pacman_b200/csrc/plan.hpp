@@ -79,44 +79,43 @@ struct DevGrid {
   DevMem start, items;
 };
 
-// Extra streams of a plan, created on first use on the plan's device: one per
+// Extra streams of a call, taken on first use for the plan's device: one per
 // independent group of large patches (high priority) and one for the small
 // patches (low priority: they fill the SMs the large-patch steps leave idle).
 // Every use joins them back into the plan's stream with events before the
-// call returns.
+// call returns.  Creating and destroying nine streams took 1.2 ms of every
+// call, so a plan's set goes back to a list kept per device (at most
+// kMaxIdle sets; streams.cu), and the next plan on that device, of any thread,
+// takes it from there: whatever the last owner left queued on it (frees) comes
+// first in stream order.
 struct AuxStreams {
   static constexpr int kN = 8;      // slot groups of the large-patch engine (at most)
   static constexpr int kDefaultGroups = 4;  // without a tuned or given count
   static constexpr int kSmall = kN; // index of the small-patch stream
-  cudaStream_t s[kN + 1] = {};
-  cudaEvent_t ev[kN + 3] = {};      // per group, fork, small fork, small join
-  bool made = false;
-  void make() {
-    if (made) return;
-    int least = 0, greatest = 0;
-    if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess)
-      throw Error{PACMAN_B200_ERR_CUDA, "cudaDeviceGetStreamPriorityRange failed"};
-    for (int i = 0; i <= kN; ++i) {
-      if (cudaStreamCreateWithPriority(&s[i], cudaStreamNonBlocking,
-                                       i == kSmall ? least : greatest) != cudaSuccess)
-        throw Error{PACMAN_B200_ERR_CUDA, "cudaStreamCreateWithPriority failed"};
-    }
-    for (int i = 0; i < kN + 3; ++i) {
-      if (cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming) != cudaSuccess)
-        throw Error{PACMAN_B200_ERR_CUDA, "cudaEventCreateWithFlags failed"};
-    }
-    made = true;
-  }
+  static constexpr size_t kMaxIdle = 4;
+  struct Set {
+    cudaStream_t s[kN + 1] = {};
+    cudaEvent_t ev[kN + 3] = {};    // per group, fork, small fork, small join
+    int device = 0;
+  };
+  cudaStream_t *s = nullptr;
+  cudaEvent_t *ev = nullptr;
+  void make();                      // for the current device
   AuxStreams() = default;
   AuxStreams(const AuxStreams &) = delete;
   AuxStreams &operator=(const AuxStreams &) = delete;
-  ~AuxStreams() {
-    for (int i = 0; i <= kN; ++i)
-      if (s[i]) cudaStreamDestroy(s[i]);
-    for (int i = 0; i < kN + 3; ++i)
-      if (ev[i]) cudaEventDestroy(ev[i]);
-  }
+  ~AuxStreams();
+
+ private:
+  Set *set_ = nullptr;
 };
+
+// A stream of the library's own for a call without one, ordered after the
+// work already queued on the legacy default stream (device inputs may still
+// be on their way there).  Kept idle like AuxStreams; give_stream waits for
+// what is queued on it first.
+cudaStream_t take_stream(int device);
+void give_stream(cudaStream_t s, int device);
 
 // Factorisations kept by an execute with PACMAN_B200_KEEP_FACTORS (defined
 // in blocked.cuh; destroyed through destroy_factor_cache).

@@ -598,25 +598,32 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   // Small patches on the low-priority stream, started where the large-patch
   // steps stop filling the GPU (the engine re-records the event there; with
   // no large patches it stays at this point of the plan's stream).
-  p.aux.make();
-  cudaStream_t ss = p.aux.s[AuxStreams::kSmall];
-  rep.tail_event = p.aux.ev[AuxStreams::kN + 1];
-  PB_CUDA(cudaEventRecord(rep.tail_event, st));
+  // Without large patches nothing runs beside them: the plan's own stream.
+  const bool beside = !big.empty();
+  cudaStream_t ss = st;
+  if (beside) {
+    p.aux.make();
+    ss = p.aux.s[AuxStreams::kSmall];
+    rep.tail_event = p.aux.ev[AuxStreams::kN + 1];
+    PB_CUDA(cudaEventRecord(rep.tail_event, st));
+  }
   if (cached) {
     // Kept factors: the small patches start at once (no factorisation steps
     // to wait for), the large ones run their sweeps on the group streams.
-    PB_CUDA(cudaStreamWaitEvent(ss, rep.tail_event, 0));
+    if (beside) PB_CUDA(cudaStreamWaitEvent(ss, rep.tail_event, 0));
     run_small_cached(*cached, a, ss);
     solve_big_cached(p, *p.fcache, basis, vals_dev, F, local_dev, p.status.as<int>(), rep, ex);
     for (const SmallRange &r : cached->ranges) rep.factors_reused += r.count;
   } else {
     solve_big(p, basis, vals_dev, F, chol ? BigSolver::kInt8Cholesky : BigSolver::kCholesky, big,
               local_dev, p.status.as<int>(), rep, ex, keep);
-    PB_CUDA(cudaStreamWaitEvent(ss, rep.tail_event, 0));
+    if (beside) PB_CUDA(cudaStreamWaitEvent(ss, rep.tail_event, 0));
     run_list(p, a, mode, small, rep, ss, keep);
   }
-  PB_CUDA(cudaEventRecord(p.aux.ev[AuxStreams::kN + 2], ss));
-  PB_CUDA(cudaStreamWaitEvent(st, p.aux.ev[AuxStreams::kN + 2], 0));
+  if (beside) {
+    PB_CUDA(cudaEventRecord(p.aux.ev[AuxStreams::kN + 2], ss));
+    PB_CUDA(cudaStreamWaitEvent(st, p.aux.ev[AuxStreams::kN + 2], 0));
+  }
   rep.tail_event = nullptr;
   std::vector<int> stat(K);
   PB_CUDA(cudaMemcpyAsync(stat.data(), p.status.p, sizeof(int) * K, cudaMemcpyDeviceToHost, st));
