@@ -130,7 +130,8 @@ __device__ __forceinline__ void mls_sweep(double *a, double *u, double *v) {
 
 template <int DIM>
 __global__ void __launch_bounds__(128) k_mls(int64_t M, const double4 *__restrict__ tgt,
-                                             GridView g, double h,
+                                             GridView g,
+                                             const double4 *__restrict__ sorted, double h,
                                              const double4 *__restrict__ src,
                                              const double *__restrict__ vals, int64_t n,
                                              double *__restrict__ out) {
@@ -153,8 +154,8 @@ __global__ void __launch_bounds__(128) k_mls(int64_t M, const double4 *__restric
     }
     auto scan = [&](int s, int e) {
       for (int i = s; i < e; ++i) {
-        const int id = g.items[i];
-        const double4 x = src[id];
+        const double4 x = sorted[i];
+        const int id = int(x.w);
         const double d2 = sqdist3(y.x, y.y, y.z, x.x, x.y, x.z);
         if (!(d2 < bd[K - 1] || (d2 == bd[K - 1] && id < bi[K - 1]))) continue;
         bd[K - 1] = d2;
@@ -268,27 +269,18 @@ void mls_interpolate(int dim, const double *src_dev, int64_t n, const double *va
     PB_CUDA(cudaMemsetAsync(out_dev, 0, sizeof(double) * size_t(m), st));
     return;
   }
-  DevMem src4, tgt4;
-  double lo[3], hi[3], tlo[3], thi[3];
-  pack_points(src_dev, dim, n, src4, lo, hi, st);
-  pack_points(tgt_dev, dim, m, tgt4, tlo, thi, st);
-  // About one source per cell: the largest extent over n^(1/dim) cells.
-  double ext = 0.0;
-  for (int d = 0; d < dim; ++d) ext = std::max(ext, hi[d] - lo[d]);
-  const double per_axis = std::ceil(std::pow(double(n), 1.0 / dim));
-  const double cell = ext > 0.0 ? ext / per_axis : 1.0;
-  DevGrid grid;
-  build_point_grid(grid, src4.as<double4>(), n, dim, lo, hi, cell, st);
-  const double h = 1.0 / grid.view.inv_h;
+  PointSearch ps;
+  build_point_search(ps, dim, src_dev, n, tgt_dev, m, st);
+  const double h = 1.0 / ps.grid.inv_h;
   const int blocks = int(std::max<int64_t>(1, std::min<int64_t>((m + 127) / 128, 148 * 16)));
   if (dim == 1)
-    k_mls<1><<<blocks, 128, 0, st>>>(m, tgt4.as<double4>(), grid.view, h, src4.as<double4>(),
+    k_mls<1><<<blocks, 128, 0, st>>>(m, ps.tgt4.as<double4>(), ps.grid, ps.sorted, h, ps.src4.as<double4>(),
                                      vals_dev, n, out_dev);
   else if (dim == 2)
-    k_mls<2><<<blocks, 128, 0, st>>>(m, tgt4.as<double4>(), grid.view, h, src4.as<double4>(),
+    k_mls<2><<<blocks, 128, 0, st>>>(m, ps.tgt4.as<double4>(), ps.grid, ps.sorted, h, ps.src4.as<double4>(),
                                      vals_dev, n, out_dev);
   else
-    k_mls<3><<<blocks, 128, 0, st>>>(m, tgt4.as<double4>(), grid.view, h, src4.as<double4>(),
+    k_mls<3><<<blocks, 128, 0, st>>>(m, ps.tgt4.as<double4>(), ps.grid, ps.sorted, h, ps.src4.as<double4>(),
                                      vals_dev, n, out_dev);
   note_launch();
   PB_CUDA(cudaGetLastError());

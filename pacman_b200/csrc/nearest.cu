@@ -22,8 +22,9 @@ namespace {
 // away, one cell less with a source that rounding put into the neighbouring
 // cell: the scan stops once the best squared distance is below ((R - 1) h)^2.
 // The shells are bounded by the grid, so the loop ends.
-__global__ void k_fe_nearest(int64_t M, const double4 *__restrict__ tgt, GridView g, double h,
-                             const double4 *__restrict__ src, const double *__restrict__ vals,
+__global__ void k_fe_nearest(int64_t M, const double4 *__restrict__ tgt, GridView g,
+                             const double4 *__restrict__ sorted, double h,
+                             const double *__restrict__ vals,
                              double *__restrict__ out) {
   const int rmax = max(g.nc[0], max(g.nc[1], g.nc[2]));
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < M;
@@ -36,8 +37,8 @@ __global__ void k_fe_nearest(int64_t M, const double4 *__restrict__ tgt, GridVie
     int bi = -1;
     auto scan = [&](int s, int e) {
       for (int i = s; i < e; ++i) {
-        const int id = g.items[i];
-        const double4 x = src[id];
+        const double4 x = sorted[i];
+        const int id = int(x.w);
         const double d2 = sqdist3(y.x, y.y, y.z, x.x, x.y, x.z);
         if (bi < 0 || d2 < best || (d2 == best && id < bi)) {
           best = d2;
@@ -78,21 +79,12 @@ void fe_nearest(int dim, const double *src_dev, int64_t n, const double *vals_de
     PB_CUDA(cudaMemsetAsync(out_dev, 0, sizeof(double) * size_t(m), st));
     return;
   }
-  DevMem src4, tgt4;
-  double lo[3], hi[3], tlo[3], thi[3];
-  pack_points(src_dev, dim, n, src4, lo, hi, st);
-  pack_points(tgt_dev, dim, m, tgt4, tlo, thi, st);
-  // About one source per cell: the largest extent over n^(1/dim) cells.
-  double ext = 0.0;
-  for (int d = 0; d < dim; ++d) ext = std::max(ext, hi[d] - lo[d]);
-  const double per_axis = std::ceil(std::pow(double(n), 1.0 / dim));
-  const double cell = ext > 0.0 ? ext / per_axis : 1.0;
-  DevGrid grid;
-  build_point_grid(grid, src4.as<double4>(), n, dim, lo, hi, cell, st);
-  const double h = 1.0 / grid.view.inv_h;
+  PointSearch ps;
+  build_point_search(ps, dim, src_dev, n, tgt_dev, m, st);
+  const double h = 1.0 / ps.grid.inv_h;
   const int blocks = int(std::max<int64_t>(1, std::min<int64_t>((m + 127) / 128, 148 * 32)));
-  k_fe_nearest<<<blocks, 128, 0, st>>>(m, tgt4.as<double4>(), grid.view, h,
-                                       src4.as<double4>(), vals_dev, out_dev);
+  k_fe_nearest<<<blocks, 128, 0, st>>>(m, ps.tgt4.as<double4>(), ps.grid, ps.sorted, h, vals_dev,
+                                       out_dev);
   note_launch();
   PB_CUDA(cudaGetLastError());
   PB_CUDA(host_sync(st));

@@ -237,12 +237,15 @@ void build_geometry(Plan &p, const double *src_dev, const double *tgt_dev);
 // stream has passed them (callers have synchronised it), then cached.
 double geometry_ms(Plan &p);
 void pu_gather(Plan &p, const double *local, int F, double *out_dev);
-// Packed double4 points with their exact bounding box, and the uniform cell
-// grid over them (geometry.cu; used by nearest.cu).
-void pack_points(const double *in_dev, int dim, int64_t n, DevMem &out4, double lo[3],
-                 double hi[3], cudaStream_t st);
-void build_point_grid(DevGrid &out, const double4 *pts, int64_t n, int dim, const double *lo,
-                      const double *hi, double cell, cudaStream_t st);
+// Packed points of a nearest-neighbour search: the sources sorted into a
+// uniform grid of about one source per cell, their ids in w (geometry.cu).
+struct PointSearch {
+  DevMem src4, tgt4, mem;
+  GridView grid{};               // start only
+  const double4 *sorted = nullptr;
+};
+void build_point_search(PointSearch &ps, int dim, const double *src_dev, int64_t n,
+                        const double *tgt_dev, int64_t m, cudaStream_t st);
 // Finite-element NEAREST_NEAREST transfer (nearest.cu).
 void fe_nearest(int dim, const double *src_dev, int64_t n, const double *vals_dev,
                 const double *tgt_dev, int64_t m, double *out_dev, cudaStream_t st);
