@@ -431,6 +431,7 @@ struct GridSpec {
   double inv_h;
   int nc[3];
   int ncells;
+  int clamp;     // points outside the domain go to the nearest cell
 };
 
 GridSpec make_grid_spec(int dim, const double *bb_lo, const double *bb_hi, double radius,
@@ -478,7 +479,7 @@ GridSpec make_grid_spec(int dim, const double *bb_lo, const double *bb_hi, doubl
 __device__ __forceinline__ int cell_of(const GridSpec &g, const double4 &p) {
   const double c[3] = {p.x, p.y, p.z};
   for (int d = 0; d < 3; ++d)
-    if (!(c[d] >= g.lo[d] && c[d] <= g.hi[d])) return -1;
+    if (!g.clamp && !(c[d] >= g.lo[d] && c[d] <= g.hi[d])) return -1;
   const int a = cell_coord(c[0], g.lo[0], g.inv_h, g.nc[0]);
   const int b = cell_coord(c[1], g.lo[1], g.inv_h, g.nc[1]);
   const int e = cell_coord(c[2], g.lo[2], g.inv_h, g.nc[2]);
@@ -1361,10 +1362,11 @@ double geometry_ms(Plan &p) {
   return p.ms_geometry < 0.0 ? 0.0 : p.ms_geometry;
 }
 
-// Both point sets packed, and the sources sorted into about one cell each for
-// the nearest-neighbour searches of nearest.cu and mls.cu.
+// Both point sets packed and sorted into the cells of the sources' grid, for
+// the nearest-neighbour searches of nearest.cu and mls.cu.  `scale` is the
+// cell's edge relative to one source per cell of a uniform cloud.
 void build_point_search(PointSearch &ps, int dim, const double *src_dev, int64_t n,
-                        const double *tgt_dev, int64_t m, cudaStream_t st) {
+                        const double *tgt_dev, int64_t m, double scale, cudaStream_t st) {
   DevMem scm;
   scm.alloc(sizeof(GeoScratch), st);
   GeoScratch *sc = scm.as<GeoScratch>();
@@ -1389,18 +1391,20 @@ void build_point_search(PointSearch &ps, int dim, const double *src_dev, int64_t
     hi[d] = to_dbl(h[3 + d]);
     ext = std::max(ext, hi[d] - lo[d]);
   }
-  // About one source per cell: the largest extent over n^(1/dim) cells.
   const double per_axis = std::ceil(std::pow(double(n), 1.0 / dim));
-  const double cell = ext > 0.0 ? ext / per_axis : 1.0;
+  const double cell = ext > 0.0 ? scale * (ext / per_axis) : 1.0;
   const GridSpec g = make_grid_spec(dim, lo, hi, cell, n);
+  GridSpec gt = g;
+  gt.clamp = 1;
   Slab slab;
-  GridView none{};
+  GridView tv{};
   for (int pass = 0; pass < 2; ++pass) {
     if (pass) {
       ps.mem.alloc(slab.used, st);
       slab = Slab{ps.mem.as<char>(), 0};
     }
-    sort_into_cells(slab, ps.src4.as<double4>(), n, g, nullptr, 0, g, ps.grid, none, ps.sorted, st);
+    sort_into_cells(slab, ps.src4.as<double4>(), n, g, ps.tgt4.as<double4>(), m, gt, ps.grid, tv,
+                    ps.sorted, st);
   }
 }
 

@@ -12,61 +12,37 @@
 #include <cmath>
 
 #include "plan.hpp"
+#include "search.cuh"
 
 namespace pacman_b200 {
 
 namespace {
 
-// One thread per target.  After shell R (cells at Chebyshev cell distance R
-// from the target's cell) every unscanned source lies at least R cell widths
-// away, one cell less with a source that rounding put into the neighbouring
-// cell: the scan stops once the best squared distance is below ((R - 1) h)^2.
-// The shells are bounded by the grid, so the loop ends.
-__global__ void k_fe_nearest(int64_t M, const double4 *__restrict__ tgt, GridView g,
-                             const double4 *__restrict__ sorted, double h,
-                             const double *__restrict__ vals,
-                             double *__restrict__ out) {
-  const int rmax = max(g.nc[0], max(g.nc[1], g.nc[2]));
+// One thread per target, in cell order: the threads of a warp scan the same few
+// cells, which then come from L1, and run equally long.  1M refined sources ->
+// 1M uniform targets: 0.40 ms, against 3.9 ms in the caller's order with a
+// bound of R - 1 cell widths after shell R (always 5^3 cells or more).
+template <int DIM>
+__global__ void k_fe_nearest(int64_t M, GridView g, const double4 *__restrict__ sorted, double h,
+                             const double *__restrict__ vals, double *__restrict__ out) {
+  const double4 *tgt = sorted + g.start[g.ncells];
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < M;
        t += int64_t(gridDim.x) * blockDim.x) {
     const double4 y = tgt[t];
-    const int cx = cell_coord(y.x, g.lo[0], g.inv_h, g.nc[0]);
-    const int cy = cell_coord(y.y, g.lo[1], g.inv_h, g.nc[1]);
-    const int cz = cell_coord(y.z, g.lo[2], g.inv_h, g.nc[2]);
-    double best = 0.0;
+    double best = INFINITY;
     int bi = -1;
-    auto scan = [&](int s, int e) {
-      for (int i = s; i < e; ++i) {
-        const double4 x = sorted[i];
-        const int id = int(x.w);
-        const double d2 = sqdist3(y.x, y.y, y.z, x.x, x.y, x.z);
-        if (bi < 0 || d2 < best || (d2 == best && id < bi)) {
-          best = d2;
-          bi = id;
-        }
-      }
-    };
-    for (int R = 0; R <= rmax; ++R) {
-      const int x0 = max(cx - R, 0), x1 = min(cx + R, g.nc[0] - 1);
-      const int y0 = max(cy - R, 0), y1 = min(cy + R, g.nc[1] - 1);
-      for (int a = x0; a <= x1; ++a)
-        for (int b = y0; b <= y1; ++b) {
-          const int base = (a * g.nc[1] + b) * g.nc[2];
-          const bool face = a == cx - R || a == cx + R || b == cy - R || b == cy + R;
-          if (face) {  // the whole z run of this column is on the shell
-            const int z0 = max(cz - R, 0), z1 = min(cz + R, g.nc[2] - 1);
-            scan(g.start[base + z0], g.start[base + z1 + 1]);
-          } else {  // only its two ends
-            if (cz - R >= 0) scan(g.start[base + cz - R], g.start[base + cz - R + 1]);
-            if (cz + R < g.nc[2]) scan(g.start[base + cz + R], g.start[base + cz + R + 1]);
+    scan_shells<DIM>(
+        g, sorted, h, y,
+        [&](const double4 &x) {
+          const int id = int(x.w);
+          const double d2 = sqdist3(y.x, y.y, y.z, x.x, x.y, x.z);
+          if (bi < 0 || d2 < best || (d2 == best && id < bi)) {
+            best = d2;
+            bi = id;
           }
-        }
-      if (bi >= 0 && R >= 1) {
-        const double lim = double(R - 1) * h;
-        if (best < lim * lim) break;
-      }
-    }
-    out[t] = bi >= 0 ? vals[bi] : 0.0;
+        },
+        [&] { return bi < 0 ? INFINITY : best; });
+    out[int(y.w)] = bi >= 0 ? vals[bi] : 0.0;
   }
 }
 
@@ -80,11 +56,15 @@ void fe_nearest(int dim, const double *src_dev, int64_t n, const double *vals_de
     return;
   }
   PointSearch ps;
-  build_point_search(ps, dim, src_dev, n, tgt_dev, m, st);
+  build_point_search(ps, dim, src_dev, n, tgt_dev, m, 1.0, st);
   const double h = 1.0 / ps.grid.inv_h;
-  const int blocks = int(std::max<int64_t>(1, std::min<int64_t>((m + 127) / 128, 148 * 32)));
-  k_fe_nearest<<<blocks, 128, 0, st>>>(m, ps.tgt4.as<double4>(), ps.grid, ps.sorted, h, vals_dev,
-                                       out_dev);
+  const int blocks = int(std::max<int64_t>(1, std::min<int64_t>((m + 127) / 128, 148 * 64)));
+  auto go = [&](auto kernel) {
+    kernel<<<blocks, 128, 0, st>>>(m, ps.grid, ps.sorted, h, vals_dev, out_dev);
+  };
+  if (dim == 1) go(k_fe_nearest<1>);
+  else if (dim == 2) go(k_fe_nearest<2>);
+  else go(k_fe_nearest<3>);
   note_launch();
   PB_CUDA(cudaGetLastError());
   PB_CUDA(host_sync(st));

@@ -237,15 +237,16 @@ void build_geometry(Plan &p, const double *src_dev, const double *tgt_dev);
 // stream has passed them (callers have synchronised it), then cached.
 double geometry_ms(Plan &p);
 void pu_gather(Plan &p, const double *local, int F, double *out_dev);
-// Packed points of a nearest-neighbour search: the sources sorted into a
-// uniform grid of about one source per cell, their ids in w (geometry.cu).
+// Packed points of a nearest-neighbour search, sorted into the cells of a
+// uniform grid over the sources with their ids in w: the sources, then from
+// grid.start[grid.ncells] on the targets (geometry.cu).
 struct PointSearch {
   DevMem src4, tgt4, mem;
   GridView grid{};               // start only
   const double4 *sorted = nullptr;
 };
 void build_point_search(PointSearch &ps, int dim, const double *src_dev, int64_t n,
-                        const double *tgt_dev, int64_t m, cudaStream_t st);
+                        const double *tgt_dev, int64_t m, double scale, cudaStream_t st);
 // Finite-element NEAREST_NEAREST transfer (nearest.cu).
 void fe_nearest(int dim, const double *src_dev, int64_t n, const double *vals_dev,
                 const double *tgt_dev, int64_t m, double *out_dev, cudaStream_t st);

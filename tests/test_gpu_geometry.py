@@ -83,3 +83,34 @@ def test_no_targets():
     rng = np.random.default_rng(6)
     S = rng.random((3000, 3))
     _same(3, S, np.zeros((0, 3)), 30)
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_point_searches_at_cell_faces_and_outside(dim):
+    # Sources and targets on the faces and corners of the search grid's cells,
+    # targets far outside, fewer sources than one shell.
+    rng = np.random.default_rng(dim)
+    for n in (3, 64, 4096):
+        side = int(round(n ** (1.0 / dim)))
+        g = np.arange(side) / max(side, 1)
+        S = np.stack(np.meshgrid(*([g] * dim), indexing="ij"), -1).reshape(-1, dim)
+        T = np.concatenate([S, S + 0.5 / side, S[:50] - 3.0, S[:50] + 7.5,
+                            rng.random((200, dim))])
+        v = np.cos(S @ np.arange(1.0, dim + 1))
+        out, _ = pacman.fe.interpolate(dim, pacman.execspaces.CUDA,
+                                       pacman.fe.methods.NEAREST_NEAREST, S, v, None, None, None, T)
+        assert np.array_equal(out, oracle.fe_nearest(dim, S, v, T)[0])
+        mls = pacman.mls.interpolate(dim, pacman.execspaces.CUDA, S, v, T)
+        assert np.array_equal(mls, oracle.mls_interpolate(dim, S, v, T, knn="brute"))
+
+
+def test_mls_target_chunks():
+    # More targets than one chunk of neighbour ids holds.
+    rng = np.random.default_rng(3)
+    S, T = rng.random((700, 1)), rng.random(((1 << 22) + 1001, 1))
+    v = np.sin(5 * S[:, 0])
+    out = pacman.mls.interpolate(1, pacman.execspaces.CUDA, S, v, T)
+    pick = np.r_[0:2000, (1 << 22) - 500:len(T)]
+    assert np.array_equal(out[pick], oracle.mls_interpolate(1, S, v, T[pick]))
+    near = rng.choice(len(T), 20000, replace=False)
+    assert np.array_equal(out[near], oracle.mls_interpolate(1, S, v, T[near]))
