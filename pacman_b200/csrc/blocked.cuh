@@ -227,52 +227,53 @@ __device__ __forceinline__ void warp_rows_trsm8(double *rows, const double *sU,
 // The blocks of U_jj are at most as ill-conditioned as U_jj (cond(U_bb) <=
 // cond(U_jj)), and the blocked solve stays backward stable blockwise.  No
 // shuffles (a 64-bit shuffle costs two of the SM's one-per-clock shuffle
-// slots): operands come from shared memory.  With up, the right-hand side is C =
-// rows - sig2 up (one rounding), formed first.
-__device__ __forceinline__ void warp_rows_trsm8_bi(double *rows, const double *sU,
-                                                   const double *sUi, int lane,
-                                                   const double *up, double sig2) {
+// slots): operands come from shared memory.
+// On return c holds the solution in the accumulator layout (lane: row g =
+// lane / 4, columns 8 nt + 2 t, + 1 with t = lane % 4); with kStore the rows
+// hold it as well, else they are scratch.
+template <bool kStore>
+__device__ __forceinline__ void warp_rows_solve8(double *rows, const double *sU, const double *sUi,
+                                                 int lane, double (&c)[8][2]) {
   const int g = lane >> 2, t = lane & 3;
   // The warp's 8 x 64 right-hand side stays in registers in the tensor
-  // cores' accumulator layout (lane: row g, columns 8 nt + 2 t, + 1); only
-  // the 8 x 16 block being solved goes through shared memory, once to be
-  // read as the products' A operand and once as the result.
-  double c[8][2];
+  // cores' accumulator layout; only the 8 x 16 block being solved goes through
+  // shared memory, once to be read as the products' A operand and once as the
+  // result.
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int o = g * LDS + 8 * nt + 2 * t + e;
-      c[nt][e] = up ? __fma_rn(-sig2, up[o], rows[o]) : rows[o];
-    }
+    *reinterpret_cast<double2 *>(c[nt]) =
+        *reinterpret_cast<const double2 *>(rows + g * LDS + 8 * nt + 2 * t);
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int cb = 16 * b;
+    if (b > 0) {  // block 0 is in the rows as it was read
+      __syncwarp();
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      rows[g * LDS + cb + 8 * h + 2 * t] = c[2 * b + h][0];
-      rows[g * LDS + cb + 8 * h + 2 * t + 1] = c[2 * b + h][1];
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<double2 *>(rows + g * LDS + cb + 8 * h + 2 * t) =
+            make_double2(c[2 * b + h][0], c[2 * b + h][1]);
     }
     __syncwarp();
     double af[4];
 #pragma unroll
     for (int k4 = 0; k4 < 4; ++k4) af[k4] = rows[g * LDS + cb + 4 * k4 + t];
-    // X_b = R_b Ui_b, two 8-column halves.
-    double x[2][2];
+    // X_b = R_b Ui_b, two 8-column halves; Ui_b is upper triangular, so the
+    // left half needs its first eight rows only.
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       double c0 = 0.0, c1 = 0.0;
 #pragma unroll
-      for (int k4 = 0; k4 < 4; ++k4)
+      for (int k4 = 0; k4 < 2 * h + 2; ++k4)
         dmma(c0, c1, af[k4], sUi[(cb + 4 * k4 + t) * kUiLd + 8 * h + g]);
-      x[h][0] = c0;
-      x[h][1] = c1;
+      c[2 * b + h][0] = c0;
+      c[2 * b + h][1] = c1;
     }
-    __syncwarp();
+    if (kStore || b < 3) {
+      __syncwarp();
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      rows[g * LDS + cb + 8 * h + 2 * t] = x[h][0];
-      rows[g * LDS + cb + 8 * h + 2 * t + 1] = x[h][1];
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<double2 *>(rows + g * LDS + cb + 8 * h + 2 * t) =
+            make_double2(c[2 * b + h][0], c[2 * b + h][1]);
     }
     if (b < 3) {
       __syncwarp();
@@ -286,7 +287,7 @@ __device__ __forceinline__ void warp_rows_trsm8_bi(double *rows, const double *s
           dmma(c[nt][0], c[nt][1], af[k4], sU[(cb + 4 * k4 + t) * LDS + 8 * nt + g]);
     }
   }
-  __syncwarp();
+  if (kStore) __syncwarp();
 }
 
 // warp_rows_trsm8 with the off-diagonal block products on the FP64 tensor
@@ -415,7 +416,8 @@ struct CholPlan {
 };
 CholPlan chol_prefix(const std::vector<BigSlot> &slots);
 void chol_set_smem_attributes();
-// Bytes of int8 slice tiles of a slot with T tile rows (strictly lower tiles).
+// Bytes of int8 slice tiles of a slot with T tile rows (strictly lower tiles,
+// plain and in row pairs).
 size_t oz_slot_bytes(int T);
 // tail_event (or null) is recorded on st at the first step that leaves SMs
 // idle (fewer than two CTAs per SM), else after the last step.

@@ -287,7 +287,10 @@ __device__ bool diag_tile_t(const double *g_in, int ld, double *rg, int rld, int
   for (int e = tid; e < TB * TB; e += 256) D[(e >> 6) * ld + (e & 63)] = (e >> 6) == (e & 63);
   sync();
   if (kTensorSolve) warp_rows_trsm8_tc(D + 8 * warp * ld, Us, dis, lane);
-  else if (blockinv) warp_rows_trsm8_bi(D + 8 * warp * ld, Us, ui, lane, nullptr, 0.0);
+  else if (blockinv) {
+    double x[8][2];
+    warp_rows_solve8<true>(D + 8 * warp * ld, Us, ui, lane, x);
+  }
   else warp_rows_trsm8(D + 8 * warp * ld, Us, dis, lane);
   sync();
   // X (row-major, gi) and y = X r.
@@ -473,7 +476,9 @@ __device__ void step_trsm(const BigArgs &a, const BigSlot &sl, int j, int i0, in
 //
 // Slice tile layout (28 KB): [16-byte K chunk (4)][slice (kOzS)][8-row group
 // (8)][8 rows x 16 bytes], i.e. the K-major core-matrix layout of the tensor
-// core, copied to shared memory with bulk async copies.
+// core, copied to shared memory with bulk async copies.  Every tile is written
+// twice: by itself, and interleaved slice by slice with the other tile of its
+// row pair (16 row groups per slice).
 constexpr int kOzS = 7;
 constexpr int kOzTileBytes = 4 * kOzS * 8 * 128;      // 28672
 constexpr int kOzTmemCols = 512;                      // 8 column groups of 64 (levels 2..9)
@@ -565,40 +570,115 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 }
 
-// The int8 digits of rows [0, nrows) of L tiles held in shared memory (row
-// stride LDS; rows 64.. belong to the second tile) straight into their slice
-// tiles in global memory (dst0: the tile of rows 0..63, dst1: rows 64..127).
-// A thread unit is (row, 16-column K chunk): it builds the 16 bytes of each of
-// the kOzS slices and stores each as one 16-byte word, consecutive units of a
-// warp writing consecutive words.  Digits: y = round(x 128^kOzS) as an
-// integer (x = L mul / 128 in [-1, 1]); balanced base-128 digits from the top,
-// d = round(y / 128^(kOzS-1-s)), y -= d 128^(kOzS-1-s).
-__device__ void slice_tile_smem(const double *sL, int nrows, double mul, uint8_t *dst0,
-                                uint8_t *dst1, int tid, int nt) {
-  for (int u = tid; u < nrows * 4; u += nt) {
-    const int r = (u & 63) + 64 * (u >> 8), c16 = (u >> 6) & 3;
-    uint32_t w[kOzS][4];
+// Slice storage of a slot with T tile rows, in bytes from its sli: first the
+// plain tiles of the strictly lower triangle, row by row (operand B: the
+// column tile row's slices stacked along N), then the pair tiles, the rows
+// 2u and 2u + 1 interleaved per slice (operand A: M = 128), pair u with its
+// 2u + 1 columns.
+constexpr int kOzPairBytes = 2 * kOzTileBytes;
+__host__ __device__ __forceinline__ int64_t oz_tile_off(int i, int p) {
+  return (int64_t(i) * (i - 1) / 2 + p) * kOzTileBytes;
+}
+__host__ __device__ __forceinline__ int64_t oz_pair_off(int T, int u, int p) {
+  return int64_t(T) * (T - 1) / 2 * kOzTileBytes + (int64_t(u) * u + p) * kOzPairBytes;
+}
+
+// The kOzS balanced base-128 digits of x = v mul / 128 in [-1, 1]: y = x
+// 128^kOzS rounded to an integer (in the low bits of a double at 1.5 2^52),
+// plus 64 in each of the lower digits, is a row of unsigned 7-bit fields f with
+// d = f - 64 and a signed top digit in [-127, 127].  bytes[s] |= the field of
+// digit s, shifted; oz_bytes turns four fields into four int8 digits.
+__device__ __forceinline__ void oz_fields(double v, double mul, int shift, uint32_t *bytes) {
+  constexpr double kOne = 0x1.8p52, kMax = 127.49 * 0x1p42;
+  constexpr long long kBias = 64ll * (1 + (1ll << 7) + (1ll << 14) + (1ll << 21) + (1ll << 28) +
+                                      (1ll << 35));
+  double t = __fma_rn(v, mul * 0x1p42, kOne);
+  t = fmin(fmax(t, kOne - kMax), kOne + kMax);
+  const long long y = __double_as_longlong(t) - __double_as_longlong(kOne) + kBias;
+  const uint32_t lo = uint32_t(y), hi = uint32_t(uint64_t(y) >> 32);
+  const uint32_t f[kOzS] = {hi >> 10,          hi >> 3,  __funnelshift_r(lo, hi, 28),
+                            lo >> 21,          lo >> 14, lo >> 7,
+                            lo};
+  bytes[0] |= (f[0] & 0xffu) << shift;
 #pragma unroll
-    for (int sl = 0; sl < kOzS; ++sl)
+  for (int s = 1; s < kOzS; ++s) bytes[s] |= (f[s] & 0x7fu) << shift;
+}
+// Four 7-bit fields -> four int8 values field - 64.
+__device__ __forceinline__ uint32_t oz_bytes(uint32_t f) {
+  const uint32_t r = f ^ 0x40404040u;
+  return r | ((r & 0x40404040u) << 1);
+}
+// Stores the 16-byte word of every slice of row r (0..63), K chunk c16 of
+// L[i, p] in the plain and the pair tile.
+__device__ __forceinline__ void oz_store(const uint4 (&w)[kOzS], int r, int c16, uint8_t *slices,
+                                         int T, int i, int p) {
+  uint8_t *tile = slices + oz_tile_off(i, p) + c16 * kOzS * 1024 + r * 16;
+  uint8_t *pair = slices + oz_pair_off(T, i >> 1, p) + c16 * kOzS * 2048 + (i & 1) * 1024 + r * 16;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[sl][q] = 0u;
-#pragma unroll
-    for (int cc = 0; cc < 16; ++cc) {
-      const double xs = fmin(fmax(sL[r * LDS + 16 * c16 + cc] * mul, -127.49), 127.49);
-      long long y = __double2ll_rn(xs * 0x1p42);  // x * 128 * 128^(kOzS-1)
-#pragma unroll
-      for (int sl = 0; sl < kOzS; ++sl) {
-        const int sh = 7 * (kOzS - 1 - sl);
-        const long long d = sh ? ((y + (1ll << (sh - 1))) >> sh) : y;
-        y -= d << sh;
-        w[sl][cc >> 2] |= uint32_t(uint8_t(int8_t(d))) << (8 * (cc & 3));
-      }
-    }
-    uint8_t *dst = (r < 64 ? dst0 : dst1) + c16 * kOzS * 1024 + (r & 63) * 16;
-#pragma unroll
-    for (int sl = 0; sl < kOzS; ++sl)
-      *reinterpret_cast<uint4 *>(dst + sl * 1024) = make_uint4(w[sl][0], w[sl][1], w[sl][2], w[sl][3]);
+  for (int sl = 0; sl < kOzS; ++sl) {
+    *reinterpret_cast<uint4 *>(tile + sl * 1024) = w[sl];
+    *reinterpret_cast<uint4 *>(pair + sl * 2048) = w[sl];
   }
+}
+
+// The digits of row r (0..63) and 16-column K chunk c16 of L[i, p], held in
+// shared memory at sL (row stride LDS).
+__device__ __forceinline__ void slice_row_chunk(const double *sL, int r, int c16, double mul,
+                                                uint8_t *slices, int T, int i, int p) {
+  uint4 w[kOzS];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint32_t b[kOzS] = {};
+#pragma unroll
+    for (int cc = 0; cc < 4; ++cc)
+      oz_fields(sL[r * LDS + 16 * c16 + 4 * q + cc], mul, 8 * cc, b);
+#pragma unroll
+    for (int sl = 0; sl < kOzS; ++sl) {
+      const uint32_t v = sl ? oz_bytes(b[sl]) : b[sl];
+      (q == 0 ? w[sl].x : q == 1 ? w[sl].y : q == 2 ? w[sl].z : w[sl].w) = v;
+    }
+  }
+  oz_store(w, r, c16, slices, T, i, p);
+}
+
+// The digits of a warp's 8 rows r0.. of L[i, p] from the accumulator layout
+// (lane: row r0 + lane / 4, columns 8 nt + 2 t, + 1): a lane's four bytes of
+// every K chunk are exchanged among the four lanes of its row, after which
+// lane t holds the whole 16-byte word of chunk t.
+__device__ __forceinline__ void slice_rows_acc(const double (&c)[8][2], int r0, int lane,
+                                               double mul, uint8_t *slices, int T, int i, int p) {
+  const int t = lane & 3;
+  uint32_t v[4][kOzS];  // [chunk][slice]: columns 2t, 2t + 1, 8 + 2t, 9 + 2t of the chunk
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) {
+    uint32_t b[kOzS] = {};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) oz_fields(c[2 * ch + (e >> 1)][e & 1], mul, 8 * e, b);
+#pragma unroll
+    for (int sl = 0; sl < kOzS; ++sl) v[ch][sl] = sl ? oz_bytes(b[sl]) : b[sl];
+  }
+  uint4 w[kOzS];
+#pragma unroll
+  for (int sl = 0; sl < kOzS; ++sl) {
+    // 4 x 4 transpose over the lanes t (bit 1, then bit 0).
+    const bool up = t & 2, odd = t & 1;
+    const uint32_t s0 = up ? v[0][sl] : v[2][sl], s1 = up ? v[1][sl] : v[3][sl];
+    const uint32_t k0 = up ? v[2][sl] : v[0][sl], k1 = up ? v[3][sl] : v[1][sl];
+    const uint32_t g0 = __shfl_xor_sync(0xffffffffu, s0, 2), g1 = __shfl_xor_sync(0xffffffffu, s1, 2);
+    // Lower lanes now hold chunks 0 and 1 of the lanes t and t + 2, upper
+    // lanes chunks 2 and 3 of the lanes t - 2 and t.
+    const uint32_t a0 = up ? g0 : k0, a1 = up ? g1 : k1;  // from the lower lane of the two
+    const uint32_t b0 = up ? k0 : g0, b1 = up ? k1 : g1;  // from the upper one
+    const uint32_t sa = odd ? a0 : a1, sb = odd ? b0 : b1;
+    const uint32_t ka = odd ? a1 : a0, kb = odd ? b1 : b0;
+    const uint32_t ga = __shfl_xor_sync(0xffffffffu, sa, 1), gb = __shfl_xor_sync(0xffffffffu, sb, 1);
+    // o[q]: the bytes of lane q of the row for this lane's chunk.
+    const uint32_t o0 = odd ? ga : ka, o1 = odd ? ka : ga;
+    const uint32_t o2 = odd ? gb : kb, o3 = odd ? kb : gb;
+    w[sl] = make_uint4(__byte_perm(o0, o1, 0x5410), __byte_perm(o2, o3, 0x5410),
+                       __byte_perm(o0, o1, 0x7632), __byte_perm(o2, o3, 0x7632));
+  }
+  oz_store(w, r0 + (lane >> 2), t, slices, T, i, p);
 }
 
 // Step j of the factorisation, one launch over all slots with T > j + 1.
@@ -695,9 +775,11 @@ __global__ void __launch_bounds__(kColThreads, 2)
   __syncthreads();
   step_trsm(a, sl, j, i0, arows, sm, sm + kColRows * LDS, sm + (kColRows + TB) * LDS);
   if (SLICE) {  // int8 slices of the new L tiles for the int8 steps that follow
-    uint8_t *srow = a.slices + sl.sli;
-    slice_tile_smem(sm, arows, a.oz_mul, srow + (int64_t(i0) * (i0 - 1) / 2 + j) * kOzTileBytes,
-                    srow + (int64_t(i0 + 1) * i0 / 2 + j) * kOzTileBytes, tid, kColThreads);
+    for (int u = tid; u < arows * 4; u += kColThreads) {
+      const int h = u >> 8;
+      slice_row_chunk(sm + h * TB * LDS, u & 63, (u >> 6) & 3, a.oz_mul, a.slices + sl.sli, sl.T,
+                      i0 + h, j);
+    }
   }
   if (l != 0) return;
 
@@ -770,51 +852,64 @@ __global__ void __launch_bounds__(kColThreads, 2)
 //
 // Step j of the factorisation with the column update on the int8 tensor
 // cores, organised so that the int8 K loop of one item overlaps the FP64
-// epilogue of the previous one on the same SM.  An item is one 64-row tile:
-// row tile i of column j (C = A[i, j] - sum_{p<j} L[i, p] L[j, p]^T, then
-// L[i, j] U_j = C solved against the diagonal tile's factor, the forward
-// substitution and the int8 slices of L[i, j]), or the diagonal item of a
-// slot (D' of tile j + 1, left in dpart for k_diag_next).  Each CTA takes a
-// contiguous range of the step's items; nothing waits on another CTA.
+// epilogue of the previous one on the same SM.  An item is the pair of row
+// tiles 2u, 2u + 1 of column j, as far as they lie below row j
+// (C = A[i, j] - sum_{p<j} L[i, p] L[j, p]^T, then L[i, j] U_j = C solved
+// against the diagonal tile's factor, the forward substitution and the int8
+// slices of L[i, j]), or the diagonal item of a slot (D' of tile j + 1, left
+// in dpart for k_diag_next).  The CTAs take the items round robin; nothing
+// waits on another CTA.
 //   warp 0 (one thread): bulk copies of the slice half-tiles (K = 32) of the
-//     item's row tile and of the column tile row through a kWsStages ring;
+//     row pair and of the column tile row through a kWsStages ring;
 //   warp 1 (one thread): the tcgen05 MMAs into one TMEM accumulator;
-//   warps 2..9: per item the Wendland tile (during the K loop), the TMEM
+//   warps 2..17: per item the Wendland tiles (during the K loop), the TMEM
 //     drain (after which the MMA thread starts the next item), the level
 //     combination and the FP64 epilogue.
-// The MMA operand A holds two consecutive slices of the ONE row tile (rows
-// 0..63 slice a, 64..127 slice a + 1), B the slices of the column tile
-// stacked along N.  With the accumulator of pair (a, a+1) starting at TMEM
-// column group a - 1, column group g (64 columns) holds level g + 2 in lanes
-// 0..63 and level g + 3 in lanes 64..127 whatever the pair, so four pairs
-// (1,2), (3,4), (5,6), (7,0) against the column slices 1..9-a and six MMAs
-// per K = 32 cover every slice pair with a + b <= 9: levels 2..9 are lanes
-// 0..63 of groups 0..7 and lanes 64..127 of groups 0..6 (lanes 64..127 of
-// group 7 hold a partial level 10, not read).  In shared memory a K = 32 half
-// of the row tile is staged as [K chunk (2)][slice (8)][8-row group (8)][128
-// B] with the eighth slice of each chunk kept zero, so that the pair (7, 0)
-// adds nothing to lanes 64..127; the column tile's half is the stored layout
-// itself ([K chunk (2)][slice (7)]...), one contiguous 14 KB copy.
-constexpr int kWsStages = 3;
+// The MMA operand A is one slice of the pair (rows 0..63 tile 2u, 64..127 tile
+// 2u + 1), B the slices of the column tile stacked along N; the accumulator
+// of slice pair (a, b) is TMEM column group a + b - 2 (64 columns), so the
+// eight groups hold the levels 2..9 of both tiles and eleven MMAs per K = 32
+// cover the 34 slice pairs with a + b <= 9, none of them twice.
+//
+// Why pairs and sixteen epilogue warps: with one row tile per item (two
+// slices stacked in M, six MMAs with 38 of the digit products per tile, eight
+// epilogue warps) a K = 32 half took 1,170 cycles for 28 KB of copies and 63
+// KB of operand reads, and up to step 12 the item's time was its epilogue, whose
+// FP64 chains eight warps could not hide.  A pair shares the column's copy and
+// operand reads (43 KB and 112 KB for two tiles) and drains two tiles in the
+// time of one.  The items go round robin, so that the CTAs at work on a slot
+// read the column's slices together from L2 (in contiguous ranges they came
+// from DRAM once per item: 5.3 TB/s, 2% L2 hits).  After the solve the rows of
+// L stay in registers for the store, the forward substitution and the digits
+// (through shared memory these took 23k cycles of an item, now 9k).
+// 1M refined points, all steps of one slot group: 68 -> 53 ms; step 18 of a
+// quarter of it, under ncu: tensor pipe 60% of active cycles, DRAM 53%.
+//
+// The FP64 tensor instructions of the solve share the tensor pipe with the
+// MMAs (6.5k cycles without, 14k beside them), and the K loop in turn is
+// slowed.  While the K loop is shorter than the rest of an item (steps below
+// kWsLate) the accumulator goes back after the solve instead of after the
+// drain: steps 2..8 take 10-15% less that way, steps from 12 on 5-8% more.
+constexpr int kWsStages = 2;
 constexpr int kWsChunk = kOzS * 1024;                    // 7168: one 16-byte K chunk, 7 slices
 constexpr int kWsHalf = 2 * kWsChunk;                    // 14336: one K = 32 half of a slice tile
-constexpr int kWsChunkA = (kOzS + 1) * 1024;             // staged row-tile chunk with a zero slice
-constexpr int kWsHalfA = 2 * kWsChunkA;                  // 16384
-constexpr int kWsStage = kWsHalfA + kWsHalf;             // row half + column half
-constexpr int kWsThreads = 320;                          // 2 issue warps + 8 epilogue warps
-constexpr int kWsCOff = kWsStages * kWsStage;            // C / D (TB x LDS doubles)
-constexpr int kWsXOff = kWsCOff + TB * LDS * 8;          // U_j, the diagonal tile's factor
-constexpr int kWsLOff = kWsXOff + TB * LDS * 8;          // upper TMEM lanes' level sums
-constexpr int kWsPtsOff = kWsLOff + TB * LDS * 8;        // row points (2 x TB), column points
-constexpr int kWsRedOff = kWsPtsOff + 2 * TB * 32 + 3 * TB * 8;  // y_j, r_i, diag_tile vectors
-constexpr int kWsUiOff = kWsRedOff + 3 * TB * kMaxF * 8;  // U_j's diagonal block inverses
+constexpr int kWsChunkA = 2 * kWsChunk;                  // the same of a row pair
+constexpr int kWsHalfA = 2 * kWsHalf;
+constexpr int kWsStage = kWsHalfA + kWsHalf;             // pair half + column half
+constexpr int kWsEpi = 512;                              // epilogue threads
+constexpr int kWsThreads = kWsEpi + 64;                  // + 2 issue warps
+constexpr int kWsRows = 2 * TB;
+constexpr int kWsLate = 9;                               // steps that hand the accumulator back late
+constexpr int kWsCOff = kWsStages * kWsStage;            // C / L / D' (kWsRows x LDS doubles)
+constexpr int kWsXOff = kWsCOff + kWsRows * LDS * 8;     // U_j, the diagonal tile's factor
+constexpr int kWsPtsOff = kWsXOff + TB * LDS * 8;        // points of two items
+constexpr int kWsPts = kWsRows + TB;
+constexpr int kWsRedOff = kWsPtsOff + 2 * kWsPts * 32;   // y_j, r_i
+constexpr int kWsUiOff = kWsRedOff + (TB + kWsRows) * kMaxF * 8;  // U_j's diagonal block inverses
 constexpr int kWsBarOff = kWsUiOff + 4 * 16 * kUiLd * 8;
 constexpr size_t kWsSmem = size_t(kWsBarOff) + 256;
 static_assert(kWsSmem <= 232448, "shared memory of k_col_step_ws");
 static_assert(kWsStage % 1024 == 0, "stages start on 1 KB boundaries");
-static_assert(kOzTileBytes <= TB * LDS * 8, "slice staging does not fit the C buffer");
-static_assert((TB * kMaxF + 2 * TB + TB) * 8 <= 3 * TB * kMaxF * 8, "diag_tile vectors");
-static_assert(2 * TB * kMaxF + 3 * TB <= 3 * TB * kMaxF, "residual rows after the diag_tile vectors");
 
 struct WsBars {
   uint64_t full[kWsStages], empty[kWsStages], acc_full, acc_empty, done;
@@ -823,8 +918,13 @@ struct WsBars {
 };
 static_assert(sizeof(WsBars) <= 256, "barrier area");
 
+// Row pairs of a slot with T tile rows that reach below row j.
+__host__ __device__ __forceinline__ int ws_pairs(int T, int j) {
+  return (T - 1) / 2 - (j + 1) / 2 + 1;
+}
 // The item `it` of step j: slot q (prefix counts ipre over the cnt active
-// slots), and r = it - ipre[q]: r == 0 the diagonal item, else row tile j + r.
+// slots), and r = it - ipre[q]: r == 0 the diagonal item, else pair
+// (j + 1) / 2 + r - 1.
 struct WsItem {
   int q, r;
 };
@@ -832,176 +932,134 @@ __device__ __forceinline__ WsItem ws_item(const int *ipre, int cnt, int it) {
   const int q = find_slot(ipre, cnt, it);
   return {q, it - ipre[q]};
 }
-// The items of a CTA's range in order: one binary search for the first,
-// then the slot advances when the item passes the next slot's first item
-// (the slot record is reloaded only then).
-struct WsCursor {
-  int q = -1, first = 0, next = 0;
-  BigSlot sl;
-  int64_t s0 = 0;  // first membership entry of the slot's patch (with soff)
-  __device__ __forceinline__ WsItem at(const int *ipre, const BigSlot *slots, const int64_t *soff,
-                                       int cnt, int it) {
-    if (q < 0 || it >= next) {
-      if (q < 0) q = find_slot(ipre, cnt, it);
-      else
-        do ++q;
-        while (it >= ipre[q + 1]);
-      first = ipre[q];
-      next = ipre[q + 1];
-      sl = slots[q];
-      if (soff) s0 = soff[sl.k];
+__device__ __forceinline__ int ws_pair(int j, int r) { return (j + 1) / 2 + (r ? r - 1 : 0); }
+// The item by a whole warp, searching on from slot q0 (at or before the
+// item's): the lanes look at 32 slots at once, one load's latency where a
+// thread stepping from slot to slot pays one for each.
+__device__ __forceinline__ WsItem ws_find(const int *__restrict__ ipre, int cnt, int it, int q0,
+                                          int lane) {
+  for (;; q0 += 32) {
+    const int e = q0 + 1 + lane;
+    const int end = e <= cnt ? ipre[e] : 0x7fffffff;
+    const unsigned int m = __ballot_sync(0xffffffffu, end > it);
+    if (m) {
+      const int q = q0 + __ffs(m) - 1;
+      return {q, it - ipre[q]};
     }
-    return {q, it - first};
   }
-};
-
-// Six MMAs of one K = 32 half: pairs (1,2), (3,4), (5,6), (7,0) of the row
-// tile's slices against the column tile's slices 1..9-a stacked along N.  On
-// the first half of an item the first MMA to reach a column overwrites it:
-// pair (1, 2) groups 0..3, pair (5, 6) groups 4..7, issued first.
-__device__ __forceinline__ void ws_mma_half(uint32_t tmem, uint32_t sA, uint32_t sB, bool first) {
-  const uint64_t b0 = umma_desc(sB, kWsChunk, 128), b4 = umma_desc(sB + 4 * 1024, kWsChunk, 128);
-  const uint32_t acc = first ? 0u : 1u;
-  const uint64_t a12 = umma_desc(sA, kWsChunkA, 128);
-  const uint64_t a34 = umma_desc(sA + 2 * 1024, kWsChunkA, 128);
-  const uint64_t a56 = umma_desc(sA + 4 * 1024, kWsChunkA, 128);
-  const uint64_t a70 = umma_desc(sA + 6 * 1024, kWsChunkA, 128);
-  umma_i8(tmem, a12, b0, umma_idesc_i8(256), acc);          // (1,2) x 1..4: groups 0..3
-  umma_i8(tmem + 256, a56, b0, umma_idesc_i8(256), acc);    // (5,6) x 1..4: groups 4..7
-  umma_i8(tmem + 256, a12, b4, umma_idesc_i8(192), 1u);     // (1,2) x 5..7: groups 4..6
-  umma_i8(tmem + 128, a34, b0, umma_idesc_i8(256), 1u);     // (3,4) x 1..4: groups 2..5
-  umma_i8(tmem + 384, a34, b4, umma_idesc_i8(128), 1u);     // (3,4) x 5..6: groups 6..7
-  umma_i8(tmem + 384, a70, b0, umma_idesc_i8(128), 1u);     // (7,0) x 1..2: groups 6..7
 }
 
-// Epilogue warp e (warp 2 + e) reads TMEM lanes 32 qd .. + 31 (qd = warp % 4)
-// and columns 32 h .. + 31 (h = e / 4) of the column groups: the level sums of
-// its half of row r (lanes 0..63: levels 2..9 in groups 0..7, rows r = lane;
-// lanes 64..127: levels 3..9 in groups 0..6, rows r = lane - 64).  The levels
-// are merged in int64 first: |level| < 2^31, so the top three shifted by 7
-// bits each stay below 2^53 and convert exactly, and the lower four or five
-// (below 2^60 in units of 128^-9) round to within 2^-57; then two FP64
-// terms (in units of sigma^2).  Lanes 0..63
-// subtract sig2 x their sum from sC (which holds A); lanes 64..127 store
-// theirs in sUp, which the caller subtracts after a barrier.
-__device__ __forceinline__ void ws_drain(uint32_t tmem, int qd, int h, double *sC, double *sUp,
-                                         double sig2, int lane) {
-  constexpr int kG = kOzS + 1;  // column groups 0..7
-  const uint32_t lane_base = uint32_t(32 * qd) << 16;
-  const bool up = qd >= 2;
-  const int ng = up ? kG - 1 : kG;  // upper lanes: group 7 holds a partial level 10
+// The MMAs of one K = 32 half.  On the first half of an item the first MMA to
+// reach a column overwrites it: slice 1 groups 0..3, slice 5 groups 4..7,
+// issued first.
+__device__ __forceinline__ void ws_mma_half(uint32_t tmem, uint32_t sA, uint32_t sB, bool first) {
+  const uint32_t acc = first ? 0u : 1u;
+  auto ad = [&](int a) { return umma_desc(sA + (a - 1) * 2048, kWsChunkA, 128); };
+  const uint64_t b1 = umma_desc(sB, kWsChunk, 128);             // slices 1..4
+  const uint64_t b5 = umma_desc(sB + 4 * 1024, kWsChunk, 128);  // slices 5..7
+  umma_i8(tmem, ad(1), b1, umma_idesc_i8(256), acc);         // groups 0..3
+  umma_i8(tmem + 256, ad(5), b1, umma_idesc_i8(256), acc);   // groups 4..7
+  umma_i8(tmem + 256, ad(1), b5, umma_idesc_i8(192), 1u);    // 1 x 5..7: groups 4..6
+  umma_i8(tmem + 64, ad(2), b1, umma_idesc_i8(256), 1u);     // 2 x 1..4: groups 1..4
+  umma_i8(tmem + 320, ad(2), b5, umma_idesc_i8(192), 1u);    // 2 x 5..7: groups 5..7
+  umma_i8(tmem + 128, ad(3), b1, umma_idesc_i8(256), 1u);    // 3 x 1..4: groups 2..5
+  umma_i8(tmem + 384, ad(3), b5, umma_idesc_i8(128), 1u);    // 3 x 5..6: groups 6..7
+  umma_i8(tmem + 192, ad(4), b1, umma_idesc_i8(256), 1u);    // 4 x 1..4: groups 3..6
+  umma_i8(tmem + 448, ad(4), b5, umma_idesc_i8(64), 1u);     // 4 x 5: group 7
+  umma_i8(tmem + 320, ad(6), b1, umma_idesc_i8(192), 1u);    // 6 x 1..3: groups 5..7
+  umma_i8(tmem + 384, ad(7), b1, umma_idesc_i8(128), 1u);    // 7 x 1..2: groups 6..7
+}
+
+// An epilogue warp reads TMEM lanes 32 qd .. + 31 (rows of the pair) and
+// columns 16 h .. + 15 of every column group: the sums of levels 2..9 of its
+// rows.  The levels are merged in int64 first: a level's sum is below 2^31
+// (at most 36,700 per column of K: 58,000 columns), so the top three shifted
+// by 7 bits each stay below 2^53 and convert exactly, and the lower five
+// (below 2^60 in units of 128^-9) round to within 2^-57; then two FP64 terms
+// (in units of sigma^2), of which sig2 x their sum is subtracted from sC
+// (which holds A).
+__device__ __forceinline__ void ws_drain(uint32_t tmem, int qd, int h, double *sC, double sig2,
+                                         int lane) {
+  constexpr int kG = 8;  // column groups, levels 2..9
+  const uint32_t base = tmem + (uint32_t(32 * qd) << 16) + uint32_t(16 * h);
   // Four columns per step: the levels are merged into (hi, lo), the loads of
   // step cb + 1 are issued, and the conversions and stores of step cb run
   // while they are in flight.
   uint32_t z[kG][4];
   auto issue = [&](int cb) {
 #pragma unroll
-    for (int g = 0; g < kG; ++g) {
-      if (g >= ng) break;
-      const uint32_t addr = tmem + lane_base + uint32_t(64 * g + 32 * h + 4 * cb);
+    for (int g = 0; g < kG; ++g)
       asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
                    : "=r"(z[g][0]), "=r"(z[g][1]), "=r"(z[g][2]), "=r"(z[g][3])
-                   : "r"(addr));
-    }
+                   : "r"(base + uint32_t(64 * g + 4 * cb)));
   };
+  double *cr = sC + (32 * qd + lane) * LDS + 16 * h;
   issue(0);
 #pragma unroll
-  for (int cb = 0; cb < 8; ++cb) {
+  for (int cb = 0; cb < 4; ++cb) {
     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
     long long hi[4], lo[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const long long z0 = int32_t(z[0][c]), z1 = int32_t(z[1][c]), z2 = int32_t(z[2][c]);
       const long long z3 = int32_t(z[3][c]), z4 = int32_t(z[4][c]), z5 = int32_t(z[5][c]);
-      const long long z6 = int32_t(z[6][c]);
+      const long long z6 = int32_t(z[6][c]), z7 = int32_t(z[7][c]);
       hi[c] = (z0 * 128 + z1) * 128 + z2;
-      lo[c] = up ? ((z3 * 128 + z4) * 128 + z5) * 128 + z6
-                 : (((z3 * 128 + z4) * 128 + z5) * 128 + z6) * 128 + int32_t(z[7][c]);
+      lo[c] = (((z3 * 128 + z4) * 128 + z5) * 128 + z6) * 128 + z7;
     }
-    if (cb < 7) issue(cb + 1);
+    if (cb < 3) issue(cb + 1);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      // Lower lanes: levels 2..4 and 5..9; upper lanes: 3..5 and 6..9.
-      const double val = __fma_rn(double(hi[c]), up ? 0x1p-35 : 0x1p-28, double(lo[c]) * 0x1p-63);
-      const int col = 32 * h + 4 * cb + c;
-      if (!up) {
-        double *cr = sC + (32 * qd + lane) * LDS + col;
-        *cr = __fma_rn(-sig2, val, *cr);
-      } else {
-        sUp[(32 * (qd - 2) + lane) * LDS + col] = val;
-      }
+      const double val = __fma_rn(double(hi[c]), 0x1p-28, double(lo[c]) * 0x1p-63);
+      cr[4 * cb + c] = __fma_rn(-sig2, val, cr[4 * cb + c]);
     }
   }
 }
 
-__device__ __forceinline__ void ws_sync() { asm volatile("bar.sync 1, 256;\n" ::: "memory"); }
+__device__ __forceinline__ void ws_sync() { asm volatile("bar.sync 1, 512;\n" ::: "memory"); }
+static_assert(kWsEpi == 512, "ws_sync counts the epilogue threads");
 
-// Row points of a tile: thread e < TB loads the membership index of row e
-// early (ws_point_index) and copies the point into prow[e] later
-// (ws_point_copy, cp.async; zeros past n), so that the next item's points
-// arrive while the current item's epilogue runs.
-__device__ __forceinline__ int ws_point_index(const BigArgs &a, const BigSlot &sl, int64_t s0,
-                                              int ti, int e) {
-  const int gi = ti * TB + e;
-  return gi < sl.n ? a.sidx[s0 + gi] : -1;
+// Points of an item, kWsPts of them: the rows 2u TB .. of the pair, then the
+// columns of tile tj.  Thread e loads the membership index of its point early
+// (ws_point_index) and copies the point into pts[e] later (ws_point_copy,
+// cp.async; zeros past n), so that the next item's points arrive while the
+// current item's epilogue runs.
+__device__ __forceinline__ int ws_point_index(const BigArgs &a, const BigSlot &sl, int u, int tj,
+                                              int e) {
+  const int gi = e < kWsRows ? 2 * u * TB + e : tj * TB + (e - kWsRows);
+  return gi < sl.n ? a.sidx[a.soff[sl.k] + gi] : -1;
 }
-__device__ __forceinline__ void ws_point_copy(const BigArgs &a, double4 *prow, int e, int idx) {
+__device__ __forceinline__ void ws_point_copy(const BigArgs &a, double4 *pts, int e, int idx) {
   if (idx >= 0) {
     const double *g = reinterpret_cast<const double *>(a.src + idx);
-    double *d = reinterpret_cast<double *>(prow + e);
+    double *d = reinterpret_cast<double *>(pts + e);
     cp_async16(d, g);
     cp_async16(d + 2, g + 2);
   } else {
-    prow[e] = make_double4(0.0, 0.0, 0.0, 0.0);
-  }
-}
-// The evaluation loop of ws_gen_tile for one basis, without branches: thread
-// t takes column c = t % 64 of rows t / 64 + 4 m, m = 0..15, and the identity
-// padding past n is selected, so that the unrolled evaluations form one block
-// whose FP64 chains (23-cycle FMA latency on this GPU) overlap.
-template <int B>
-__device__ __forceinline__ void ws_gen_rows(const BigArgs &a, const BigSlot &sl, int ti, int tj,
-                                            double *sT, const double4 *prow, const double *cpts,
-                                            int t) {
-  const double *cx = cpts, *cy = cx + TB, *cz = cy + TB;
-  const int c = t & 63, gj = tj * TB + c;
-  const double px = cx[c], py = cy[c], pz = cz[c];
-#pragma unroll 8
-  for (int m = 0; m < TB * TB / 256; ++m) {
-    const int r = (t >> 6) + 4 * m;
-    const int gi = ti * TB + r;
-    const double4 pr = prow[r];
-    const double w =
-        wendland<double>(B, __dsqrt_rn(sqdist3(pr.x, pr.y, pr.z, px, py, pz)), a.rinv);
-    const double pad = (gi == gj) ? 1.0 : 0.0;
-    sT[r * LDS + c] = (gi < sl.n && gj < sl.n) ? w : pad;
+    pts[e] = make_double4(0.0, 0.0, 0.0, 0.0);
   }
 }
 
-// A[ti, tj] of the slot (gen_tile) into sT, by the 256 epilogue threads, from
-// the row points in prow (staged and waited for by the caller) and the
-// column points in cpts (3 x TB, reloaded when load_cols).
-__device__ __forceinline__ void ws_gen_tile(const BigArgs &a, const BigSlot &sl, int64_t s0,
-                                            int ti, int tj, double *sT, const double4 *prow,
-                                            double *cpts, int t, bool load_cols) {
-  double *cx = cpts, *cy = cx + TB, *cz = cy + TB;
-  if (load_cols)
-    for (int e = t; e < TB; e += 256) {
-      const int gj = tj * TB + e;
-      double4 p = make_double4(0.0, 0.0, 0.0, 0.0);
-      if (gj < sl.n) p = a.src[a.sidx[s0 + gj]];
-      cx[e] = p.x;
-      cy[e] = p.y;
-      cz[e] = p.z;
+// Rows [64 h0, 64 h1) of A[2u.., tj] into sT (row stride LDS) by the epilogue
+// threads from the item's points.  Thread t takes column t % 64 of every
+// eighth row; the evaluations are free of branches, so that their FP64 chains
+// overlap.
+__device__ __forceinline__ void ws_gen_rows(const BigArgs &a, const BigSlot &sl, int u, int tj,
+                                            int h0, int h1, double *sT, const double4 *pts,
+                                            int t) {
+  const int c = t & 63, gj = tj * TB + c;
+  const double4 pc = pts[kWsRows + c];
+  with_basis(a.basis, [&](auto B) {
+#pragma unroll 4
+    for (int m = 8 * h0; m < 8 * h1; ++m) {
+      const int r = (t >> 6) + 8 * m;
+      const int gi = 2 * u * TB + r;
+      const double4 pr = pts[r];
+      const double w = phi_at<B>(sqdist3(pr.x, pr.y, pr.z, pc.x, pc.y, pc.z), a.rinv);
+      const double pad = (gi == gj) ? 1.0 : 0.0;
+      sT[r * LDS + c] = (gi < sl.n && gj < sl.n) ? w : pad;
     }
-  ws_sync();
-  switch (a.basis) {
-  case kWendlandC0: ws_gen_rows<kWendlandC0>(a, sl, ti, tj, sT, prow, cpts, t); break;
-  case kWendlandC2: ws_gen_rows<kWendlandC2>(a, sl, ti, tj, sT, prow, cpts, t); break;
-  case kWendlandC4: ws_gen_rows<kWendlandC4>(a, sl, ti, tj, sT, prow, cpts, t); break;
-  case kWendlandC6: ws_gen_rows<kWendlandC6>(a, sl, ti, tj, sT, prow, cpts, t); break;
-  default: ws_gen_rows<kWendlandC8>(a, sl, ti, tj, sT, prow, cpts, t); break;
-  }
+  });
 }
 
 __global__ void __launch_bounds__(kWsThreads, 1)
@@ -1012,19 +1070,15 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   volatile int *abort_flag = &bar->abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nitems = ipre[cnt];
-  const int it0 = int(int64_t(blockIdx.x) * nitems / gridDim.x);
-  const int it1 = int(int64_t(blockIdx.x + 1) * nitems / gridDim.x);
+  const int it0 = blockIdx.x, it1 = nitems, step = gridDim.x;
   const int nh = 2 * j;  // K = 32 halves per item
-  auto slice_row = [&](const BigSlot &sl, int i) {
-    return a.slices + sl.sli + (int64_t(i) * (i - 1) / 2) * kOzTileBytes;
-  };
   if (tid == 0) {
     for (int i = 0; i < kWsStages; ++i) {
       mbar_init(&bar->full[i], 1);
       mbar_init(&bar->empty[i], 1);
     }
     mbar_init(&bar->acc_full, 1);
-    mbar_init(&bar->acc_empty, 8);
+    mbar_init(&bar->acc_empty, kWsEpi / 32);
     mbar_init(&bar->done, 1);
     bar->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -1036,29 +1090,23 @@ __global__ void __launch_bounds__(kWsThreads, 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  // The zero eighth slice of each staged row-tile chunk, made visible to the
-  // tensor core (async proxy); the copies never write it.
-  for (int u = tid; u < kWsStages * 2 * 64; u += kWsThreads) {
-    const int st = u >> 7, ch = (u >> 6) & 1, w16 = u & 63;
-    *reinterpret_cast<uint4 *>(smb + st * kWsStage + ch * kWsChunkA + kWsChunk + 16 * w16) =
-        make_uint4(0u, 0u, 0u, 0u);
-  }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bar->tmem;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // Producer.
-      int hc = 0;
-      WsCursor cur;
-      for (int it = it0; it < it1 && !*abort_flag; ++it) {
-        const WsItem w = cur.at(ipre, slots, nullptr, cnt, it);
-        const BigSlot &sl = cur.sl;
-        const uint8_t *ra = slice_row(sl, w.r == 0 ? j + 1 : j + w.r);
-        const uint8_t *rb = slice_row(sl, w.r == 0 ? j + 1 : j);
+    // Producer: the warp finds the items, lane 0 issues the copies.
+    int hc = 0;
+    bool ok = true;
+    WsItem w{0, 0};
+    for (int it = it0; it < it1 && ok; it += step) {
+      w = ws_find(ipre, cnt, it, w.q, lane);
+      if (lane == 0) {
+        const int T = slots[w.q].T;
+        const uint8_t *sl0 = a.slices + slots[w.q].sli;
+        const uint8_t *ra = sl0 + oz_pair_off(T, ws_pair(j, w.r), 0);
+        const uint8_t *rb = sl0 + oz_tile_off(w.r == 0 ? j + 1 : j, 0);
         for (int hh = 0; hh < nh; ++hh, ++hc) {
           const int st = hc % kWsStages, u = hc / kWsStages;
           if (hc >= kWsStages &&
@@ -1067,27 +1115,27 @@ __global__ void __launch_bounds__(kWsThreads, 1)
             break;
           }
           uint8_t *sA = smb + st * kWsStage;
-          const int64_t off = int64_t(hh >> 1) * kOzTileBytes + (hh & 1) * kWsHalf;
-          mbar_expect_tx(&bar->full[st], uint32_t(2 * kWsHalf));
-          bulk_g2s(sA, ra + off, kWsChunk, &bar->full[st]);
-          bulk_g2s(sA + kWsChunkA, ra + off + kWsChunk, kWsChunk, &bar->full[st]);
-          bulk_g2s(sA + kWsHalfA, rb + off, kWsHalf, &bar->full[st]);
+          mbar_expect_tx(&bar->full[st], uint32_t(kWsHalfA + kWsHalf));
+          bulk_g2s(sA, ra + int64_t(hh) * kWsHalfA, kWsHalfA, &bar->full[st]);
+          bulk_g2s(sA + kWsHalfA, rb + int64_t(hh) * kWsHalf, kWsHalf, &bar->full[st]);
         }
+        ok = !*abort_flag;
       }
-      // Drain: only the latest use of each stage can still be in flight.
-      const int issued = hc;
-      for (int st = 0; st < kWsStages && st < issued; ++st) {
-        const int last = st + kWsStages * ((issued - 1 - st) / kWsStages);
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    }
+    // Drain: only the latest use of each stage can still be in flight.
+    if (lane == 0)
+      for (int st = 0; st < kWsStages && st < hc; ++st) {
+        const int last = st + kWsStages * ((hc - 1 - st) / kWsStages);
         if (!mbar_wait(&bar->full[st], uint32_t((last / kWsStages) & 1), kOzDrainLimit))
           *abort_flag = 1;
       }
-    }
   } else if (warp == 1) {
     if (lane == 0) {
       // MMA issue.
       int hc = 0, k = 0;
       bool ok = true;
-      for (int it = it0; it < it1 && ok; ++it, ++k) {
+      for (int it = it0; it < it1 && ok; it += step, ++k) {
         // The accumulator is free once the epilogue drained the previous item.
         if (k > 0 && !mbar_wait_pipe(&bar->acc_empty, uint32_t((k - 1) & 1), a.wait_limit,
                                      abort_flag)) {
@@ -1113,18 +1161,16 @@ __global__ void __launch_bounds__(kWsThreads, 1)
       umma_commit(&bar->done);  // arrives once every MMA issued above has completed
     }
   } else {
-    // Epilogue: 8 warps, etid 0..255.
+    // Epilogue: 16 warps, etid 0..511.
     const int etid = tid - 64, ew = warp - 2;
-    const int qd = warp & 3, h = ew >> 2;
+    const int qd = warp & 3, h4 = ew >> 2;
     double *sC = reinterpret_cast<double *>(smb + kWsCOff);
     double *sX = reinterpret_cast<double *>(smb + kWsXOff);
-    double *sL = reinterpret_cast<double *>(smb + kWsLOff);
-    double4 *prows = reinterpret_cast<double4 *>(smb + kWsPtsOff);              // 2 x TB
-    double *cpts = reinterpret_cast<double *>(smb + kWsPtsOff + 2 * TB * 32);  // 3 x TB
-    double *ysh = reinterpret_cast<double *>(smb + kWsRedOff);  // TB x kMaxF
-    double *rsh = ysh + TB * kMaxF + 3 * TB;                     // r_i, TB x kMaxF
-    double *sUi = reinterpret_cast<double *>(smb + kWsUiOff);   // [b][k][c] = U_bb^-1[k][c]
-                                                                 // (row stride kUiLd)
+    double4 *pts = reinterpret_cast<double4 *>(smb + kWsPtsOff);  // 2 x kWsPts
+    double *ysh = reinterpret_cast<double *>(smb + kWsRedOff);    // TB x kMaxF
+    double *rsh = ysh + TB * kMaxF;                               // r_i, kWsRows x kMaxF
+    double *sUi = reinterpret_cast<double *>(smb + kWsUiOff);     // [b][k][c] = U_bb^-1[k][c]
+                                                                  // (row stride kUiLd)
     volatile int *ep_stop = &bar->ep_stop;  // written by epilogue threads only
     if (etid == 0) *ep_stop = 0;
     // The step may be launched while the previous launch (k_diag_next of
@@ -1132,58 +1178,61 @@ __global__ void __launch_bounds__(kWsThreads, 1)
     // the copy and MMA warps need only the slices of earlier steps, which
     // the launch before that wrote, but the epilogue waits for it here.
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    ws_sync();
     int xq = -1;  // slot whose U_j (factor of the diagonal tile, transposed) is in sX
-    int pq = -1, ptj = -1;  // slot and column tile whose points are in cpts
     int k = 0;
-    WsCursor cur, nxt;  // the item, and the next one (its row points are prefetched)
-    int nidx = -1;      // membership index of this thread's row point of the next item
+    WsItem nw{0, 0};  // the next item, whose points are prefetched
+    int nidx = -1;    // membership index of this thread's point of it
+    auto next_index = [&](int it) {
+      nw = ws_find(ipre, cnt, it, nw.q, lane);
+      if (etid < kWsPts)
+        nidx = ws_point_index(a, slots[nw.q], ws_pair(j, nw.r), nw.r ? j : j + 1, etid);
+    };
     if (it0 < it1) {
-      const WsItem w0 = nxt.at(ipre, slots, a.soff, cnt, it0);
-      if (etid < TB)
-        ws_point_copy(a, prows, etid,
-                      ws_point_index(a, nxt.sl, nxt.s0, w0.r == 0 ? j + 1 : j + w0.r, etid));
+      next_index(it0);
+      if (etid < kWsPts) ws_point_copy(a, pts, etid, nidx);
     }
     cp_async_commit();
-    for (int it = it0; it < it1; ++it, ++k) {
-      const WsItem w = cur.at(ipre, slots, a.soff, cnt, it);
-      const BigSlot sl = cur.sl;
+    for (int it = it0; it < it1; it += step, ++k) {
+      const WsItem w = nw;
+      const BigSlot &sl = slots[w.q];
       const int ld = sl.ld, F = a.F;
       double *W = a.W + sl.base;
       double *rcol = W + int64_t(sl.T) * TB;
       const bool diag = w.r == 0;
-      const int i = diag ? j + 1 : j + w.r;
+      const int u = ws_pair(j, w.r);
+      // The halves of the pair that the item needs: [h0, h1).
+      const int h0 = diag ? (j + 1) & 1 : (2 * u > j ? 0 : 1);
+      const int h1 = diag ? h0 + 1 : (2 * u + 1 < sl.T ? 2 : 1);
+      const int rows0 = TB * h0, rows1 = TB * h1;
+      // The item's points have landed, and every warp is done with the
+      // previous item's C, factor and residual rows.
+      cp_async_wait<0>();
+      ws_sync();
       if (!diag) {
         // U_j (and its block inverses) and y_j once per slot, the
-        // residual rows r_i of every item: copied while the tile is made.
+        // residual rows r_i of every item: copied while the tiles are made.
         if (xq != w.q) {
-          load_factor_async(sX, W + int64_t(j) * TB * ld + int64_t(j) * TB, ld, etid, 256);
+          load_factor_async(sX, W + int64_t(j) * TB * ld + int64_t(j) * TB, ld, etid, kWsEpi);
           // U_bb^-1 = (X_j's diagonal block b)^T, X_j = L_jj^-1 row-major.
           const double *xg = a.inv + sl.inv + int64_t(j) * TB * TB;
-          for (int e = etid; e < 4 * 256; e += 256) {
-            const int b = e >> 8, k = (e >> 4) & 15, c = e & 15;
-            cp_async8(sUi + (16 * b + k) * kUiLd + c, xg + (16 * b + c) * TB + 16 * b + k);
+          for (int e = etid; e < 4 * 256; e += kWsEpi) {
+            const int b = e >> 8, kk = (e >> 4) & 15, c = e & 15;
+            cp_async8(sUi + (16 * b + kk) * kUiLd + c, xg + (16 * b + c) * TB + 16 * b + kk);
           }
           const double *yg = rcol + int64_t(j) * TB * ld;
-          for (int e = etid; e < TB * F; e += 256)
+          for (int e = etid; e < TB * F; e += kWsEpi)
             cp_async8(ysh + (e / F) * kMaxF + e % F, yg + int64_t(e / F) * ld + e % F);
           xq = w.q;
         }
-        const double *rg = rcol + int64_t(i) * TB * ld;
-        for (int e = etid; e < TB * F; e += 256)
+        const double *rg = rcol + int64_t(2 * u) * TB * ld;
+        for (int e = rows0 * F + etid; e < rows1 * F; e += kWsEpi)
           cp_async8(rsh + (e / F) * kMaxF + e % F, rg + int64_t(e / F) * ld + e % F);
       }
       cp_async_commit();
-      // A[i, j] (or A[j+1, j+1]) while the MMAs of this item run, once the
-      // row points (the group before the one just committed) have landed;
-      // the column points stay in cpts while the slot and column tile do.
-      cp_async_wait<1>();
-      const int tj = diag ? j + 1 : j;
-      ws_gen_tile(a, sl, cur.s0, i, tj, sC, prows + (k & 1) * TB, cpts, etid,
-                  pq != w.q || ptj != tj);
-      pq = w.q;
-      ptj = tj;
-      ws_sync();
+      // The next item's membership index, loaded while this one runs.
+      if (it + step < it1) next_index(it + step);
+      // A[i, j] (or A[j+1, j+1]) while the MMAs of this item run.
+      ws_gen_rows(a, sl, u, diag ? j + 1 : j, h0, h1, sC, pts + (k & 1) * kWsPts, etid);
       // Drain the accumulator, then hand it back to the MMA thread.
       // Every epilogue thread waits; the decision to stop is made uniform
       // through ep_stop (the global abort flag may change at any time).
@@ -1194,76 +1243,55 @@ __global__ void __launch_bounds__(kWsThreads, 1)
         break;
       }
       tc_fence_after();
-      // C = A - sigma^2 (lower-lane levels + upper-lane levels): sC gets A
-      // minus the lower lanes' sums, sL the upper lanes' sums.  At j = 0
-      // there are no products (no MMAs were issued) and C = A.
-      if (j > 0) ws_drain(tmem, qd, h, sC, sL, a.oz_sig2, lane);
+      // C = A - sigma^2 (level sums).  At j = 0 there are no products (no
+      // MMAs were issued) and C = A.
+      if (j > 0 && (qd >> 1) >= h0 && (qd >> 1) < h1) ws_drain(tmem, qd, h4, sC, a.oz_sig2, lane);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cnt(&bar->acc_empty, 1);
-      ws_sync();
-      // The next item's membership indices, loaded while this one finishes.
-      if (it + 1 < it1 && etid < TB) {
-        const WsItem wn = nxt.at(ipre, slots, a.soff, cnt, it + 1);
-        nidx = ws_point_index(a, nxt.sl, nxt.s0, wn.r == 0 ? j + 1 : j + wn.r, etid);
-      }
-      // C = sC - sigma^2 sL is formed where it is read: by the diagonal
-      // item's copy, or by the triangular solve's loads.  The copies of the
-      // next item's row points go out as one commit group per item.
-      auto next_points = [&]() {
-        if (it + 1 < it1) {
-          if (etid < TB) ws_point_copy(a, prows + ((k + 1) & 1) * TB, etid, nidx);
-          cp_async_commit();
-        }
+      auto release = [&] {
+        if (lane == 0) mbar_arrive_cnt(&bar->acc_empty, 1);
       };
+      cp_async_wait<0>();  // the factor and the residual rows
+      ws_sync();
+      if (it + step < it1 && etid < kWsPts)
+        ws_point_copy(a, pts + ((k + 1) & 1) * kWsPts, etid, nidx);
+      cp_async_commit();
+      const int r0 = 8 * ew;
+      const bool mine = !diag && r0 >= rows0 && r0 < rows1;
+      const bool late = mine && j < kWsLate;
+      if (!late) release();
       if (diag) {
         // D' to dpart, where the next launch (k_diag_next) factors D.
         double *dst = a.dpart + int64_t(sl.q) * TB * TB;
-        for (int e = etid; e < TB * TB; e += 256) {
-          const int o = (e >> 6) * LDS + (e & 63);
-          dst[e] = j > 0 ? __fma_rn(-a.oz_sig2, sL[o], sC[o]) : sC[o];
-        }
-        next_points();
-      } else {
-        // L[i, j] U_j = C by blocked row solves (warp ew: rows 8 ew .. + 7),
-        // stored; forward substitution; int8 slices.
-        cp_async_wait<0>();
-        ws_sync();
-        const int r0 = 8 * ew;
-        warp_rows_trsm8_bi(sC + r0 * LDS, sX, sUi, lane, j > 0 ? sL + r0 * LDS : nullptr,
-                           a.oz_sig2);
-        next_points();
-        double lo[8], hi[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          lo[q] = sC[(r0 + q) * LDS + lane];
-          hi[q] = sC[(r0 + q) * LDS + 32 + lane];
-        }
-        {
-          double *Lg = W + int64_t(i) * TB * ld + int64_t(j) * TB;
-          double *rg = rcol + int64_t(i) * TB * ld;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            Lg[int64_t(r0 + q) * ld + lane] = lo[q];
-            Lg[int64_t(r0 + q) * ld + 32 + lane] = hi[q];
-          }
-          for (int f = 0; f < F; ++f) {
-            const double yl = ysh[lane * kMaxF + f], yh = ysh[(lane + 32) * kMaxF + f];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              double sum = __fma_rn(lo[q], yl, hi[q] * yh);
-              for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-              if (lane == 0) rg[int64_t(r0 + q) * ld + f] = rsh[(r0 + q) * kMaxF + f] - sum;
-            }
-          }
-        }
-        ws_sync();
-        {
-          uint8_t *dst = slice_row(sl, i) + int64_t(j) * kOzTileBytes;
-          slice_tile_smem(sC, TB, a.oz_mul, dst, dst, etid, 256);
-        }
+        for (int e = etid; e < TB * TB; e += kWsEpi)
+          dst[e] = sC[(rows0 + (e >> 6)) * LDS + (e & 63)];
+        continue;
       }
-      ws_sync();
+      // Warp ew's rows 8 ew .. + 7: L[i, j] U_j = C by blocked row solves, then
+      // from the registers the store, the forward substitution and the int8
+      // slices.
+      if (!mine) continue;
+      double c[8][2];
+      warp_rows_solve8<false>(sC + r0 * LDS, sX, sUi, lane, c);
+      if (late) release();
+      const int row = r0 + (lane >> 2), t2 = 2 * (lane & 3);
+      double *Lg = W + (int64_t(2 * u) * TB + row) * ld + int64_t(j) * TB + t2;
+#pragma unroll
+      for (int nt = 0; nt < 8; ++nt)
+        *reinterpret_cast<double2 *>(Lg + 8 * nt) = make_double2(c[nt][0], c[nt][1]);
+      double *rg = rcol + (int64_t(2 * u) * TB + row) * ld;
+      for (int f = 0; f < F; ++f) {
+        double sum = 0.0;
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+          sum = __fma_rn(c[nt][0], ysh[(8 * nt + t2) * kMaxF + f], sum);
+          sum = __fma_rn(c[nt][1], ysh[(8 * nt + t2 + 1) * kMaxF + f], sum);
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (t2 == 0) rg[f] = rsh[row * kMaxF + f] - sum;
+      }
+      slice_rows_acc(c, r0 & 63, lane, a.oz_mul, a.slices + sl.sli, sl.T, 2 * u + (r0 >> 6), j);
     }
     cp_async_wait<0>();
   }
@@ -1274,7 +1302,7 @@ __global__ void __launch_bounds__(kWsThreads, 1)
   // After a time-out, the patches of every item of this CTA's range are
   // marked for the FP64 LU.
   if (*abort_flag)
-    for (int it = it0 + tid; it < it1; it += kWsThreads)
+    for (int it = it0 + tid * step; it < it1; it += kWsThreads * step)
       atomicOr(&a.status[slots[ws_item(ipre, cnt, it).q].k], 8);
   tc_fence_before();
   __syncthreads();
@@ -1761,8 +1789,8 @@ CholPlan chol_prefix(const std::vector<BigSlot> &slots) {
     if (acc > 0x7fffffffll) throw Error{PACMAN_B200_ERR_LIMIT, "too many tiles in one launch"};
   }
   cp.off[steps] = int(cp.pre.size());
-  // Items of the warp-specialised int8 step: T - j per slot (its diagonal
-  // item, then its row tiles j + 1 .. T - 1).
+  // Items of the warp-specialised int8 step: per slot its diagonal item, then
+  // the pairs of row tiles that reach below row j.
   cp.ioff.resize(steps);
   for (int j = 0; j < steps; ++j) {
     const int c = cp.cnt[j];
@@ -1770,7 +1798,7 @@ CholPlan chol_prefix(const std::vector<BigSlot> &slots) {
     int64_t acc = 0;
     cp.pre.push_back(0);
     for (int q = 0; q < c; ++q) {
-      acc += slots[q].T - j;
+      acc += 1 + ws_pairs(slots[q].T, j);
       cp.pre.push_back(int(acc));
     }
     if (acc > 0x7fffffffll) throw Error{PACMAN_B200_ERR_LIMIT, "too many tiles in one launch"};
@@ -1948,6 +1976,6 @@ void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, cudaStream
   note_launch();
 }
 
-size_t oz_slot_bytes(int T) { return size_t(T) * size_t(T - 1) / 2 * size_t(kOzTileBytes); }
+size_t oz_slot_bytes(int T) { return size_t(oz_pair_off(T, (T + 1) / 2, 0)); }
 
 }  // namespace pacman_b200

@@ -7,6 +7,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace pacman_b200 {
@@ -95,6 +96,59 @@ __device__ __forceinline__ T wendland(int basis, T r, T rinv) {
   }
   }
   return mask * v;
+}
+
+// sqrt(x) for x >= 0 without branches: the hardware's 1 / sqrt(x) and one
+// Goldschmidt step for g ~ sqrt(x), h ~ 1 / (2 sqrt(x)), then the residual
+// correction g + (x - g g) h (Markstein, IBM J. Res. Dev. 34(1), 1990).  Zero
+// and what the approximation flushes give zero, overflowed squares pass.
+__device__ __forceinline__ double root(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  double g = x * y, h = 0.5 * y;
+  const double e = __fma_rn(-g, h, 0.5);
+  g = __fma_rn(g, e, g);
+  h = __fma_rn(h, e, h);
+  g = __fma_rn(__fma_rn(-g, g, x), h, g);
+  g = x < 1e-290 ? 0.0 : g;
+  return x > 1e290 ? x : g;
+}
+
+// phi at squared distance d2 (common.cuh: wendland with its mask, r >= 0).
+template <int B>
+__device__ __forceinline__ double phi_at(double d2, double rinv) {
+  const double p = root(d2) * rinv;
+  const double q = 1.0 - p, q2 = q * q;
+  double v;
+  if (B == kWendlandC0) {
+    v = q2;
+  } else if (B == kWendlandC2) {
+    v = (q2 * q2) * fma(4.0, p, 1.0);
+  } else if (B == kWendlandC4) {
+    v = (q2 * q2 * q2) * fma(35.0, p * p, fma(18.0, p, 3.0));
+  } else if (B == kWendlandC6) {
+    const double q4 = q2 * q2, p2 = p * p;
+    v = (q4 * q4) * (fma(32.0, p2 * p, 25.0 * p2) + fma(8.0, p, 1.0));
+  } else {
+    const double q4 = q2 * q2, p2 = p * p;
+    double t = fma(1287.0, p2 * p2, 1350.0 * p2 * p);
+    t = fma(630.0, p2, t);
+    v = (q4 * q4 * q2) * (t + fma(150.0, p, 15.0));
+  }
+  return p >= 1.0 ? 0.0 : v;
+}
+
+// Calls fn(basis constant) with the basis as a compile-time constant, so that
+// the loops inside hold no switch.
+template <typename Fn>
+__device__ __forceinline__ void with_basis(int basis, Fn &&fn) {
+  switch (basis) {
+  case kWendlandC0: fn(std::integral_constant<int, kWendlandC0>{}); break;
+  case kWendlandC2: fn(std::integral_constant<int, kWendlandC2>{}); break;
+  case kWendlandC4: fn(std::integral_constant<int, kWendlandC4>{}); break;
+  case kWendlandC6: fn(std::integral_constant<int, kWendlandC6>{}); break;
+  default: fn(std::integral_constant<int, kWendlandC8>{}); break;
+  }
 }
 
 // d phi / d p of the Wendland bases (p = r / rho), zero outside the support.
