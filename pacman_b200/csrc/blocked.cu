@@ -915,7 +915,7 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
                           g == 0 ? rep.tail_event : nullptr);
         // Each group sweeps and evaluates as soon as its own steps end, so
         // the sweeps overlap the other groups' last steps.
-        chol_launch_finish(a, gds[g], int(gs[g].size()), adjoint, sg);
+        chol_launch_finish(a, gds[g], int(gs[g].size()), chol_long_slots(gs[g]), adjoint, sg);
         if (adjoint) {
           k_big_adj_finish<<<int(gs[g].size()), 256, 0, sg>>>(a, gds[g]);
           note_launch();
@@ -933,6 +933,7 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
         w.act = a.act;
         w.red = a.red_out;
         w.ns = ns;
+        w.nlong = chol_long_slots(slots);
         for (const BigSlot &q : slots) w.sum_T += q.T;
         w.ds = ds;
         keep->waves.push_back(std::move(w));
@@ -1018,8 +1019,8 @@ void solve_big_cached(Plan &p, FactorCache &c, int basis, const double *vals, in
     PB_CUDA(cudaStreamWaitEvent(hs, p.aux.ev[AuxStreams::kN], 0));
     k_big_poly<<<w.ns, 256, 0, hs>>>(a, w.ds);
     note_launch();
-    chol_launch_forward(a, w.ds, w.ns, hs);
-    chol_launch_finish(a, w.ds, w.ns, false, hs);
+    chol_launch_forward(a, w.ds, w.ns, w.nlong, hs);
+    chol_launch_finish(a, w.ds, w.ns, w.nlong, false, hs);
     PB_CUDA(cudaEventRecord(p.aux.ev[0], hs));
     PB_CUDA(cudaStreamWaitEvent(st, p.aux.ev[0], 0));
     PB_CUDA(cudaGetLastError());

@@ -432,7 +432,7 @@ struct CholWaveCache {             // one wave of the large-patch engine
   DevMem small;                    // tile inverses, beta, act, slot tables
   double *inv = nullptr, *beta = nullptr, *red = nullptr;
   int *act = nullptr;
-  int ns = 0;
+  int ns = 0, nlong = 0;           // slots, and those swept by clusters
   int64_t sum_T = 0;               // zc holds sum_T * TB * kMaxF doubles (slot offsets)
   BigSlot *ds = nullptr;           // device slot table (in small), largest first
 };
@@ -454,8 +454,10 @@ struct FactorCache {
 inline size_t small_fac_doubles(int N) { return size_t(N) * N; }
 
 // Forward sweep L y = r from kept factors (an execute that reuses them).
-void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, cudaStream_t st);
-void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, bool adjoint,
+// nlong: how many of the ns slots, the first ones, a cluster sweeps.
+int chol_long_slots(const std::vector<BigSlot> &hs);
+void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, int nlong, cudaStream_t st);
+void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, int nlong, bool adjoint,
                         cudaStream_t st);
 
 }  // namespace pacman_b200

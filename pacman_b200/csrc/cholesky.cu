@@ -1327,16 +1327,40 @@ __global__ void __launch_bounds__(kWsThreads, 1)
 // (patch, source).  Every wait is bounded; a time-out marks the patch
 // (status 8), the CTA keeps its barrier sequence, stops issuing copies and
 // waits for the copies it issued before it returns.
+//
+// A slot of many tile rows is swept by a thread-block cluster of C CTAs (C = 1:
+// one CTA).  Level l solves block l of the sweep; rank r of the cluster holds
+// the solved blocks p = r (mod C): in every level it multiplies its own tiles
+// by its own blocks and sends the 64 x F partial sums to the level's solver,
+// rank l mod C, through distributed shared memory (an mbarrier there counts
+// the senders' warps).  The solver adds them in rank order and finishes the
+// block, which only it needs again.  A rank's partial of level l + C contains
+// a block solved after level l was consumed, so one receive buffer per rank
+// suffices.
 constexpr int kBkTile = TB * TB * 8;  // bytes of one stage
 // Ring depth: 3 stages for one or two fields, two CTAs per SM (the many short
 // slots are latency-bound, and a second CTA hides it); 5 stages, one CTA per
 // SM, for more fields (registers).
 constexpr int bk_stages(int F) { return F <= 2 ? 3 : 5; }
 
-size_t chol_back_smem(int F, int S = 0) {
-  // stages, part, accs, full/empty barriers, abort flag and issue counter
+// Cluster size for the slots with at least kBkLong tile rows, whose sweep one
+// SM's copy rate would draw out (15-30 GB/s: 5.8 ms for the slot group with T =
+// 78); its ring has four stages for eight fields (the receive buffer's room).
+// The line: a cluster's level costs about 4 us whatever its few tiles, so short
+// slots are faster one to an SM.  A kept-factor call at 400k refined points
+// takes 5.9, 5.0, 4.7, 5.1, 5.6, 5.5 ms with the line at 12, 24, 32, 40, 56 and
+// without clusters; the two sweep launches of a slot group at 1M 2.1 instead of
+// 4.5-5.8 ms.
+constexpr int kBkCluster = 8;
+constexpr int kBkLong = 32;
+constexpr int bk_cluster_stages(int F) { return F <= 2 ? 3 : 4; }
+
+size_t chol_back_smem(int F, int S = 0, int C = 1) {
+  // stages, part, accs, receive buffer, full/empty barriers, the receive
+  // barrier, abort flag and issue counter
   if (S == 0) S = bk_stages(F);
-  return size_t(S) * kBkTile + size_t(8 * TB * F + TB * F) * 8 + 2 * S * 8 + 16;
+  return size_t(S) * kBkTile + size_t(8 * TB * F + TB * F + (C > 1 ? C * TB * F : 0)) * 8 +
+         2 * S * 8 + 8 + 16;
 }
 // The deep ring of the one-field backward sweep (one CTA per SM, twice the
 // tiles in flight): a slot's sweep streams its T (T - 1) / 2 tiles through
@@ -1363,6 +1387,45 @@ __device__ __forceinline__ void warp_tile_g2s(double *dst, const double *src, in
                : "memory");
 }
 
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::
+                   : "memory");
+}
+// The address of this CTA's shared variable p in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(saddr(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar)
+               : "memory");
+}
+// Bounded wait for the partial sums of all ranks.
+__device__ __forceinline__ bool cluster_wait(uint64_t *b, uint32_t parity,
+                                             volatile int *abort_flag) {
+  for (int it = 0; it < kOzWaitLimit; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(saddr(b)), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (*abort_flag) return false;
+  }
+  return false;
+}
+
 // Bounded wait until item x is issued, then for its data.
 template <int kBkStages>
 __device__ __forceinline__ bool bk_wait_item(volatile int *issued, volatile int *abort_flag,
@@ -1375,18 +1438,21 @@ __device__ __forceinline__ bool bk_wait_item(volatile int *issued, volatile int 
   return ok && mbar_wait_abort(&full[x % kBkStages], uint32_t((x / kBkStages) & 1), abort_flag);
 }
 
-template <int KF, int kBkStages>  // fields held in registers (F <= KF), ring depth
+template <int KF, int kBkStages, int C = 1>  // fields in registers (F <= KF), ring depth, cluster
 __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
     k_chol_back(BigArgs a, const BigSlot *__restrict__ slots) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const BigSlot sl = slots[blockIdx.x];
+  const BigSlot sl = slots[blockIdx.x / C];
+  const int rank = C > 1 ? int(cluster_rank()) : 0;
   const int F = a.F, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double *stage0 = reinterpret_cast<double *>(smem);
   double *part = reinterpret_cast<double *>(smem + size_t(kBkStages) * kBkTile);  // [8][TB][F]
   double *accs = part + 8 * TB * F;                                                // [TB][F]
-  uint64_t *full = reinterpret_cast<uint64_t *>(accs + TB * F);
+  double *recv = accs + TB * F;                                                    // [C][TB][F]
+  uint64_t *full = reinterpret_cast<uint64_t *>(recv + (C > 1 ? C * TB * F : 0));
   uint64_t *empty = full + kBkStages;
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + kBkStages);
+  uint64_t *got = empty + kBkStages;
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(got + 1);
   // Items the producer has issued.  A consumer waits on the full barrier of
   // item x only once x is issued: x - kBkStages, the previous item of that
   // stage, has then landed and been released, so the barrier is in the
@@ -1402,17 +1468,20 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
       mbar_init(&full[i], 32);  // one arrival per producer lane
       mbar_init(&empty[i], 8);
     }
+    mbar_init(got, 8 * C);
     *abort_flag = 0;
     *issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  if (C > 1) cluster_sync_all();  // every rank's barriers are ready
   if (warp == 8) {
     // Producer: item g of the stream goes to stage g % kBkStages.
     int g = 0;
     bool ok = true;
-    for (int s = T - 1; s >= 0 && ok; --s) {
-      for (int t = s + 1; t <= T && ok; ++t, ++g) {  // t == T: X_s
+    for (int l = 0; l < T && ok; ++l) {
+      const int s = T - 1 - l, nq = l > rank ? (l - 1 - rank) / C + 1 : 0;
+      for (int q = 0; q < nq + (l % C == rank ? 1 : 0) && ok; ++q, ++g) {  // q == nq: X_s
         const int st = g % kBkStages, u = g / kBkStages;
         if (g >= kBkStages) {
           if (lane == 0) ok = mbar_wait_abort(&empty[st], uint32_t((u - 1) & 1), abort_flag);
@@ -1420,7 +1489,8 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
           if (!ok) break;
         }
         double *dst = reinterpret_cast<double *>(smem + size_t(st) * kBkTile);
-        if (t < T)
+        const int t = T - 1 - (rank + C * q);
+        if (q < nq)
           warp_tile_g2s(dst, W + int64_t(t) * TB * ld + int64_t(s) * TB, ld, lane, &full[st]);
         else
           warp_tile_g2s(dst, X0 + int64_t(s) * TB * TB, TB, lane, &full[st]);
@@ -1445,8 +1515,11 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
   } else {
     int g = 0;
     const int rr = tid & 63, quarter = tid >> 6;
-    for (int s = T - 1; s >= 0; --s) {
-      const int nt = T - 1 - s;
+    for (int l = 0; l < T; ++l) {
+      const int s = T - 1 - l;
+      const int nt = l > rank ? (l - 1 - rank) / C + 1 : 0;  // this rank's tiles of the level
+      // Block t of the rank's q-th tile.
+      auto block_of = [&](int q) { return T - 1 - (rank + C * q); };
       double acc0[KF], acc1[KF];
 #pragma unroll
       for (int f = 0; f < KF; ++f) acc0[f] = acc1[f] = 0.0;
@@ -1455,7 +1528,7 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
       // rows c are then broadcast from the lanes by shuffles.
       double zn0[KF], zn1[KF];
       if (warp < nt) {
-        const double *zt = zc + int64_t(s + 1 + warp) * TB * F;
+        const double *zt = zc + int64_t(block_of(warp)) * TB * F;
 #pragma unroll
         for (int f = 0; f < KF; ++f) {
           zn0[f] = f < F ? zt[lane * F + f] : 0.0;
@@ -1471,7 +1544,7 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
           z1[f] = zn1[f];
         }
         if (k + 8 < nt) {
-          const double *zt = zc + int64_t(s + 1 + k + 8) * TB * F;
+          const double *zt = zc + int64_t(block_of(k + 8)) * TB * F;
 #pragma unroll
           for (int f = 0; f < KF; ++f)
             if (f < F) {
@@ -1513,7 +1586,25 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
         double sum = 0.0;
 #pragma unroll
         for (int w = 0; w < 8; ++w) sum += part[(w * TB + r) * F + f];
-        accs[r * F + f] = rcol[int64_t(s * TB + r) * ld + f] - sum;
+        if (C == 1) accs[r * F + f] = rcol[int64_t(s * TB + r) * ld + f] - sum;
+        else cluster_store(cluster_addr(recv + rank * TB * F + e, l % C), sum);
+      }
+      if (C > 1) {
+        __syncwarp();
+        if (lane == 0) cluster_arrive(cluster_addr(got, l % C));
+        if (l % C != rank) {
+          // part is written again in the next level.
+          asm volatile("bar.sync 1, 256;\n" ::: "memory");
+          continue;
+        }
+        if (!cluster_wait(got, uint32_t((l / C) & 1), abort_flag)) *abort_flag = 1;
+        for (int e = tid; e < TB * F; e += 256) {
+          const int r = e / F, f = e % F;
+          double sum = 0.0;
+#pragma unroll
+          for (int c = 0; c < C; ++c) sum += recv[c * TB * F + e];
+          accs[e] = rcol[int64_t(s * TB + r) * ld + f] - sum;
+        }
       }
       // X_s: every consumer warp reads it, each releases one of 8 arrivals.
       const int st = g % kBkStages;
@@ -1556,6 +1647,7 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
     if (tid == 0 && *abort_flag) atomicOr(&a.status[sl.k], 8);
   }
   __syncthreads();
+  if (C > 1) cluster_sync_all();  // no rank leaves while others write to it
 }
 
 // Forward sweep L y = r of one slot from kept factors (CTA per slot), for
@@ -1567,17 +1659,20 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
 // cp.async ring as k_chol_back; every consumer warp reads
 // every tile: warp w owns rows 8w .. 8w + 7 and its lanes the columns c and
 // c + 32, so the partial sums stay in registers until the level ends.
-template <int KF, int kBkStages>  // fields held in registers (F <= KF), ring depth
+template <int KF, int kBkStages, int C = 1>  // fields in registers (F <= KF), ring depth, cluster
 __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
     k_chol_fwd(BigArgs a, const BigSlot *__restrict__ slots) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const BigSlot sl = slots[blockIdx.x];
+  const BigSlot sl = slots[blockIdx.x / C];
+  const int rank = C > 1 ? int(cluster_rank()) : 0;
   const int F = a.F, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double *stage0 = reinterpret_cast<double *>(smem);
   double *accs = reinterpret_cast<double *>(smem + size_t(kBkStages) * kBkTile);  // [TB][F]
-  uint64_t *full = reinterpret_cast<uint64_t *>(accs + 9 * TB * F);
+  double *recv = accs + TB * F;                                                    // [C][TB][F]
+  uint64_t *full = reinterpret_cast<uint64_t *>(recv + (C > 1 ? C * TB * F : 0));
   uint64_t *empty = full + kBkStages;
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + kBkStages);
+  uint64_t *got = empty + kBkStages;
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(got + 1);
   volatile int *issued = abort_flag + 1;  // as in k_chol_back
   const int ld = sl.ld, T = sl.T;
   const double *W = a.W + sl.base;
@@ -1588,16 +1683,20 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
       mbar_init(&full[i], 32);  // one arrival per producer lane
       mbar_init(&empty[i], 8);
     }
+    mbar_init(got, 8 * C);
     *abort_flag = 0;
     *issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
+  if (C > 1) cluster_sync_all();  // every rank's barriers are ready
   if (warp == 8) {
     int g = 0;
     bool ok = true;
     for (int s = 0; s < T && ok; ++s) {
-      for (int t = 0; t <= s && ok; ++t, ++g) {  // t == s: X_s
+      const int nq = s > rank ? (s - 1 - rank) / C + 1 : 0;
+      for (int q = 0; q < nq + (s % C == rank ? 1 : 0) && ok; ++q, ++g) {  // q == nq: X_s
+        const int t = rank + C * q;
         const int st = g % kBkStages, u = g / kBkStages;
         if (g >= kBkStages) {
           if (lane == 0) ok = mbar_wait_abort(&empty[st], uint32_t((u - 1) & 1), abort_flag);
@@ -1605,7 +1704,7 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
           if (!ok) break;
         }
         double *dst = reinterpret_cast<double *>(smem + size_t(st) * kBkTile);
-        if (t < s)
+        if (q < nq)
           warp_tile_g2s(dst, W + int64_t(s) * TB * ld + int64_t(t) * TB, ld, lane, &full[st]);
         else
           warp_tile_g2s(dst, X0 + int64_t(s) * TB * TB, TB, lane, &full[st]);
@@ -1639,18 +1738,19 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
       double yn0[KF], yn1[KF];
 #pragma unroll
       for (int f = 0; f < KF; ++f) {
-        yn0[f] = (s > 0 && f < F) ? rcol[int64_t(lane) * ld + f] : 0.0;
-        yn1[f] = (s > 0 && f < F) ? rcol[int64_t(lane + 32) * ld + f] : 0.0;
+        const double *y0 = rcol + int64_t(rank) * TB * ld;
+        yn0[f] = (rank < s && f < F) ? y0[int64_t(lane) * ld + f] : 0.0;
+        yn1[f] = (rank < s && f < F) ? y0[int64_t(lane + 32) * ld + f] : 0.0;
       }
-      for (int t = 0; t < s; ++t, ++g) {
+      for (int t = rank; t < s; t += C, ++g) {
         double y0[KF], y1[KF];
 #pragma unroll
         for (int f = 0; f < KF; ++f) {
           y0[f] = yn0[f];
           y1[f] = yn1[f];
         }
-        if (t + 1 < s) {
-          const double *yt = rcol + int64_t(t + 1) * TB * ld;
+        if (t + C < s) {
+          const double *yt = rcol + int64_t(t + C) * TB * ld;
 #pragma unroll
           for (int f = 0; f < KF; ++f)
             if (f < F) {
@@ -1683,8 +1783,22 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
           if (f < F) {
             double v = part[r][f];
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) accs[(r0 + r) * F + f] = rcol[int64_t(s * TB + r0 + r) * ld + f] - v;
+            if (lane != 0) continue;
+            if (C == 1) accs[(r0 + r) * F + f] = rcol[int64_t(s * TB + r0 + r) * ld + f] - v;
+            else cluster_store(cluster_addr(recv + rank * TB * F + (r0 + r) * F + f, s % C), v);
           }
+      if (C > 1) {
+        if (lane == 0) cluster_arrive(cluster_addr(got, s % C));
+        if (s % C != rank) continue;
+        if (!cluster_wait(got, uint32_t((s / C) & 1), abort_flag)) *abort_flag = 1;
+        for (int e = lane; e < 8 * F; e += 32) {  // the warp's rows
+          const int r = r0 + e / F, f = e % F;
+          double sum = 0.0;
+#pragma unroll
+          for (int c = 0; c < C; ++c) sum += recv[c * TB * F + r * F + f];
+          accs[r * F + f] = rcol[int64_t(s * TB + r) * ld + f] - sum;
+        }
+      }
       bool okx = !*abort_flag;
       if (okx) okx = bk_wait_item<kBkStages>(issued, abort_flag, full, g);
       if (!okx) *abort_flag = 1;
@@ -1714,12 +1828,13 @@ __global__ void __launch_bounds__(288, kBkStages == 3 ? 2 : 1)
     if (tid == 0 && *abort_flag) atomicOr(&a.status[sl.k], 8);
   }
   __syncthreads();
+  if (C > 1) cluster_sync_all();  // no rank leaves while others write to it
 }
 
-size_t chol_fwd_smem(int F) {
-  // stages, accs (with room), full/empty barriers, abort flag and issue counter
-  const int S = bk_stages(F);
-  return size_t(S) * kBkTile + size_t(9 * TB * F) * 8 + 2 * S * 8 + 16;
+size_t chol_fwd_smem(int F, int S = 0, int C = 1) {
+  // as chol_back_smem without part
+  if (S == 0) S = bk_stages(F);
+  return size_t(S) * kBkTile + size_t(TB * F + (C > 1 ? C * TB * F : 0)) * 8 + 2 * S * 8 + 8 + 16;
 }
 
 // local = E alpha + V beta for the targets of one slot (warp per target).
@@ -1822,7 +1937,10 @@ void chol_set_smem_attributes() {
   {
 #define PB_SWEEP_ATTR(K, F)                                                                   \
   PB_CUDA(cudaFuncSetAttribute(K<F, bk_stages(F)>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                               int(std::max(chol_back_smem(F), chol_fwd_smem(F)))))
+                               int(std::max(chol_back_smem(F), chol_fwd_smem(F)))));         \
+  PB_CUDA(cudaFuncSetAttribute(K<F, bk_cluster_stages(F), kBkCluster>,                          \
+                               cudaFuncAttributeMaxDynamicSharedMemorySize,                   \
+                               int(chol_back_smem(F, bk_cluster_stages(F), kBkCluster))))
     PB_SWEEP_ATTR(k_chol_back, 1);
     PB_CUDA(cudaFuncSetAttribute(k_chol_back<1, kBkDeep>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1949,31 +2067,76 @@ void finish_kernel_timing(SolveReport &rep, cudaEvent_t ref) {
   rep.ms_update += span[2];
 }
 
-void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, bool adjoint,
+int chol_long_slots(const std::vector<BigSlot> &hs) {
+  int c = 0;
+  while (c < int(hs.size()) && hs[c].T >= kBkLong) ++c;
+  return c;
+}
+
+namespace {
+
+// The first nlong slots by clusters, the others by single CTAs.
+template <typename Single, typename Long>
+void launch_sweep(const BigArgs &a, const BigSlot *ds, int ns, int nlong, size_t smem,
+                  size_t smem_long, Single single, Long clusters, cudaStream_t st) {
+  if (nlong > 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nlong * kBkCluster);
+    cfg.blockDim = dim3(288);
+    cfg.dynamicSmemBytes = smem_long;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kBkCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PB_CUDA(cudaLaunchKernelEx(&cfg, clusters, a, ds));
+    note_launch();
+  }
+  if (ns > nlong) {
+    single<<<ns - nlong, 288, smem, st>>>(a, ds + nlong);
+    note_launch();
+  }
+}
+
+}  // namespace
+
+void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, int nlong, bool adjoint,
                         cudaStream_t st) {
-  const size_t smem = chol_back_smem(a.F);
+  auto go = [&](auto F, auto single, int S) {
+    constexpr int kF = decltype(F)::value, kS = bk_cluster_stages(kF);
+    launch_sweep(a, ds, ns, nlong, chol_back_smem(a.F, S), chol_back_smem(a.F, kS, kBkCluster),
+                 single, k_chol_back<kF, kS, kBkCluster>, st);
+  };
   const bool deep = tuned_int("PACMAN_B200_BACK_STAGES", tuning_for_current_device().back_stages) ==
                     kBkDeep;
-  if (a.F == 1 && deep)
-    k_chol_back<1, kBkDeep><<<ns, 288, chol_back_smem(1, kBkDeep), st>>>(a, ds);
-  else if (a.F == 1) k_chol_back<1, bk_stages(1)><<<ns, 288, smem, st>>>(a, ds);
-  else if (a.F <= 2) k_chol_back<2, bk_stages(2)><<<ns, 288, smem, st>>>(a, ds);
-  else if (a.F <= 4) k_chol_back<4, bk_stages(4)><<<ns, 288, smem, st>>>(a, ds);
-  else k_chol_back<kMaxF, bk_stages(kMaxF)><<<ns, 288, smem, st>>>(a, ds);
-  note_launch();
+  using std::integral_constant;
+  if (a.F == 1 && deep) go(integral_constant<int, 1>{}, k_chol_back<1, kBkDeep>, kBkDeep);
+  else if (a.F == 1) go(integral_constant<int, 1>{}, k_chol_back<1, bk_stages(1)>, bk_stages(1));
+  else if (a.F <= 2) go(integral_constant<int, 2>{}, k_chol_back<2, bk_stages(2)>, bk_stages(2));
+  else if (a.F <= 4) go(integral_constant<int, 4>{}, k_chol_back<4, bk_stages(4)>, bk_stages(4));
+  else go(integral_constant<int, kMaxF>{}, k_chol_back<kMaxF, bk_stages(kMaxF)>, bk_stages(kMaxF));
   if (!adjoint) {
     k_chol_eval<<<ns, 256, 0, st>>>(a, ds);
     note_launch();
   }
 }
 
-void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, cudaStream_t st) {
-  const size_t smem = chol_fwd_smem(a.F);
-  if (a.F == 1) k_chol_fwd<1, bk_stages(1)><<<ns, 288, smem, st>>>(a, ds);
-  else if (a.F <= 2) k_chol_fwd<2, bk_stages(2)><<<ns, 288, smem, st>>>(a, ds);
-  else if (a.F <= 4) k_chol_fwd<4, bk_stages(4)><<<ns, 288, smem, st>>>(a, ds);
-  else k_chol_fwd<kMaxF, bk_stages(kMaxF)><<<ns, 288, smem, st>>>(a, ds);
-  note_launch();
+void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, int nlong,
+                         cudaStream_t st) {
+  auto go = [&](auto F) {
+    constexpr int kF = decltype(F)::value, kS = bk_cluster_stages(kF);
+    launch_sweep(a, ds, ns, nlong, chol_fwd_smem(a.F, bk_stages(kF)),
+                 chol_fwd_smem(a.F, kS, kBkCluster), k_chol_fwd<kF, bk_stages(kF)>,
+                 k_chol_fwd<kF, kS, kBkCluster>, st);
+  };
+  using std::integral_constant;
+  if (a.F == 1) go(integral_constant<int, 1>{});
+  else if (a.F <= 2) go(integral_constant<int, 2>{});
+  else if (a.F <= 4) go(integral_constant<int, 4>{});
+  else go(integral_constant<int, kMaxF>{});
 }
 
 size_t oz_slot_bytes(int T) { return size_t(oz_pair_off(T, (T + 1) / 2, 0)); }
