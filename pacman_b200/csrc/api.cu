@@ -45,6 +45,24 @@ HostArena &HostArena::get() {
   return arena;
 }
 
+namespace {
+
+// Blocks of arenas whose threads have ended (a batch's geometry threads live
+// for one call, and a pinned allocation takes milliseconds): at most
+// kMaxIdleBlocks of at most kMaxIdleBytes each, the rest is freed.  Never
+// destroyed: the CUDA runtime may be gone when statics are.
+constexpr size_t kMaxIdleBlocks = 16, kMaxIdleBytes = size_t(4) << 20;
+struct IdleBlocks {
+  std::mutex mu;
+  std::vector<std::pair<char *, size_t>> blocks;
+};
+IdleBlocks &idle_blocks() {
+  static IdleBlocks *idle = new IdleBlocks;
+  return *idle;
+}
+
+}  // namespace
+
 void HostArena::reset() {
   for (char *b : retired_) cudaFreeHost(b);
   retired_.clear();
@@ -56,7 +74,17 @@ void *HostArena::alloc(size_t bytes) {
   if (used_ + bytes > cap_) {
     size_t cap = std::max<size_t>(cap_ * 2, std::max<size_t>(bytes, size_t(1) << 20));
     char *nb = nullptr;
-    if (cudaHostAlloc(reinterpret_cast<void **>(&nb), cap, cudaHostAllocDefault) != cudaSuccess) {
+    if (!base_) {
+      IdleBlocks &idle = idle_blocks();
+      std::lock_guard<std::mutex> lock(idle.mu);
+      for (size_t i = 0; i < idle.blocks.size() && !nb; ++i)
+        if (idle.blocks[i].second >= bytes) {
+          nb = idle.blocks[i].first;
+          cap = idle.blocks[i].second;
+          idle.blocks.erase(idle.blocks.begin() + std::ptrdiff_t(i));
+        }
+    }
+    if (!nb && cudaHostAlloc(reinterpret_cast<void **>(&nb), cap, cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       throw Error{PACMAN_B200_ERR_NOMEM, "pinned host staging allocation failed"};
     }
@@ -72,7 +100,16 @@ void *HostArena::alloc(size_t bytes) {
 
 HostArena::~HostArena() {
   reset();
-  if (base_) cudaFreeHost(base_);
+  if (!base_) return;
+  if (cap_ <= kMaxIdleBytes) {
+    IdleBlocks &idle = idle_blocks();
+    std::lock_guard<std::mutex> lock(idle.mu);
+    if (idle.blocks.size() < kMaxIdleBlocks) {
+      idle.blocks.emplace_back(base_, cap_);
+      return;
+    }
+  }
+  cudaFreeHost(base_);
 }
 
 namespace {
