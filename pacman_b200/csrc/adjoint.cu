@@ -40,12 +40,12 @@ struct WeightTerm {
 // Centres within r of y in ascending order, with their C2 weights and
 // weight gradients.  Returns the count (cnt > kMaxC: only the first kMaxC
 // are stored and the caller re-scans).
-__device__ int centre_terms(const GridView &cg, const double4 *centers, double4 y, double r,
-                            double rinv, WeightTerm *out, int after, bool want_grad) {
+__device__ int centre_terms(const GridView &cg, double4 y, double r, double rinv, WeightTerm *out,
+                            int after, bool want_grad) {
   int cnt = 0;
-  for_neighbors(cg, y.x, y.y, y.z, [&](int k) {
+  for_neighbors(cg, y.x, y.y, y.z, [&](const double4 &c) {
+    const int k = int(c.w);
     if (k <= after) return;
-    const double4 c = centers[k];
     const double d = __dsqrt_rn(sqdist3(y.x, y.y, y.z, c.x, c.y, c.z));
     if (!(d <= r)) return;
     if (cnt < kMaxC) {
@@ -72,17 +72,18 @@ __device__ int centre_terms(const GridView &cg, const double4 *centers, double4 
 }
 
 // S_t (and grad S_t) in ascending centre order, as the forward gather sums it.
-__global__ void k_weight_sums(int64_t M, const double4 *__restrict__ tgt, GridView cg,
-                              const double4 *__restrict__ centers, double r, double rinv,
+__global__ void k_weight_sums(int64_t M, const int *__restrict__ torder,
+                              const double4 *__restrict__ tgt, GridView cg, double r, double rinv,
                               double *wsum, double *wgrad) {
   WeightTerm terms[kMaxC];
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < M;
-       t += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < M;
+       it += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = torder[it];
     const double4 y = tgt[t];
     double S = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
     int after = -1;
     for (;;) {
-      const int cnt = centre_terms(cg, centers, y, r, rinv, terms, after, wgrad != nullptr);
+      const int cnt = centre_terms(cg, y, r, rinv, terms, after, wgrad != nullptr);
       const int c = cnt < kMaxC ? cnt : kMaxC;
       for (int i = 0; i < c; ++i) {
         S = __dadd_rn(S, terms[i].w);
@@ -252,25 +253,24 @@ __device__ __forceinline__ int64_t find_sorted(const int *a, int64_t n, int v) {
 }
 
 // d (sum_f G_f out_f) / d y per target.
-__global__ void k_target_grad(int64_t M, const int *__restrict__ tlist, int dim,
-                              const double4 *__restrict__ tgt, GridView cg,
-                              const double4 *__restrict__ centers, double r, double rinv,
+__global__ void k_target_grad(int64_t M, const int *__restrict__ torder, int dim,
+                              const double4 *__restrict__ tgt, GridView cg, double r, double rinv,
                               const double *__restrict__ wsum, const double *__restrict__ wgrad,
                               const int64_t *__restrict__ toff, const int *__restrict__ tidx,
                               const double *__restrict__ local, const double *__restrict__ dloc,
                               const double *__restrict__ gout, int F, double *grad) {
   WeightTerm terms[kMaxC];
-  // M targets: all (tlist null) or those of a shard's list.
+  // The M targets of torder: all, or those of a shard's list.
   for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < M;
        it += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t t = tlist ? tlist[it] : it;
+    const int64_t t = torder[it];
     const double4 y = tgt[t];
     const double S = wsum[t];
     const double gS[3] = {wgrad[3 * t], wgrad[3 * t + 1], wgrad[3 * t + 2]};
     double acc[3] = {0.0, 0.0, 0.0};
     int after = -1;
     for (;;) {
-      const int cnt = centre_terms(cg, centers, y, r, rinv, terms, after, true);
+      const int cnt = centre_terms(cg, y, r, rinv, terms, after, true);
       const int c = cnt < kMaxC ? cnt : kMaxC;
       for (int i = 0; i < c; ++i) {
         const int k = terms[i].k;
@@ -370,7 +370,7 @@ void adjoint(Plan &p, const double *gout, double *grad_values, double *grad_targ
   wsum.alloc(sizeof(double) * M, st);
   if (grad_targets) wgrad.alloc(sizeof(double) * 3 * M, st);
   k_weight_sums<<<blocks_for(M, 128, 148 * 64), 128, 0, st>>>(
-      M, p.tgt4.as<double4>(), p.cgrid.view, p.centers.as<double4>(), r, rinv, wsum.as<double>(),
+      M, p.torder.as<int>(), p.tgt4.as<double4>(), p.cgrid.view, r, rinv, wsum.as<double>(),
       grad_targets ? wgrad.as<double>() : nullptr);
   note_launch();
   if (grad_values) {
@@ -406,8 +406,8 @@ void adjoint(Plan &p, const double *gout, double *grad_values, double *grad_targ
     const int64_t Mg = sharded ? p.m_owned : M;
     if (Mg > 0) {
       k_target_grad<<<blocks_for(Mg, 128, 148 * 64), 128, 0, st>>>(
-          Mg, sharded ? p.tlist.as<int>() : nullptr, p.dim, p.tgt4.as<double4>(), p.cgrid.view,
-          p.centers.as<double4>(), r, rinv, wsum.as<double>(), wgrad.as<double>(),
+          Mg, sharded ? p.tlist.as<int>() : p.torder.as<int>(), p.dim, p.tgt4.as<double4>(),
+          p.cgrid.view, r, rinv, wsum.as<double>(), wgrad.as<double>(),
           p.toff.as<int64_t>(), p.tidx.as<int>(), p.local.as<double>(), dloc.as<double>(), gout,
           F, grad_targets);
       note_launch();

@@ -192,7 +192,9 @@ struct GridView {
   int nc[3];
   int ncells;
   const int *start;  // ncells + 1
-  const int *items;  // point ids grouped by cell, ascending within a cell
+  // The grid of centres: the points grouped by cell, ids (in w) ascending
+  // within a cell.
+  const double4 *sorted;
 };
 
 __device__ __forceinline__ int cell_coord(double x, double lo, double inv_h, int nc) {
@@ -201,7 +203,7 @@ __device__ __forceinline__ int cell_coord(double x, double lo, double inv_h, int
   return c;
 }
 
-// Calls fn(point_id) for every point in the 3^3 cells around q.
+// Calls fn(point) for every point of g.sorted in the 3^3 cells around q.
 template <typename Fn>
 __device__ __forceinline__ void for_neighbors(const GridView &g, double qx, double qy,
                                               double qz, Fn &&fn) {
@@ -216,7 +218,7 @@ __device__ __forceinline__ void for_neighbors(const GridView &g, double qx, doub
       const int base = (a * g.nc[1] + b) * g.nc[2];
       const int s = g.start[base + z0];
       const int e = g.start[base + z1 + 1];
-      for (int i = s; i < e; ++i) fn(g.items[i]);
+      for (int i = s; i < e; ++i) fn(g.sorted[i]);
     }
 }
 

@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(128)
     k_mls_search(int64_t t0, int64_t M, GridView g, const double4 *__restrict__ sorted, double h,
                  int *__restrict__ nbr) {
   constexpr int K = Mls<DIM>::K;
-  const double4 *tgt = sorted + g.start[g.ncells] + t0;
+  const double4 *tgt = sorted + g.start[g.ncells + 1] + t0;
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < M;
        t += int64_t(gridDim.x) * blockDim.x) {
     const double4 y = tgt[t];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(128, 2)
   constexpr int NP = Mls<DIM>::NP;
   __shared__ double us[K][128], vs[K][128];
   const MlsColumn u{&us[0][threadIdx.x]}, b{&vs[0][threadIdx.x]};
-  const double4 *tgt = sorted + g.start[g.ncells] + t0;
+  const double4 *tgt = sorted + g.start[g.ncells + 1] + t0;
   const int kk = n < K ? int(n) : K;
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < M;
        t += int64_t(gridDim.x) * blockDim.x) {

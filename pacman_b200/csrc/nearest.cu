@@ -25,7 +25,7 @@ namespace {
 template <int DIM>
 __global__ void k_fe_nearest(int64_t M, GridView g, const double4 *__restrict__ sorted, double h,
                              const double *__restrict__ vals, double *__restrict__ out) {
-  const double4 *tgt = sorted + g.start[g.ncells];
+  const double4 *tgt = sorted + g.start[g.ncells + 1];
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < M;
        t += int64_t(gridDim.x) * blockDim.x) {
     const double4 y = tgt[t];

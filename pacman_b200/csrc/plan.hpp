@@ -76,7 +76,7 @@ struct DevMem {
 
 struct DevGrid {
   GridView view{};
-  DevMem start, items;
+  DevMem start, sorted;
 };
 
 // Extra streams of a call, taken on first use for the plan's device: one per
@@ -143,6 +143,7 @@ struct Plan {
   int64_t snnz = 0, tnnz = 0;
   std::vector<int> n_host, m_host;  // per patch sizes
   DevGrid cgrid;                    // grid of centres (weights)
+  DevMem torder;                    // targets in the order of the search grid's cells
   DevMem scratch;                   // solver workspace
   DevMem local;                     // per (patch, target) local values
   DevMem status;                    // per patch status words
@@ -239,7 +240,7 @@ double geometry_ms(Plan &p);
 void pu_gather(Plan &p, const double *local, int F, double *out_dev);
 // Packed points of a nearest-neighbour search, sorted into the cells of a
 // uniform grid over the sources with their ids in w: the sources, then from
-// grid.start[grid.ncells] on the targets (geometry.cu).
+// grid.start[grid.ncells + 1] on the targets (geometry.cu).
 struct PointSearch {
   DevMem src4, tgt4, mem;
   GridView grid{};               // start only
