@@ -693,6 +693,26 @@ int pipeline_wait_limit() {
   return 1 << 22;
 }
 
+// Runs fn(first slot, slots, clusters, stream) for the nlong long slots of a
+// list on st and for the others beside them, on the aux stream of index `alt`
+// (with event `alt`), joined back: neither set fills the GPU alone, and their
+// sweeps are chains.
+template <typename Fn>
+static void beside_long(AuxStreams &aux, int alt, int ns, int nlong, cudaStream_t st, Fn &&fn) {
+  const bool split = nlong > 0 && nlong < ns;
+  cudaStream_t other = split ? aux.s[alt] : st;
+  if (split) {
+    PB_CUDA(cudaEventRecord(aux.ev[alt], st));
+    PB_CUDA(cudaStreamWaitEvent(other, aux.ev[alt], 0));
+  }
+  if (nlong > 0) fn(0, nlong, true, st);
+  if (nlong < ns) fn(nlong, ns - nlong, false, other);
+  if (split) {
+    PB_CUDA(cudaEventRecord(aux.ev[alt], other));
+    PB_CUDA(cudaStreamWaitEvent(st, aux.ev[alt], 0));
+  }
+}
+
 void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
                const std::vector<int> &patches, double *local, int *status, SolveReport &rep,
                const BigExtra &extra, FactorCache *keep) {
@@ -915,7 +935,11 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
                           g == 0 ? rep.tail_event : nullptr);
         // Each group sweeps and evaluates as soon as its own steps end, so
         // the sweeps overlap the other groups' last steps.
-        chol_launch_finish(a, gds[g], int(gs[g].size()), chol_long_slots(gs[g]), adjoint, sg);
+        const int alt = G <= AuxStreams::kN / 2 ? g + AuxStreams::kN / 2 : g;
+        beside_long(p.aux, alt, ng, alt == g ? 0 : chol_long_slots(gs[g]), sg,
+                    [&](int first, int cnt, bool clusters, cudaStream_t s2) {
+                      chol_launch_finish(a, gds[g] + first, cnt, clusters, adjoint, s2);
+                    });
         if (adjoint) {
           k_big_adj_finish<<<int(gs[g].size()), 256, 0, sg>>>(a, gds[g]);
           note_launch();
@@ -1019,8 +1043,11 @@ void solve_big_cached(Plan &p, FactorCache &c, int basis, const double *vals, in
     PB_CUDA(cudaStreamWaitEvent(hs, p.aux.ev[AuxStreams::kN], 0));
     k_big_poly<<<w.ns, 256, 0, hs>>>(a, w.ds);
     note_launch();
-    chol_launch_forward(a, w.ds, w.ns, w.nlong, hs);
-    chol_launch_finish(a, w.ds, w.ns, w.nlong, false, hs);
+    beside_long(p.aux, 1, w.ns, w.nlong, hs,
+                [&](int first, int cnt, bool clusters, cudaStream_t s2) {
+                  chol_launch_forward(a, w.ds + first, cnt, clusters, s2);
+                  chol_launch_finish(a, w.ds + first, cnt, clusters, false, s2);
+                });
     PB_CUDA(cudaEventRecord(p.aux.ev[0], hs));
     PB_CUDA(cudaStreamWaitEvent(st, p.aux.ev[0], 0));
     PB_CUDA(cudaGetLastError());

@@ -454,10 +454,12 @@ struct FactorCache {
 inline size_t small_fac_doubles(int N) { return size_t(N) * N; }
 
 // Forward sweep L y = r from kept factors (an execute that reuses them).
-// nlong: how many of the ns slots, the first ones, a cluster sweeps.
+// Sweeps and evaluation of ns slots, by clusters (the slots that
+// chol_long_slots counts at the front of a list) or by single CTAs.
 int chol_long_slots(const std::vector<BigSlot> &hs);
-void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, int nlong, cudaStream_t st);
-void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, int nlong, bool adjoint,
+void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, bool clusters,
+                         cudaStream_t st);
+void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, bool clusters, bool adjoint,
                         cudaStream_t st);
 
 }  // namespace pacman_b200

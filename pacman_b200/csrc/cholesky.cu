@@ -2120,15 +2120,15 @@ int chol_long_slots(const std::vector<BigSlot> &hs) {
 
 namespace {
 
-// The first nlong slots by clusters, the others by single CTAs.
+// One sweep over ns slots, by clusters or by single CTAs.
 template <typename Single, typename Long>
-void launch_sweep(const BigArgs &a, const BigSlot *ds, int ns, int nlong, size_t smem,
-                  size_t smem_long, Single single, Long clusters, cudaStream_t st) {
-  if (nlong > 0) {
+void launch_sweep(const BigArgs &a, const BigSlot *ds, int ns, bool clusters, size_t smem,
+                  size_t smem_cluster, Single single, Long cluster, cudaStream_t st) {
+  if (clusters) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nlong * kBkCluster);
+    cfg.gridDim = dim3(ns * kBkCluster);
     cfg.blockDim = dim3(288);
-    cfg.dynamicSmemBytes = smem_long;
+    cfg.dynamicSmemBytes = smem_cluster;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2137,22 +2137,20 @@ void launch_sweep(const BigArgs &a, const BigSlot *ds, int ns, int nlong, size_t
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PB_CUDA(cudaLaunchKernelEx(&cfg, clusters, a, ds));
-    note_launch();
+    PB_CUDA(cudaLaunchKernelEx(&cfg, cluster, a, ds));
+  } else {
+    single<<<ns, 288, smem, st>>>(a, ds);
   }
-  if (ns > nlong) {
-    single<<<ns - nlong, 288, smem, st>>>(a, ds + nlong);
-    note_launch();
-  }
+  note_launch();
 }
 
 }  // namespace
 
-void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, int nlong, bool adjoint,
+void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, bool clusters, bool adjoint,
                         cudaStream_t st) {
   auto go = [&](auto F, auto single, int S) {
     constexpr int kF = decltype(F)::value, kS = bk_cluster_stages(kF);
-    launch_sweep(a, ds, ns, nlong, chol_back_smem(a.F, S), chol_back_smem(a.F, kS, kBkCluster),
+    launch_sweep(a, ds, ns, clusters, chol_back_smem(a.F, S), chol_back_smem(a.F, kS, kBkCluster),
                  single, k_chol_back<kF, kS, kBkCluster>, st);
   };
   const bool deep = tuned_int("PACMAN_B200_BACK_STAGES", tuning_for_current_device().back_stages) ==
@@ -2173,11 +2171,11 @@ void chol_launch_finish(const BigArgs &a, const BigSlot *ds, int ns, int nlong, 
   }
 }
 
-void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, int nlong,
+void chol_launch_forward(const BigArgs &a, const BigSlot *ds, int ns, bool clusters,
                          cudaStream_t st) {
   auto go = [&](auto F) {
     constexpr int kF = decltype(F)::value, kS = bk_cluster_stages(kF);
-    launch_sweep(a, ds, ns, nlong, chol_fwd_smem(a.F, bk_stages(kF)),
+    launch_sweep(a, ds, ns, clusters, chol_fwd_smem(a.F, bk_stages(kF)),
                  chol_fwd_smem(a.F, kS, kBkCluster), k_chol_fwd<kF, bk_stages(kF)>,
                  k_chol_fwd<kF, kS, kBkCluster>, st);
   };
