@@ -54,10 +54,13 @@ struct PatchArgs {
   int fac_mode;
 };
 
-// Register-resident LU of the patches with n <= kSmallMax (small.cu).  The
-// list of launch_small_lu holds patches of one size class N = small_class(n);
-// launch_small_poly must have run on the same list (pbeta, pact, status).
-constexpr int kSmallMax = 64;
+// Register-resident LU of the patches with n <= kSmallWide (small.cu), in size
+// classes up to kSmallMax and one above, whose other choice is a shared-memory
+// LU with two block barriers per pivot (one patch of 70 sources: 142 us there,
+// 44 here).  The list of launch_small_lu holds patches of one size class
+// N = small_class(n); launch_small_poly must have run on the same list (pbeta,
+// pact, status).
+constexpr int kSmallMax = 64, kSmallWide = 96;
 int small_class(int n);
 void launch_small_poly(const PatchArgs &a, const int *plist, int np, bool adj, cudaStream_t st);
 void launch_small_lu(const PatchArgs &a, const int *plist, int np, int N, bool adj,

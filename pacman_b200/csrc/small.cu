@@ -1,4 +1,4 @@
-// Register-resident solver for the small patches (n <= 64) of the B200
+// Register-resident solver for the small patches (n <= 96) of the B200
 // RBF-PUM transfer: both precisions of the forward transfer and the adjoint.
 //
 // Per patch (src/rbf_pum/solver/solver.hpp:180-286): A = phi(|x_i - x_j|),
@@ -31,6 +31,10 @@
 // patches): all small-patch launches 2.1 ms, against 8.6 ms for a 256-thread
 // team per patch on the padded 64 x 64 block with the explicit L^{-1}; 200,000
 // points, C6, 1 field, FP64: 0.77 ms against 4.5 ms for the shared-memory LU.
+// The class of 65 to 96 sources is three warps at 255 registers, two blocks
+// per SM: 44 us for one patch against 142 for the shared-memory LU (a 2D
+// transfer between meshes of 3,000 and 4,000 points 0.62 -> 0.49 ms; 48 mixed
+// transfers of 1,000 to 30,000 points 13.5 -> 11.9 ms).
 #include <type_traits>
 
 #include "patch.cuh"
@@ -39,8 +43,8 @@ namespace pacman_b200 {
 
 namespace {
 
-constexpr int kMomWarps = 4;          // patches per block of k_small_moments
-constexpr int kMomLd = kSmallMax + 1; // column stride: odd, one bank per column
+constexpr int kMomWarps = 4;            // patches per block of k_small_moments
+constexpr int kMomLd = kSmallWide + 1;  // column stride: odd, one bank per column
 
 // Moments of the patch's centred monomials (poly.cuh: red layout up to the
 // coordinate ranges), a warp per patch and a lane per value: every value is a
@@ -139,13 +143,18 @@ __global__ void __launch_bounds__(32)
 
 template <int N, int KF, bool ADJ>
 struct SmallCfg {
-  static constexpr int kT = N <= 32 ? 32 : 64;  // threads
-  static constexpr int kLd = N + 2;             // row stride: 16-byte rows, spread over the banks
-  static constexpr int kBlk = 16;               // pivots per unrolled group
+  static constexpr int kT = (N + 31) / 32 * 32;  // threads
+  static constexpr int kLd = N + 2;              // row stride: 16-byte rows, spread over the banks
+  static constexpr int kBlk = 16;                // pivots per unrolled group
+  static constexpr size_t kSmem = size_t(N) * kLd * sizeof(double);
   // Resident blocks per SM the registers are shared out for.  A row takes 2 N
   // registers; four, three or two warps per scheduler leave 128, 168 or 255.
-  static constexpr int kMinBlocks = 
-      N <= 32 ? 16 : (N <= 40 ? 8 : (N <= 48 || (KF == 1 ? N <= 56 || !ADJ : N <= 56 && !ADJ) ? 5 : 4));
+  static constexpr int kMinBlocks = N <= 32   ? 16
+                                    : N <= 40 ? 8
+                                    : N <= 48 ? 5
+                                    : N <= 56 ? (KF == 1 || !ADJ ? 5 : 4)
+                                    : N <= 64 ? 4
+                                              : 2;
 };
 
 template <int N, int KF, bool ADJ>
@@ -153,7 +162,7 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
     k_small_lu(PatchArgs a, const int *__restrict__ plist) {
   using C = SmallCfg<N, KF, ADJ>;
   constexpr int T = C::kT, LD = C::kLd, BLK = C::kBlk;
-  __shared__ __align__(16) double As[N * LD];
+  extern __shared__ __align__(16) double As[];  // N x LD
   __shared__ __align__(16) double col[2][T + BLK];
   __shared__ double xs[T], ys[T], zs[T];
   __shared__ double rp[2][KF];
@@ -351,13 +360,14 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
     const double *ar = As + (i < n ? i : 0) * LD;
     const double dg = i < n ? ar[i] : 1.0;
     const double inv = recip(dg);
-    if (T > 32) {
-      if (warp == 1) {
-        for (int j = n - 1; j >= 32; --j) {
+    for (int w = T / 32 - 1; w >= 0; --w) {
+      const int j0 = 32 * w, j1 = n < j0 + 32 ? n : j0 + 32;
+      if (warp == w) {
+        for (int j = j1 - 1; j >= j0; --j) {
           const double u = (i < j) ? ar[j] : 0.0;
 #pragma unroll
           for (int f = 0; f < KF; ++f) {
-            const double xj = __shfl_sync(0xffffffffu, quot(r[f], dg, inv), j - 32);
+            const double xj = __shfl_sync(0xffffffffu, quot(r[f], dg, inv), j - j0);
             if (i == j) r[f] = xj;
             else r[f] = __fma_rn(-u, xj, r[f]);
           }
@@ -366,28 +376,14 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
         for (int f = 0; f < KF; ++f) al[f][i] = r[f];
       }
       __syncthreads();
-      if (warp == 0) {
-        for (int j = 32; j < n; ++j) {
+      if (warp < w) {
+        for (int j = j0; j < j1; ++j) {
           const double u = ar[j];
 #pragma unroll
           for (int f = 0; f < KF; ++f) r[f] = __fma_rn(-u, al[f][j], r[f]);
         }
       }
     }
-    if (warp == 0) {
-      for (int j = (n < 32 ? n : 32) - 1; j >= 0; --j) {
-        const double u = (i < j) ? ar[j] : 0.0;
-#pragma unroll
-        for (int f = 0; f < KF; ++f) {
-          const double xj = __shfl_sync(0xffffffffu, quot(r[f], dg, inv), j);
-          if (i == j) r[f] = xj;
-          else r[f] = __fma_rn(-u, xj, r[f]);
-        }
-      }
-#pragma unroll
-      for (int f = 0; f < KF; ++f) al[f][i] = r[f];
-    }
-    __syncthreads();
   }
 
   bool nonfinite = false;
@@ -486,17 +482,23 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
 
 template <int N, bool ADJ>
 void launch_n(const PatchArgs &a, const int *plist, int np, cudaStream_t st) {
-  const int T = SmallCfg<N, 1, ADJ>::kT;
-  if (a.F == 1) k_small_lu<N, 1, ADJ><<<np, T, 0, st>>>(a, plist);
-  else if (a.F <= 4) k_small_lu<N, 4, ADJ><<<np, T, 0, st>>>(a, plist);
-  else k_small_lu<N, 8, ADJ><<<np, T, 0, st>>>(a, plist);
+  using C = SmallCfg<N, 1, ADJ>;
+  auto go = [&](auto kernel) {
+    if (C::kSmem > 40 * 1024)
+      PB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   int(C::kSmem)));
+    kernel<<<np, C::kT, C::kSmem, st>>>(a, plist);
+  };
+  if (a.F == 1) go(k_small_lu<N, 1, ADJ>);
+  else if (a.F <= 4) go(k_small_lu<N, 4, ADJ>);
+  else go(k_small_lu<N, 8, ADJ>);
   note_launch();
   PB_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
-int small_class(int n) { return n <= 32 ? 32 : (n + 7) / 8 * 8; }
+int small_class(int n) { return n <= 32 ? 32 : (n <= 64 ? (n + 7) / 8 * 8 : kSmallWide); }
 
 void launch_small_poly(const PatchArgs &a, const int *plist, int np, bool adj, cudaStream_t st) {
   if (np == 0) return;
@@ -517,7 +519,8 @@ void launch_small_lu(const PatchArgs &a, const int *plist, int np, int N, bool a
     case 40: launch_n<40, kAdjoint>(a, plist, np, st); break;
     case 48: launch_n<48, kAdjoint>(a, plist, np, st); break;
     case 56: launch_n<56, kAdjoint>(a, plist, np, st); break;
-    default: launch_n<64, kAdjoint>(a, plist, np, st); break;
+    case 64: launch_n<64, kAdjoint>(a, plist, np, st); break;
+    default: launch_n<kSmallWide, kAdjoint>(a, plist, np, st); break;
     }
   };
   if (adj) go(std::true_type{});

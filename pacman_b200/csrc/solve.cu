@@ -382,8 +382,8 @@ static void run_register_ranges(PatchArgs a, const std::vector<SmallRange> &rang
   }
 }
 
-// Runs one mode over a list of patches: n <= kSmallMax in the register kernel,
-// by size class; the rest in k_patch_solve, in buckets of doubling size so
+// Runs one mode over a list of patches: n <= kSmallWide in the register
+// kernel, by size class; the rest in k_patch_solve, in buckets of doubling size so
 // that the dynamic shared memory follows the bucket's largest patch, patches
 // too large for shared memory in a global workspace.  general: every patch in
 // k_patch_solve.
@@ -399,20 +399,21 @@ static void run_list(Plan &p, PatchArgs a, int mode, const std::vector<int> &pat
   host_list.reserve(patches.size());
   std::vector<SmallRange> ranges;
   if (!general) {
-    constexpr int kClasses = (kSmallMax - 32) / 8 + 1;
-    std::vector<int> cls[kClasses];  // sizes 64, 56, 48, 40, 32
+    static const int kSizes[] = {kSmallWide, 64, 56, 48, 40, 32};
+    constexpr int kClasses = 6;
+    std::vector<int> cls[kClasses];
     for (int k : patches) {
       const int n = p.n_host[k];
-      if (n > kSmallMax) rest.push_back(k);
-      else cls[(kSmallMax - small_class(n)) / 8].push_back(k);
+      if (n > kSmallWide) rest.push_back(k);
+      else cls[n > kSmallMax ? 0 : 1 + (kSmallMax - small_class(n)) / 8].push_back(k);
     }
     // A class that would not fill the GPU joins the next larger one: its own
     // launch would only add the latency of one patch.
     const size_t fill = size_t(5) * size_t(tuning_for_current_device().sms);
-    for (int c = 1; c < kClasses; ++c)
+    for (int c = 2; c < kClasses; ++c)  // the widest class stays by itself
       if (!cls[c].empty() && cls[c].size() < fill) {
         int to = c - 1;
-        while (to > 0 && cls[to].empty()) --to;
+        while (to > 1 && cls[to].empty()) --to;
         if (cls[to].empty()) continue;
         cls[to].insert(cls[to].end(), cls[c].begin(), cls[c].end());
         cls[c].clear();
@@ -424,7 +425,7 @@ static void run_list(Plan &p, PatchArgs a, int mode, const std::vector<int> &pat
       SmallRange sr;
       sr.first = host_list.size();
       sr.count = int(c.size());
-      sr.nclass = kSmallMax - 8 * ci;
+      sr.nclass = kSizes[ci];
       sr.fac_off = tot;
       tot += c.size() * small_fac_doubles(sr.nclass);
       ranges.push_back(sr);
@@ -513,17 +514,23 @@ void solve_big_cached(Plan &p, FactorCache &c, int basis, const double *vals, in
                       double *local, int *status, SolveReport &rep, const BigExtra &extra);
 
 // Patches above this size use the blocked engine (blocked.cu): for the mixed
-// path the tuned value, at most kSmallMax (the register kernel's largest
-// patch); 128 for the FP64 and adjoint paths, whose shared-memory kernel is as
+// path the tuned value, at most kSmallMax, but kSmallWide where no patch is
+// larger (the register kernel then takes them all, which saves the engine's
+// set-up and launches: 500k uniform points 3.85 -> 3.68 ms; where the engine
+// runs anyway it takes the patches above 64 along); 128 for the FP64 and adjoint paths, whose shared-memory kernel is as
 // fast up to there and takes one launch (250k refined points, 685 patches of
 // 65 to 128 sources: 46.7 ms a call with either line; 150k uniform points,
 // 154 such patches, gradients: 7.77 against 7.97 ms with 64).
 // PACMAN_B200_BIG_N overrides both.
-static int big_threshold(int mode) {
+static int big_threshold(const Plan &p, int mode) {
   const char *e = std::getenv("PACMAN_B200_BIG_N");
   if (e) return std::max(1, std::atoi(e));
   if (mode != kChol) return 128;
-  return std::min(kSmallMax, std::max(1, tuning_for_current_device().big_n_chol));
+  const int tuned = tuning_for_current_device().big_n_chol;
+  if (tuned < kSmallMax) return std::max(1, tuned);
+  for (int k = 0; k < p.K; ++k)
+    if (p.n_host[k] > kSmallWide && p.m_host[k] > 0) return kSmallMax;
+  return kSmallWide;
 }
 
 static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F, int precision,
@@ -585,7 +592,7 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   // 5.8e-15 -> 4.4e-15, C4 2.5e-13 -> 2.8e-13.  A patch that is not positive
   // definite in FP64 is solved again by the LU below.
   const int mode = precision == PACMAN_B200_FP64 ? kLU : kChol;
-  const int nbig = big_threshold(mode);
+  const int nbig = big_threshold(p, mode);
   std::vector<int> small, big;
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;  // no target: the patch contributes nothing
@@ -643,8 +650,8 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
     if (p.m_host[k] == 0) continue;
     if (stat[k] & kStatusDropped) rep.dropped++;
     // Every patch that the LU has not solved already (k_patch_solve takes
-    // kSmallMax < n <= nbig of the FP64 path).
-    const bool other = mode == kChol || p.n_host[k] <= kSmallMax || p.n_host[k] > nbig;
+    // kSmallWide < n <= nbig of the FP64 path).
+    const bool other = mode == kChol || p.n_host[k] <= kSmallWide || p.n_host[k] > nbig;
     if ((other && (stat[k] & (kStatusBreakdown | kStatusNonFinite | kStatusTimeout))) ||
         (cached && redo_mark[k]))
       (p.n_host[k] > nbig ? redo_big : redo_small).push_back(k);
@@ -711,7 +718,7 @@ void solve_adjoint(Plan &p, int basis, int F, const double *h, double *g_out, So
   a.basis = basis;
   a.h = h;
   a.g_out = g_out;
-  const int nbig = big_threshold(kAdj);
+  const int nbig = big_threshold(p, kAdj);
   std::vector<int> small, big;
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;  // h = 0 there: g = 0 (the caller zeroes g)
@@ -731,7 +738,7 @@ void solve_adjoint(Plan &p, int basis, int F, const double *h, double *g_out, So
   PB_CUDA(host_sync(st));
   std::vector<int> redo;
   for (int k : small)
-    if (p.n_host[k] <= kSmallMax && (stat[k] & (kStatusBreakdown | kStatusNonFinite)))
+    if (p.n_host[k] <= kSmallWide && (stat[k] & (kStatusBreakdown | kStatusNonFinite)))
       redo.push_back(k);
   run_list(p, a, kAdj, redo, rep, st, nullptr, true);
   for (int k = 0; k < K; ++k)

@@ -85,3 +85,25 @@ def test_adjoint_is_the_transpose(fields):
     # Both sums round each of their terms once more: n eps of the larger norm.
     scale = np.linalg.norm(out) * np.linalg.norm(G) + np.linalg.norm(v) * np.linalg.norm(gv)
     assert abs((G * out).sum() - (v * gv).sum()) <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("precision", sorted(TOL))
+@pytest.mark.parametrize("n", [65, 66, 80, 95, 96, 97])
+def test_three_warp_class_matches_oracle(precision, n):
+    # 65 to 96 sources: three warps, the last of them full or ragged.
+    rng = np.random.default_rng(n)
+    S = rng.random((n, 3))
+    T = S.min(0) + (S.max(0) - S.min(0)) * rng.random((50, 3))
+    plan = pacman.rbf.Plan(3, S, T, nodes_per_cluster=128, precision=precision)
+    assert n in np.diff(plan.patch_lists("source")[0])
+    for fields in (1, 3, 8):
+        v = _fields(S, fields)
+        out = plan.execute(0x11, v, save_for_adjoint=True)
+        for f in range(fields):
+            ref = oracle.interpolate(3, 0x11, S, np.ascontiguousarray(v[:, f]), T, 128)
+            assert rel_l2(out[:, f], ref) <= TOL[precision]
+        G = rng.standard_normal((len(T), fields))
+        gv, _ = plan.adjoint(G, targets=False)
+        scale = np.linalg.norm(out) * np.linalg.norm(G) + np.linalg.norm(v) * np.linalg.norm(gv)
+        assert abs((G * out).sum() - (v * gv).sum()) <= 1e-10 * scale
+    assert not (plan.patch_status() & (2 | 4 | 16)).any()
