@@ -210,17 +210,50 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
   zs[i] = x.z;
   __syncthreads();
 
-  if (ADJ && i < n) {
-    // Right-hand sides E^T h, E_ij = phi(|y_i - x_j|).
+  // Adjoint: thread i sums value vq = 4 field + monomial over every kParts-th
+  // point, from part i / (4 KF).
+  constexpr int kParts = T / (4 * KF);
+  __shared__ double vpart[ADJ ? T : 1];
+  const int vq = i % (4 * KF), vf = vq >> 2, vax = vq & 3;
+  if (ADJ) {
+    // Right-hand sides E^T h, E_ij = phi(|y_i - x_j|), and the parts of V'^T h:
+    // T targets at a time are staged in As, a target per thread (read one after
+    // another from memory by all, they cost a third of the block's time: all
+    // adjoint launches for 150,000 uniform points and 4 fields 1.09 -> 0.75 ms).
+    static_assert((3 + KF) * T <= N * LD, "staged targets");
+    const double4 c = a.centers[k];
+    const double cc = vax == 1 ? c.x : (vax == 2 ? c.y : c.z);
+    double v = 0.0;
     with_basis(a.basis, [&](auto B) {
-      for (int t = 0; t < m; ++t) {
-        const double4 y = a.tgt[a.tidx[t0 + t]];
-        const double ph = phi_at<B>(sqdist3(y.x, y.y, y.z, x.x, x.y, x.z), a.rinv);
+      for (int tb = 0; tb < m; tb += T) {
+        const int cnt = m - tb < T ? m - tb : T;
+        if (i < cnt) {
+          const double4 y = a.tgt[a.tidx[t0 + tb + i]];
+          As[i] = y.x;
+          As[T + i] = y.y;
+          As[2 * T + i] = y.z;
 #pragma unroll
-        for (int f = 0; f < KF; ++f)
-          if (f < F) r[f] = __fma_rn(ph, a.h[(t0 + t) * F + f], r[f]);
+          for (int f = 0; f < KF; ++f)
+            As[(3 + f) * T + i] = f < F ? a.h[(t0 + tb + i) * F + f] : 0.0;
+        }
+        __syncthreads();
+        for (int t = 0; t < cnt; ++t) {
+          const double ph = phi_at<B>(
+              sqdist3(As[t], As[T + t], As[2 * T + t], x.x, x.y, x.z), a.rinv);
+#pragma unroll
+          for (int f = 0; f < KF; ++f) r[f] = __fma_rn(ph, As[(3 + f) * T + t], r[f]);
+        }
+        const double *yc = As + (vax > 0 ? vax - 1 : 0) * T;
+        for (int t = i / (4 * KF); t < cnt; t += kParts)
+          v += (vax == 0 ? 1.0 : yc[t] - cc) * As[(3 + vf) * T + t];
+        __syncthreads();
       }
     });
+    vpart[i] = v;
+    if (i >= n) {
+#pragma unroll
+      for (int f = 0; f < KF; ++f) r[f] = 0.0;
+    }
   }
 
   bool bad = false;
@@ -388,22 +421,26 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
 
   bool nonfinite = false;
   if (ADJ) {
-    // g = z - Q' G'^{-1} (Q'^T z - V'^T h), centred monomials q' = [1, x - c]:
-    // the sums by one thread per (field, monomial), points in order.
+    // g = z - Q' G'^{-1} (Q'^T z - V'^T h), centred monomials q' = [1, x - c].
     __shared__ double corr[4 * KF];
+    __shared__ double upart[T];
     const double4 c = a.centers[k];
-    if (i < 4 * KF && (i >> 2) < F) {
-      const int f = i >> 2, ax = i & 3;
-      const double cc = ax == 1 ? c.x : (ax == 2 ? c.y : c.z);
-      const double *xc = ax == 1 ? xs : (ax == 2 ? ys : zs);
+    {
+      const double cc = vax == 1 ? c.x : (vax == 2 ? c.y : c.z);
+      const double *xc = vax == 1 ? xs : (vax == 2 ? ys : zs);
+      double u = 0.0;
+      for (int j = i / (4 * KF); j < n; j += kParts)
+        u += (vax == 0 ? 1.0 : xc[j] - cc) * al[vf][j];
+      upart[i] = u;
+    }
+    __syncthreads();
+    if (i < 4 * KF) {
       double u = 0.0, v = 0.0;
-      for (int j = 0; j < n; ++j) u += (ax == 0 ? 1.0 : xc[j] - cc) * al[f][j];
-      for (int t = 0; t < m; ++t) {
-        const double4 y = a.tgt[a.tidx[t0 + t]];
-        const double yc = ax == 1 ? y.x : (ax == 2 ? y.y : y.z);
-        v += (ax == 0 ? 1.0 : yc - cc) * a.h[(t0 + t) * F + f];
+      for (int q = i; q < kParts * 4 * KF; q += 4 * KF) {
+        u += upart[q];
+        v += vpart[q];
       }
-      corr[4 * f + ax] = u - v;
+      corr[i] = u - v;
     }
     __syncthreads();
     if (i < F) {
