@@ -59,11 +59,12 @@ struct PatchArgs {
 // LU with two block barriers per pivot (one patch of 70 sources: 142 us there,
 // 44 here).  The list of launch_small_lu holds patches of one size class
 // N = small_class(n); launch_small_poly must have run on the same list (pbeta,
-// pact, status).
+// pact, status).  behind: the launch before on this stream is another class of
+// the same list (they share nothing, so the two may overlap).
 constexpr int kSmallMax = 64, kSmallWide = 96;
 int small_class(int n);
 void launch_small_poly(const PatchArgs &a, const int *plist, int np, bool adj, cudaStream_t st);
-void launch_small_lu(const PatchArgs &a, const int *plist, int np, int N, bool adj,
+void launch_small_lu(const PatchArgs &a, const int *plist, int np, int N, bool adj, bool behind,
                      cudaStream_t st);
 
 }  // namespace pacman_b200

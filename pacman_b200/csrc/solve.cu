@@ -378,7 +378,7 @@ static void run_register_ranges(PatchArgs a, const std::vector<SmallRange> &rang
     b.pact = a.pact + r.first * 8;
     b.fac = fac ? fac + r.fac_off : nullptr;
     b.fac_mode = fac ? fac_mode : 0;
-    launch_small_lu(b, list + r.first, r.count, r.nclass, adj, st);
+    launch_small_lu(b, list + r.first, r.count, r.nclass, adj, &r != &ranges.front(), st);
   }
 }
 
