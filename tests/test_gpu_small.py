@@ -107,3 +107,44 @@ def test_three_warp_class_matches_oracle(precision, n):
         scale = np.linalg.norm(out) * np.linalg.norm(G) + np.linalg.norm(v) * np.linalg.norm(gv)
         assert abs((G * out).sum() - (v * gv).sum()) <= 1e-10 * scale
     assert not (plan.patch_status() & (2 | 4 | 16)).any()
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3])
+@pytest.mark.parametrize("n", [60, 200])
+@pytest.mark.parametrize("ratio", [1e-3, 0.2, 0.45, 0.55, 0.99, 1.01, 3.0])
+def test_axis_drop_decision_near_the_limit(dim, n, ratio):
+    # The last axis is scaled so that cond([1, x]) = ratio 1e5: an axis is
+    # dropped in exactly the patches above the limit (1% is far above the rounding
+    # of a condition number of 1e5, about 1e-11).
+    rng = np.random.default_rng(n + dim)
+    S = 1.0 + rng.random((n, dim))
+    T = S[:20].copy()
+
+    def cond(h):
+        P = S.copy()
+        P[:, -1] = 1.5 + (P[:, -1] - 1.5) * h
+        return np.linalg.cond(np.column_stack([np.ones(n), P])), P
+
+    lo, hi = 1e-8, 1.0
+    for _ in range(200):
+        mid = np.sqrt(lo * hi)
+        lo, hi = (mid, hi) if cond(mid)[0] > ratio * 1e5 else (lo, mid)
+    c, P = cond(hi)
+    assert abs(c / (ratio * 1e5) - 1) < 1e-3
+    T[:, -1] = P[:20, -1]
+    plan = pacman.rbf.Plan(dim, P, T, nodes_per_cluster=256)
+    v = np.sin(P.sum(axis=1))
+    out = plan.execute(0x12, v)
+    assert np.isfinite(out).all()
+    off, idx = plan.patch_lists("source")[:2]
+    toff = plan.patch_lists("target")[0]
+    status = plan.patch_status()
+    checked = 0
+    for k in range(len(off) - 1):
+        own = P[idx[off[k]:off[k + 1]]]
+        if toff[k + 1] > toff[k] and len(own) > dim:
+            c = np.linalg.cond(np.column_stack([np.ones(len(own)), own])) / 1e5
+            if abs(c - 1) > 0.005:
+                assert (status[k] & 1) == (c > 1)
+                checked += 1
+    assert checked
