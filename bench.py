@@ -491,7 +491,7 @@ def measure_mls(pacman, S, V0, T, timed, steps):
     mms = statistics.median(mt)
     return {"value": T.shape[0] / (mms * 1e-3), "unit": UNIT, "ms_per_call": mms,
             "what": "pacman.MLS.interpolate, same sources, targets and first field, "
-                    "device-resident (k_mls: 10-nearest search, Jacobi pseudo-inverse of the "
+                    "device-resident (10-nearest search, Jacobi pseudo-inverse of the "
                     "10 x 10 moment matrix)"}
 
 
@@ -630,7 +630,7 @@ def main():
     h2d = (w["src"].nbytes + w["tgt"].nbytes + np.ascontiguousarray(vals_np).nbytes)
     d2h = o_np.nbytes
 
-    # Plain FP64 path (the reference's unpivoted-LU algorithm) over the same
+    # Plain FP64 path (unpivoted LU of small patches, Cholesky above) over the same
     # number of timed steps, and the agreement of the two paths.
     extra = {"ms_per_step_median": statistics.median(times),
              "e2e_ms_per_step_median": statistics.median(e2e_times),

@@ -57,7 +57,8 @@ extern "C" {
 #define PACMAN_B200_EXEC_SYCL 0x05
 
 /* Precision of the per-patch solves. */
-#define PACMAN_B200_FP64 0  /* the reference algorithm: unpivoted LU in FP64 */
+#define PACMAN_B200_FP64 0  /* FP64 throughout: the reference's unpivoted LU up
+                               to 128 sources, Cholesky above */
 #define PACMAN_B200_MIXED 1 /* Cholesky (A is symmetric positive definite):
                                small patches in FP64 registers, the column
                                updates of large patches as split-integer

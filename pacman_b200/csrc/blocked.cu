@@ -8,18 +8,18 @@
 //        [ E   0 ]      E: m x n evaluation matrix (TeamFillE, team_ops.hpp:78-97)
 //                       r: n x F residuals b - Q beta (solver.hpp:451-468)
 //
-// stored in 64 x 64 tiles (A padded with an identity block).  Unpivoted
-// elimination of the first n columns leaves the Schur complement
+// stored in 64 x 64 tiles (A padded with an identity block).  This file has
+// the unpivoted LU of that matrix, the path of the patches that are not
+// positive definite (cholesky.cu has the others' solver), and the driver of
+// both.  Unpivoted elimination of the first n columns leaves the Schur complement
 // S = -E A^{-1} r in the bottom-right block, i.e. minus the RBF part of the
 // local interpolant (solver.hpp:474-478); no triangular solves and no
 // separate evaluation pass are needed.  All large patches advance in lockstep,
 // one 64-column pivot block per step:
-//   k_diag    factor the diagonal tile (LU or Cholesky) and invert it,
-//   k_trsm    apply the inverse to the panel tiles,
-//   k_update  trailing update C -= A * op(B) of every remaining tile,
+//   k_diag          factor the diagonal tile,
+//   k_trsm          solve the panel tiles with it,
+//   k_update_strip  trailing update C -= A * B of every remaining tile,
 // with the tile products on the FP64 tensor cores (mma.sync m8n8k4 f64).
-// Mode kLU is the reference's unpivoted LU; mode kChol uses the symmetry of A
-// (lower tiles only, half the work) and flags non-positive pivots.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -29,47 +29,14 @@
 
 namespace pacman_b200 {
 
-// Tiles filled by the assembly of one slot: LU every (row, column) tile of
-// the augmented matrix; Cholesky the lower A tiles, every E tile and the
-// residual column (row t < T: t + 2 tiles, row t >= T: T + 1 tiles).
-__device__ __forceinline__ void decode_assemble(bool lu, const BigSlot &sl, int l, int &ti,
-                                                int &tj) {
-  if (lu) {
-    ti = l / (sl.T + 1);
-    tj = l % (sl.T + 1);
-    return;
-  }
-  int t = 0;
-  for (;;) {
-    const int len = (t < sl.T) ? t + 2 : sl.T + 1;
-    if (l < len) {
-      ti = t;
-      tj = (t < sl.T) ? (l <= t ? l : sl.T) : l;
-      return;
-    }
-    l -= len;
-    ++t;
-  }
-}
-
-// Panel tiles of step s.  LU: row panel (s, s+1..T) then column panel
-// (s+1..R-1, s).  Cholesky: residual tile (s, T) then column panel.
-__device__ __forceinline__ void decode_trsm(bool lu, const BigSlot &sl, int s, int l, int &ti,
-                                            int &tj) {
-  if (lu) {
-    const int nrow = sl.T - s;
-    if (l < nrow) {
-      ti = s;
-      tj = s + 1 + l;
-    } else {
-      ti = s + 1 + (l - nrow);
-      tj = s;
-    }
-  } else if (l == 0) {
+// Panel tiles of step s: row panel (s, s+1..T), then column panel (s+1..R-1, s).
+__device__ __forceinline__ void decode_trsm(const BigSlot &sl, int s, int l, int &ti, int &tj) {
+  const int nrow = sl.T - s;
+  if (l < nrow) {
     ti = s;
-    tj = sl.T;
+    tj = s + 1 + l;
   } else {
-    ti = s + l;
+    ti = s + 1 + (l - nrow);
     tj = s;
   }
 }
@@ -79,49 +46,29 @@ __device__ __forceinline__ void decode_trsm(bool lu, const BigSlot &sl, int s, i
 // prefetches the next B tile while the current product runs.
 constexpr int kStrip = 4;
 
-// Strip l of a slot at step s -> (row t, first list index j0, count).  The
-// column list of row t is LU: s+1..T; Cholesky: s+1..min(t, T-1), then T.
-__device__ __forceinline__ void decode_strip(bool lu, const BigSlot &sl, int s, int l, int &t,
-                                             int &j0, int &count) {
-  if (lu) {
-    const int W = sl.T - s, cpr = (W + kStrip - 1) / kStrip;
-    t = s + 1 + l / cpr;
-    j0 = (l % cpr) * kStrip;
-    count = min(kStrip, W - j0);
-    return;
-  }
-  t = s + 1;
-  for (;;) {
-    const int len = (t < sl.T) ? (t - s + 1) : (sl.T - s);
-    const int ch = (len + kStrip - 1) / kStrip;
-    if (l < ch) {
-      j0 = l * kStrip;
-      count = min(kStrip, len - j0);
-      return;
-    }
-    l -= ch;
-    ++t;
-  }
+// Strip l of a slot at step s -> (row t, first of its columns s+1..T, count).
+__device__ __forceinline__ void decode_strip(const BigSlot &sl, int s, int l, int &t, int &j0,
+                                             int &count) {
+  const int W = sl.T - s, cpr = (W + kStrip - 1) / kStrip;
+  t = s + 1 + l / cpr;
+  j0 = (l % cpr) * kStrip;
+  count = min(kStrip, W - j0);
 }
 
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
 
-
-
-
 // Fills one 64 x 64 tile of an augmented matrix.
 __global__ void __launch_bounds__(256)
-    k_assemble(BigArgs a, const BigSlot *__restrict__ slots, const int *__restrict__ pre, int cnt,
-               int lu) {
+    k_assemble(BigArgs a, const BigSlot *__restrict__ slots, const int *__restrict__ pre, int cnt) {
   __shared__ double rx[TB], ry[TB], rz[TB], cx[TB], cy[TB], cz[TB];
   const int q = find_slot(pre, cnt, blockIdx.x);
   const BigSlot sl = slots[q];
+  const int l = blockIdx.x - pre[q];  // every (row, column) tile
   struct {
     int ti, tj;
-  } it;
-  decode_assemble(lu != 0, sl, blockIdx.x - pre[q], it.ti, it.tj);
+  } it = {l / (sl.T + 1), l % (sl.T + 1)};
   const int tid = threadIdx.x;
   double *tile = a.W + sl.base + int64_t(it.ti) * TB * sl.ld + int64_t(it.tj) * TB;
   if (it.tj == sl.T) {  // residual columns: zero (the polynomial pass writes r)
@@ -284,48 +231,25 @@ __global__ void __launch_bounds__(256) k_big_poly(BigArgs a, const BigSlot *__re
 }
 
 // Factors diagonal tile (s, s) of each listed slot in place: unpivoted LU
-// (unit lower L below the diagonal, U on and above it) or Cholesky.
-template <bool LU>
+// (unit lower L below the diagonal, U on and above it).
 __global__ void __launch_bounds__(256) k_diag(BigArgs a, const BigSlot *__restrict__ slots, int s) {
   extern __shared__ double sm[];
   double *T = sm;                 // the tile
-  __shared__ double piv;
-  __shared__ int bad;
-  const int slot = blockIdx.x;
-  const BigSlot sl = slots[slot];
+  const BigSlot sl = slots[blockIdx.x];
   const int tid = threadIdx.x;
   double *g = a.W + sl.base + int64_t(s) * TB * sl.ld + int64_t(s) * TB;
   load_tile(T, g, sl.ld, tid, blockDim.x);
-  if (tid == 0) bad = 0;
   __syncthreads();
   for (int p = 0; p < TB; ++p) {
-    if (LU) {
-      const double d = T[p * LDS + p];
-      for (int i = p + 1 + tid; i < TB; i += blockDim.x) T[i * LDS + p] /= d;
-      __syncthreads();
-      const int w = TB - 1 - p;
-      for (int e = tid; e < w * w; e += blockDim.x) {
-        const int i = p + 1 + e / w, j = p + 1 + e % w;
-        T[i * LDS + j] = __fma_rn(-T[i * LDS + p], T[p * LDS + j], T[i * LDS + j]);
-      }
-      __syncthreads();
-    } else {
-      if (tid == 0) {
-        const double app = T[p * LDS + p];
-        if (!(app > 0.0)) bad = 1;
-        piv = sqrt(app);
-      }
-      __syncthreads();
-      const double d = piv;
-      for (int i = p + tid; i < TB; i += blockDim.x) T[i * LDS + p] = (i == p) ? d : T[i * LDS + p] / d;
-      __syncthreads();
-      const int w = TB - 1 - p;
-      for (int e = tid; e < w * w; e += blockDim.x) {
-        const int i = p + 1 + e / w, j = p + 1 + e % w;
-        if (j <= i) T[i * LDS + j] = __fma_rn(-T[i * LDS + p], T[j * LDS + p], T[i * LDS + j]);
-      }
-      __syncthreads();
+    const double d = T[p * LDS + p];
+    for (int i = p + 1 + tid; i < TB; i += blockDim.x) T[i * LDS + p] /= d;
+    __syncthreads();
+    const int w = TB - 1 - p;
+    for (int e = tid; e < w * w; e += blockDim.x) {
+      const int i = p + 1 + e / w, j = p + 1 + e % w;
+      T[i * LDS + j] = __fma_rn(-T[i * LDS + p], T[p * LDS + j], T[i * LDS + j]);
     }
+    __syncthreads();
   }
   // The factors go back to the workspace, where the panel solves (k_trsm)
   // and the backward sweep read them.
@@ -334,26 +258,14 @@ __global__ void __launch_bounds__(256) k_diag(BigArgs a, const BigSlot *__restri
     *reinterpret_cast<double2 *>(g + int64_t(r) * sl.ld + 2 * c2) =
         *reinterpret_cast<const double2 *>(T + r * LDS + 2 * c2);
   }
-  if (tid == 0 && bad) atomicOr(&a.status[sl.k], 4);
-}
-
-__device__ __forceinline__ void load_inv(double *s, const double *g, int tid, int nt) {
-  for (int idx = tid; idx < TB * TB / 2; idx += nt) {
-    const int r = idx >> 5, c2 = idx & 31;
-    *reinterpret_cast<double2 *>(s + r * LDS + 2 * c2) =
-        *reinterpret_cast<const double2 *>(g + r * TB + 2 * c2);
-  }
 }
 
 // Panel tiles of step s: row panel X := L^{-1} X (ti == s), column panel
-// X := X U^{-1} (LU) or X := X L^{-T} (Cholesky), by triangular solves with
-// the factors of the diagonal tile (s, s) as k_diag left them in the
-// workspace (unit lower L below the diagonal, U on and above it, or the
-// Cholesky factor below and on it): backward stable, unlike a product with
+// X := X U^{-1}, by triangular solves with the factors of the diagonal tile
+// (s, s) as k_diag left them in the workspace: backward stable, unlike a product with
 // the explicit inverse, whose error grows with the condition number of the
 // diagonal tile.  Each of the 8 warps solves 8 rows of X (column panel) or 8
 // columns (row panel, as rows of X^T against L^T) with warp_row_solve.
-template <bool LU>
 __global__ void __launch_bounds__(256)
     k_trsm(BigArgs a, const BigSlot *__restrict__ slots, const int *__restrict__ pre, int cnt,
            int s) {
@@ -363,26 +275,24 @@ __global__ void __launch_bounds__(256)
   const int q = find_slot(pre, cnt, blockIdx.x);
   const BigSlot sl = slots[q];
   struct {
-    int slot, ti, tj;
+    int ti, tj;
   } it;
-  it.slot = q;
-  decode_trsm(LU, sl, s, blockIdx.x - pre[q], it.ti, it.tj);
+  decode_trsm(sl, s, blockIdx.x - pre[q], it.ti, it.tj);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double *X = a.W + sl.base + int64_t(it.ti) * TB * sl.ld + int64_t(it.tj) * TB;
   const double *D = a.W + sl.base + int64_t(s) * TB * sl.ld + int64_t(s) * TB;
   const bool left = it.ti == s;
   load_tile(sX, X, sl.ld, tid, blockDim.x);
-  // The upper triangular operand of x U = c: U itself (LU column panel), or
-  // the transpose of the lower factor (row panel: unit L; Cholesky: L).
+  // The upper triangular operand of x U = c: U itself (column panel), or the
+  // transpose of the unit lower factor (row panel).
   for (int e = tid; e < TB * TB; e += blockDim.x) {
     const int r = e >> 6, c = e & 63;
     const double v = D[int64_t(r) * sl.ld + c];
-    if (LU && !left) sU[r * LDS + c] = c >= r ? v : 0.0;
-    else if (LU) sU[c * LDS + r] = r > c ? v : (r == c ? 1.0 : 0.0);
-    else sU[c * LDS + r] = r >= c ? v : 0.0;
+    if (!left) sU[r * LDS + c] = c >= r ? v : 0.0;
+    else sU[c * LDS + r] = r > c ? v : (r == c ? 1.0 : 0.0);
   }
   __syncthreads();
-  if (tid < TB) dinv[tid] = (LU && left) ? 1.0 : 1.0 / sU[tid * LDS + tid];
+  if (tid < TB) dinv[tid] = left ? 1.0 : 1.0 / sU[tid * LDS + tid];
   __syncthreads();
   {
     const int r0 = 8 * warp;
@@ -412,7 +322,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <bool LU>
 __global__ void __launch_bounds__(128, 2)
     k_update_strip(BigArgs a, const BigSlot *__restrict__ slots, const int *__restrict__ pre,
                    int cnt, int s) {
@@ -422,18 +331,13 @@ __global__ void __launch_bounds__(128, 2)
   const int q = find_slot(pre, cnt, blockIdx.x);
   const BigSlot sl = slots[q];
   int t, j0, count;
-  decode_strip(LU, sl, s, blockIdx.x - pre[q], t, j0, count);
+  decode_strip(sl, s, blockIdx.x - pre[q], t, j0, count);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
   double *base = a.W + sl.base;
   const int ld = sl.ld;
-  const int ncol = LU ? sl.T - s : ((t < sl.T) ? (t - s) : (sl.T - s - 1));
-  auto column = [&](int j) { return LU ? s + 1 + j : (j < ncol ? s + 1 + j : sl.T); };
-  auto bsrc = [&](int u) -> const double * {
-    const bool bt = !LU && u < sl.T;
-    return bt ? base + int64_t(u) * TB * ld + int64_t(s) * TB
-              : base + int64_t(s) * TB * ld + int64_t(u) * TB;
-  };
+  auto column = [&](int j) { return s + 1 + j; };
+  auto bsrc = [&](int u) { return base + int64_t(s) * TB * ld + int64_t(u) * TB; };
   async_tile(sA, base + int64_t(t) * TB * ld + int64_t(s) * TB, ld, tid, blockDim.x);
   async_tile(sB[0], bsrc(column(j0)), ld, tid, blockDim.x);
   cp_async_commit();
@@ -449,8 +353,7 @@ __global__ void __launch_bounds__(128, 2)
     if (jj + 1 < count) cp_async_wait<1>();
     else cp_async_wait<0>();
     __syncthreads();
-    if (!LU && u < sl.T) mma64<false, true>(sA, sB[jj & 1], acc, -1.0, wr, wc, lane);
-    else mma64<false, false>(sA, sB[jj & 1], acc, -1.0, wr, wc, lane);
+    mma64<false, false>(sA, sB[jj & 1], acc, -1.0, wr, wc, lane);
     acc_store(acc, C, ld, wr, wc, lane);
     __syncthreads();
   }
@@ -505,10 +408,8 @@ __global__ void __launch_bounds__(256) k_big_adj_rhs(BigArgs a, const BigSlot *_
 }
 
 // Backward sweep after the elimination: the residual column holds
-// y = L^{-1} r; solves U z = y (LU) or L^T z = y (Cholesky) tile row by tile
-// row from the last, in place.  In forward-save mode z (the RBF coefficients
+// y = L^{-1} r; solves U z = y tile row by tile row from the last, in place.  In forward-save mode z (the RBF coefficients
 // alpha) is also written per (patch, source).
-template <bool LU>
 __global__ void __launch_bounds__(256) k_back_sweep(BigArgs a, const BigSlot *__restrict__ slots) {
   __shared__ double tile[TB][TB + 1];
   __shared__ double zt[TB][kMaxF];
@@ -524,8 +425,7 @@ __global__ void __launch_bounds__(256) k_back_sweep(BigArgs a, const BigSlot *__
       acc[r][f] = rcol[int64_t(s * TB + r) * ld + f];
     }
     for (int t = s + 1; t < sl.T; ++t) {
-      const double *g = LU ? W + int64_t(s) * TB * ld + int64_t(t) * TB
-                           : W + int64_t(t) * TB * ld + int64_t(s) * TB;
+      const double *g = W + int64_t(s) * TB * ld + int64_t(t) * TB;
       __syncthreads();
       for (int e = tid; e < TB * TB; e += blockDim.x) tile[e >> 6][e & 63] = g[int64_t(e >> 6) * ld + (e & 63)];
       for (int e = tid; e < TB * F; e += blockDim.x) {
@@ -536,7 +436,7 @@ __global__ void __launch_bounds__(256) k_back_sweep(BigArgs a, const BigSlot *__
       const int o = tid & 63;
       for (int f = tid >> 6; f < F; f += 4) {
         double sum = 0.0;
-        for (int c = 0; c < TB; ++c) sum = __fma_rn(LU ? tile[o][c] : tile[c][o], zt[c][f], sum);
+        for (int c = 0; c < TB; ++c) sum = __fma_rn(tile[o][c], zt[c][f], sum);
         acc[o][f] -= sum;
       }
     }
@@ -548,7 +448,7 @@ __global__ void __launch_bounds__(256) k_back_sweep(BigArgs a, const BigSlot *__
       const int f = warp;
       for (int i = TB - 1; i >= 0; --i) {
         double sum = 0.0;
-        for (int j = i + 1 + lane; j < TB; j += 32) sum = __fma_rn(LU ? tile[i][j] : tile[j][i], acc[j][f], sum);
+        for (int j = i + 1 + lane; j < TB; j += 32) sum = __fma_rn(tile[i][j], acc[j][f], sum);
         sum = warp_sum(sum);
         if (lane == 0) acc[i][f] = (acc[i][f] - sum) / tile[i][i];
         __syncwarp();
@@ -650,32 +550,22 @@ static size_t slot_doubles(int n, int m) {
   return size_t(T + TE) * TB * size_t(T + 1) * TB;
 }
 
-static int64_t count_assemble(bool lu, const BigSlot &q) {
-  return lu ? int64_t(q.T + q.TE) * (q.T + 1) : int64_t(q.T) * (q.T + 3) / 2 + int64_t(q.TE) * (q.T + 1);
-}
-static int64_t count_trsm(bool lu, const BigSlot &q, int s) {
-  const int R = q.T + q.TE;
-  return lu ? int64_t(q.T - s) + (R - s - 1) : int64_t(R - s);
+static int64_t count_assemble(const BigSlot &q) { return int64_t(q.T + q.TE) * (q.T + 1); }
+static int64_t count_trsm(const BigSlot &q, int s) {
+  return int64_t(q.T - s) + (q.T + q.TE - s - 1);
 }
 static int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
-// sum_{L=1}^{W} ceil(L / kStrip)
-static int64_t strip_sum(int64_t W) {
-  const int64_t qq = W / kStrip, r = W % kStrip;
-  return kStrip * qq * (qq + 1) / 2 + r * (qq + 1);
-}
-static int64_t count_strips(bool lu, const BigSlot &q, int s) {
-  const int64_t R = q.T + q.TE, W = q.T - s;
-  return lu ? (R - s - 1) * ceil_div(W, kStrip) : (strip_sum(W) - 1) + int64_t(q.TE) * ceil_div(W, kStrip);
+static int64_t count_strips(const BigSlot &q, int s) {
+  return (int64_t(q.T) + q.TE - s - 1) * ceil_div(q.T - s, kStrip);
 }
 
 static void set_smem_attributes() {
   static bool done = false;
   if (done) return;
   const int s3 = 3 * TB * LDS * sizeof(double), s2 = 2 * TB * LDS * sizeof(double);
-  PB_CUDA(cudaFuncSetAttribute(k_diag<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
-  PB_CUDA(cudaFuncSetAttribute(k_trsm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
-  PB_CUDA(cudaFuncSetAttribute(k_update_strip<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               3 * TB * LDS * int(sizeof(double))));
+  PB_CUDA(cudaFuncSetAttribute(k_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
+  PB_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
+  PB_CUDA(cudaFuncSetAttribute(k_update_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
   done = true;
 }
 
@@ -820,11 +710,10 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
     }
     const int ns = int(slots.size());
     const int steps = slots.front().T;
-    // Prefix counts: assembly over all slots, then per step the trsm and
-    // update counts over the active slots (a prefix of the sorted slots).
-    std::vector<int> pre_asm(ns + 1, 0);
-    for (int q = 0; q < ns; ++q) {
-      const int64_t v = pre_asm[q] + count_assemble(lu, slots[q]);
+    // LU: prefix counts of the assembly's tiles over all slots.
+    std::vector<int> pre_asm(lu ? ns + 1 : 0, 0);
+    for (int q = 0; lu && q < ns; ++q) {
+      const int64_t v = pre_asm[q] + count_assemble(slots[q]);
       if (v > 0x7fffffffll) throw Error{PACMAN_B200_ERR_LIMIT, "too many tiles in one launch"};
       pre_asm[q + 1] = int(v);
     }
@@ -840,11 +729,11 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
         off[s] = int(pre.size());
         int64_t acc = 0;
         pre.push_back(0);
-        for (int q = 0; q < c; ++q) pre.push_back(int(acc += count_trsm(lu, slots[q], s)));
+        for (int q = 0; q < c; ++q) pre.push_back(int(acc += count_trsm(slots[q], s)));
         acc = 0;
         pre.push_back(0);
         for (int q = 0; q < c; ++q) {
-          acc += count_strips(lu, slots[q], s);
+          acc += count_strips(slots[q], s);
           if (acc > 0x7fffffffll) throw Error{PACMAN_B200_ERR_LIMIT, "too many tiles in one launch"};
           pre.push_back(int(acc));
         }
@@ -964,7 +853,7 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
       }
       continue;
     }
-    k_assemble<<<pre_asm[ns], 256, 0, st>>>(a, ds, dpre_asm, ns, 1);
+    k_assemble<<<pre_asm[ns], 256, 0, st>>>(a, ds, dpre_asm, ns);
     note_launch();
     k_big_poly<<<ns, 256, 0, st>>>(a, ds);
     note_launch();
@@ -975,15 +864,15 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
       const int *pu = pt + c + 1;
       const int nt = pre[off[s] + c];
       const int nu = pre[off[s] + c + 1 + c];
-      k_diag<true><<<c, 256, s3, st>>>(a, ds, s);
-      if (nt) k_trsm<true><<<nt, 256, s2, st>>>(a, ds, pt, c, s);
-      if (nu) k_update_strip<true><<<nu, 128, s3, st>>>(a, ds, pu, c, s);
+      k_diag<<<c, 256, s3, st>>>(a, ds, s);
+      if (nt) k_trsm<<<nt, 256, s2, st>>>(a, ds, pt, c, s);
+      if (nu) k_update_strip<<<nu, 128, s3, st>>>(a, ds, pu, c, s);
       note_launch(1 + (nt ? 1 : 0) + (nu ? 1 : 0));
     }
     k_big_finish<<<ns, 128, 0, st>>>(a, ds);
     note_launch();
     if (extra.mode == kBigForwardSave) {
-      k_back_sweep<true><<<ns, 256, 0, st>>>(a, ds);
+      k_back_sweep<<<ns, 256, 0, st>>>(a, ds);
       note_launch();
     }
     PB_CUDA(cudaGetLastError());

@@ -114,13 +114,6 @@ __device__ __forceinline__ void acc_store(const double (&acc)[4][4][2], double *
           make_double2(acc[i][j][0], acc[i][j][1]);
 }
 
-__device__ __forceinline__ void acc_zero(double (&acc)[4][4][2]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-}
-
 // Row solves x U = c for R rows of a 64-column tile by one warp: U upper
 // triangular (row-major, row stride LDS, exact zeros below the diagonal) in
 // shared memory and dinv[c] = 1 / U[c][c] (1 for a unit diagonal); on entry
@@ -160,65 +153,10 @@ __device__ __forceinline__ void warp_row_solve(double (&lo)[R], double (&hi)[R],
 }
 
 // In-place row solve X U = C for 8 rows (row stride LDS, 64 columns) by one
-// warp, blocked by 16 columns, all in registers: lane l holds column
-// 16 b + l % 16 of rows l / 16 + 2 q (q = 0..3) for the four column blocks
-// b.  Block b is solved by right-looking substitution against U's 16 x 16
-// diagonal block, then the blocks right of it are updated with the block's
-// result (broadcast by shuffles) times U's off-diagonal block, by FMAs on the
-// FP64 pipe: on B200 the FP64 tensor instructions are no faster than FMAs and
-// would compete with the int8 tensor-core MMAs of the same SM.  U: upper
-// triangular with exact zeros below the diagonal; dinv[c] = 1 / U[c][c].
-// Only the warp's own rows are touched, so no block barrier is needed; this
-// is a blocked triangular solve (diagonal blocks by substitution, off-
-// diagonal blocks by products), backward stable.
-__device__ __forceinline__ void warp_rows_trsm8(double *rows, const double *sU,
-                                                const double *dinv, int lane) {
-  const int col16 = lane & 15, half = lane & 16, rsel = lane >> 4;
-  double v[4][4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[b][q] = rows[(rsel + 2 * q) * LDS + 16 * b + col16];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int cb = 16 * b;
-#pragma unroll 4
-    for (int c = 0; c < 16; ++c) {
-      const double d = dinv[cb + c];
-      const double u = sU[(cb + c) * LDS + cb + col16];
-      const bool own = col16 == c;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const double x = __shfl_sync(0xffffffffu, v[b][q], half | c) * d;
-        v[b][q] = own ? x : __fma_rn(-x, u, v[b][q]);
-      }
-    }
-    if (b < 3) {
-#pragma unroll 4
-      for (int k = 0; k < 16; ++k) {
-        double x[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) x[q] = __shfl_sync(0xffffffffu, v[b][q], half | k);
-        const double *ur = sU + (cb + k) * LDS + col16;
-#pragma unroll
-        for (int bb = b + 1; bb < 4; ++bb) {
-          const double u = ur[16 * bb];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) v[bb][q] = __fma_rn(-x[q], u, v[bb][q]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int b = 0; b < 4; ++b)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) rows[(rsel + 2 * q) * LDS + 16 * b + col16] = v[b][q];
-  __syncwarp();
-}
-
-// warp_rows_trsm8 with each 16-column block solved by a product with the
-// inverse of U's 16 x 16 diagonal block instead of by substitution, all
-// products on the FP64 tensor cores (mma.sync m8n8k4: the warp's 8 rows are
+// warp; U: upper triangular with exact zeros below the diagonal.  Only the
+// warp's own rows are touched, so no block barrier is needed.  Each 16-column
+// block is solved by a product with the inverse of U's 16 x 16 diagonal block
+// (warp_rows_trsm8_tc: by substitution), all products on the FP64 tensor cores (mma.sync m8n8k4: the warp's 8 rows are
 // the instruction's M): X_b = R_b Ui_b, then R_c -= X_b U_bc for the blocks
 // c right of b.  Ui_b = U_bb^-1 is stored as sUi[(16 b + k) kUiLd + c] =
 // U_bb^-1[k][c] (the diagonal blocks of X_j = L_jj^-1 read as X_j[16 b +
@@ -290,8 +228,9 @@ __device__ __forceinline__ void warp_rows_solve8(double *rows, const double *sU,
   if (kStore) __syncwarp();
 }
 
-// warp_rows_trsm8 with the off-diagonal block products on the FP64 tensor
-// cores (mma.sync m8n8k4) through shared memory, for the FP64 step kernel,
+// The same solve with the diagonal blocks by right-looking substitution
+// (dinv[c] = 1 / U[c][c]) and only the off-diagonal block products on the FP64
+// tensor cores (mma.sync m8n8k4) through shared memory, backward stable, for the FP64 step kernel,
 // which runs no int8 MMAs and has fewer registers to spare.
 __device__ __forceinline__ void warp_rows_trsm8_tc(double *rows, const double *sU,
                                                    const double *dinv, int lane) {

@@ -193,16 +193,15 @@ __device__ __noinline__ void warp_trinv16(const double *D, int ld, int kb, const
 // blocks: warp 0 factors the diagonal block (16 column steps synchronised
 // within the warp), the eight warps solve the panel below it by substitution
 // and update the trailing blocks on the FP64 tensor cores, three barriers per
-// block.  X comes from the row solves X^T U = I (warp_rows_trsm8, or with
-// kTensorSolve warp_rows_trsm8_tc).  Us (TB x LDS) is shared scratch for U,
+// block.  X comes from the row solves X^T U = I: warp_rows_trsm8_tc, or with ui
+// (scratch for U's diagonal blocks' inverses) warp_rows_solve8.  Us (TB x LDS) is shared scratch for U,
 // dis (TB) for 1 / diag(L_c), ys (TB x kMaxF) for r.  Returns true on a
 // non-positive pivot (status 4 for the caller).
-template <class Sync, bool kTensorSolve = false>
+template <class Sync, bool kBlockInv>
 __device__ bool diag_tile_t(const double *g_in, int ld, double *rg, int rld, int F, double *gi,
-                            double *Us, double (*cv)[TB], double *dis, double (*ys)[kMaxF],
-                            int tid, Sync sync, double *gu = nullptr, int uld = 0,
-                            double *ui = nullptr, bool ys_loaded = false) {
-  (void)cv;
+                            double *Us, double *dis, double (*ys)[kMaxF], int tid, Sync sync,
+                            double *gu = nullptr, int uld = 0, double *ui = nullptr,
+                            bool ys_loaded = false) {
   double *D = const_cast<double *>(g_in);
   const int lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tq = lane & 3;
@@ -213,7 +212,6 @@ __device__ bool diag_tile_t(const double *g_in, int ld, double *rg, int rld, int
       const int r = e / kMaxF, f = e % kMaxF;
       ys[r][f] = f < F ? __ldcg(rg + int64_t(r) * rld + f) : 0.0;
     }
-  const bool blockinv = !kTensorSolve && ui != nullptr;
   // (a) the first diagonal block, warp 0 (warp_chol16).
   if (warp == 0) bad |= warp_chol16(D, ld, 0, dis, lane);
   sync();
@@ -281,17 +279,17 @@ __device__ bool diag_tile_t(const double *g_in, int ld, double *rg, int rld, int
   }
   // With ui: the inverses of U's four 16 x 16 diagonal blocks, one warp each,
   // for the block-inverse row solves of X below.
-  if (blockinv && warp < 4) warp_trinv16(D, ld, 16 * warp, dis, ui + 16 * warp * kUiLd, lane);
+  if (kBlockInv && warp < 4) warp_trinv16(D, ld, 16 * warp, dis, ui + 16 * warp * kUiLd, lane);
   sync();
   // X^T from X^T U = I: rows of the identity solved in place of D.
   for (int e = tid; e < TB * TB; e += 256) D[(e >> 6) * ld + (e & 63)] = (e >> 6) == (e & 63);
   sync();
-  if (kTensorSolve) warp_rows_trsm8_tc(D + 8 * warp * ld, Us, dis, lane);
-  else if (blockinv) {
+  if (kBlockInv) {
     double x[8][2];
     warp_rows_solve8<true>(D + 8 * warp * ld, Us, ui, lane, x);
+  } else {
+    warp_rows_trsm8_tc(D + 8 * warp * ld, Us, dis, lane);
   }
-  else warp_rows_trsm8(D + 8 * warp * ld, Us, dis, lane);
   sync();
   // X (row-major, gi) and y = X r.
   for (int e = tid; e < TB * TB; e += 256) {
@@ -314,19 +312,17 @@ __device__ bool diag_tile_t(const double *g_in, int ld, double *rg, int rld, int
 }
 
 __device__ __forceinline__ bool diag_tile(const double *g, int ld, double *rg, int rld, int F,
-                                          double *gi, double *Xs, double (*cv)[TB], double *dis,
-                                          double (*ys)[kMaxF], double *gu = nullptr,
-                                          int uld = 0) {
+                                          double *gi, double *Xs, double *dis,
+                                          double (*ys)[kMaxF], double *gu, int uld) {
   auto sync = [] { __syncthreads(); };
-  return diag_tile_t<decltype(sync), true>(g, ld, rg, rld, F, gi, Xs, cv, dis, ys,
-                                            int(threadIdx.x), sync, gu, uld);
+  return diag_tile_t<decltype(sync), false>(g, ld, rg, rld, F, gi, Xs, dis, ys, int(threadIdx.x),
+                                            sync, gu, uld);
 }
 
 // The diagonal tile of step 0 of every slot.
 __global__ void __launch_bounds__(256, 4) k_diag_chol(BigArgs a, const BigSlot *__restrict__ slots,
                                                       int j) {
   extern __shared__ double sm[];
-  __shared__ double cv[2][TB];
   __shared__ double dis[TB];
   __shared__ double ys[TB][kMaxF];
   const BigSlot sl = slots[blockIdx.x];
@@ -337,7 +333,7 @@ __global__ void __launch_bounds__(256, 4) k_diag_chol(BigArgs a, const BigSlot *
   __syncthreads();
   double *rg = a.W + sl.base + int64_t(j) * TB * ld + int64_t(sl.T) * TB;
   const bool bad =
-      diag_tile(gt, LDS, rg, ld, a.F, a.inv + sl.inv + int64_t(j) * TB * TB, sm, cv, dis, ys,
+      diag_tile(gt, LDS, rg, ld, a.F, a.inv + sl.inv + int64_t(j) * TB * TB, sm, dis, ys,
                 a.W + sl.base + int64_t(j) * TB * ld + int64_t(j) * TB, ld);
   if (threadIdx.x == 0 && bad) atomicOr(&a.status[sl.k], 4);
 }
@@ -352,15 +348,14 @@ __global__ void __launch_bounds__(256, 4) k_diag_chol(BigArgs a, const BigSlot *
 // of microseconds, and here two CTAs per SM overlap their chains while the
 // step kernel's CTAs go on with their items.
 constexpr size_t kDiagNextSmem =
-    (size_t(2) * TB * LDS + size_t(4) * 16 * kUiLd + 3 * TB + TB * kMaxF) * sizeof(double);
+    (size_t(2) * TB * LDS + size_t(4) * 16 * kUiLd + TB + TB * kMaxF) * sizeof(double);
 __global__ void __launch_bounds__(256, 2) k_diag_next(BigArgs a, const BigSlot *__restrict__ slots,
                                                       int j) {
   extern __shared__ __align__(16) double smn[];
   double *D = smn;                  // D' and then D (TB x LDS)
   double *Ls = D + TB * LDS;        // L[j+1, j], then U scratch
   double *ui = Ls + TB * LDS;       // U's 16 x 16 diagonal block inverses
-  double(*cv)[TB] = reinterpret_cast<double(*)[TB]>(ui + 4 * 16 * kUiLd);
-  double *dis = ui + 4 * 16 * kUiLd + 2 * TB;
+  double *dis = ui + 4 * 16 * kUiLd;
   double(*ys)[kMaxF] = reinterpret_cast<double(*)[kMaxF]>(dis + TB);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // The next step's launch may start now (its epilogue waits for this grid).
@@ -394,9 +389,9 @@ __global__ void __launch_bounds__(256, 2) k_diag_next(BigArgs a, const BigSlot *
   }
   __syncthreads();
   auto sync = [] { __syncthreads(); };
-  const bool bad = diag_tile_t(D, LDS, rg, ld, a.F, a.inv + sl.inv + int64_t(j + 1) * TB * TB, Ls,
-                               cv, dis, ys, tid, sync,
-                               W + int64_t(j + 1) * TB * ld + int64_t(j + 1) * TB, ld, ui, true);
+  const bool bad = diag_tile_t<decltype(sync), true>(
+      D, LDS, rg, ld, a.F, a.inv + sl.inv + int64_t(j + 1) * TB * TB, Ls, dis, ys, tid, sync,
+      W + int64_t(j + 1) * TB * ld + int64_t(j + 1) * TB, ld, ui, true);
   if (tid == 0 && bad) atomicOr(&a.status[sl.k], 4);
 }
 
@@ -838,10 +833,9 @@ __global__ void __launch_bounds__(kColThreads, 2)
   // Scratch of the factorisation over the consumed L[j+1, j] (sL).
   double *Xs = sm + TB * LDS;
   double(*ysd)[kMaxF] = reinterpret_cast<double(*)[kMaxF]>(Xs + TB * LDS);
-  double(*cv)[TB] = reinterpret_cast<double(*)[TB]>(Xs + TB * LDS + TB * kMaxF);
-  double *dis = Xs + TB * LDS + TB * kMaxF + 2 * TB;
+  double *dis = Xs + TB * LDS + TB * kMaxF;
   const bool bad = diag_tile(Ds, LDS, rcol + int64_t(j + 1) * TB * ld, ld, F,
-                             a.inv + sl.inv + int64_t(j + 1) * TB * TB, Xs, cv, dis, ysd,
+                             a.inv + sl.inv + int64_t(j + 1) * TB * TB, Xs, dis, ysd,
                              W + int64_t(j + 1) * TB * ld + int64_t(j + 1) * TB, ld);
   if (tid == 0 && bad) atomicOr(&a.status[sl.k], 4);
 }

@@ -35,10 +35,6 @@ __device__ __forceinline__ double sqdist3(double ax, double ay, double az,
   return acc;
 }
 
-__device__ __forceinline__ double sqdist(const double4 &a, const double4 &b) {
-  return sqdist3(a.x, a.y, a.z, b.x, b.y, b.z);
-}
-
 // 1 / d: the hardware's approximation r refined to r (1 + e + e^2), e = 1 - d r
 // (the series of the reciprocal), without branches so that it overlaps other
 // work.  Quotients formed with it are corrected (quot below).

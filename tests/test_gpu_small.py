@@ -1,4 +1,4 @@
-"""Register-kernel patches (n <= 64): every size class and its edges, field
+"""Register-kernel patches (n <= 96): every size class and its edges, field
 counts, both precisions, the adjoint, and clouds whose matrices are singular,
 against the CPU oracle."""
 import numpy as np
