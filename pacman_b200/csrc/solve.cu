@@ -514,11 +514,13 @@ void solve_big_cached(Plan &p, FactorCache &c, int basis, const double *vals, in
                       double *local, int *status, SolveReport &rep, const BigExtra &extra);
 
 // Patches above this size use the blocked engine (blocked.cu): for the mixed
-// path the tuned value, at most kSmallMax, but kSmallWide where no patch is
-// larger (the register kernel then takes them all, which saves the engine's
-// set-up and launches: 500k uniform points 3.85 -> 3.68 ms; where the engine
-// runs anyway it takes the patches above 64 along); 128 for the FP64 and adjoint paths, whose shared-memory kernel is as
-// fast up to there and takes one launch (250k refined points, 685 patches of
+// path the tuned value, at most kSmallMax, but kSmallWide where no patch of the
+// plan is larger (the register kernel then takes them all, which saves the
+// engine's set-up and launches: 500k uniform points 3.85 -> 3.68 ms; where the
+// engine runs anyway it takes the patches above 64 along).  Patches without
+// targets count too: a shard of a plan then solves its patches as the whole
+// plan does.  128 for the FP64 and adjoint paths, whose shared-memory kernel is
+// as fast up to there and takes one launch (250k refined points, 685 patches of
 // 65 to 128 sources: 46.7 ms a call with either line; 150k uniform points,
 // 154 such patches, gradients: 7.77 against 7.97 ms with 64).
 // PACMAN_B200_BIG_N overrides both.
@@ -529,7 +531,7 @@ static int big_threshold(const Plan &p, int mode) {
   const int tuned = tuning_for_current_device().big_n_chol;
   if (tuned < kSmallMax) return std::max(1, tuned);
   for (int k = 0; k < p.K; ++k)
-    if (p.n_host[k] > kSmallWide && p.m_host[k] > 0) return kSmallMax;
+    if (p.n_host[k] > kSmallWide) return kSmallMax;
   return kSmallWide;
 }
 

@@ -148,3 +148,29 @@ def test_axis_drop_decision_near_the_limit(dim, n, ratio):
                 assert (status[k] & 1) == (c > 1)
                 checked += 1
     assert checked
+
+
+def test_shards_choose_the_solver_of_the_whole_plan():
+    # Patches of 65 to 96 sources go to the register kernel where the plan has no
+    # larger one; shards whose own patches are all smaller answer as the whole does.
+    rng = np.random.default_rng(12)
+    S = np.r_[rng.random((12000, 3)), 0.02 * rng.random((150, 3))]
+    T = rng.random((9000, 3))
+    v = _fields(S, 1)[:, 0]
+
+    def plan():
+        return pacman.rbf.Plan(3, S, T, nodes_per_cluster=60, precision="mixed")
+
+    full = plan()
+    n = np.diff(full.patch_lists("source")[0])
+    assert n.max() > 96
+    ref = full.execute(0x12, v)
+    total, without = np.zeros_like(ref), 0
+    for rank in range(4):
+        p = plan()
+        p.shard(rank, 4)
+        live = n[np.diff(p.patch_lists("target")[0]) > 0]
+        without += live.max() <= 96 and (live > 64).any()
+        total += p.execute(0x12, v)
+    assert without
+    assert np.array_equal(total, ref)
