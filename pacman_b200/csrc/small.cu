@@ -357,43 +357,34 @@ __global__ void __launch_bounds__(SmallCfg<N, KF, ADJ>::kT, SmallCfg<N, KF, ADJ>
             *reinterpret_cast<const double2 *>(facp + rr * N + cc);
     }
     __syncthreads();
-    const int n0 = n < 32 ? n : 32;
+    // L y = r: each warp its own rows from the first, what later warps need of
+    // them through shared memory.
     const double *ar = As + (i < n ? i : 0) * LD;
-    if (warp == 0) {
-      for (int p = 0; p < n0; ++p) {
-        const double l = (lane > p && i < n) ? ar[p] : 0.0;
+    for (int w = 0; w < T / 32; ++w) {
+      const int j0 = 32 * w, j1 = n < j0 + 32 ? n : j0 + 32;
+      if (warp == w) {
+        for (int p = j0; p < j1; ++p) {
+          const double l = (i > p && i < n) ? ar[p] : 0.0;
 #pragma unroll
-        for (int f = 0; f < KF; ++f)
-          r[f] = __fma_rn(-l, __shfl_sync(0xffffffffu, r[f], p), r[f]);
-      }
-    }
-    if (T > 32) {
-      if (warp == 0) {
+          for (int f = 0; f < KF; ++f)
+            r[f] = __fma_rn(-l, __shfl_sync(0xffffffffu, r[f], p - j0), r[f]);
+        }
 #pragma unroll
         for (int f = 0; f < KF; ++f) al[f][i] = r[f];
       }
       __syncthreads();
-      if (warp == 1) {
-        if (i < n) {
-          for (int p = 0; p < 32; ++p) {
-            const double l = ar[p];
+      if (warp > w && i < n) {
+        for (int p = j0; p < j1; ++p) {
+          const double l = ar[p];
 #pragma unroll
-            for (int f = 0; f < KF; ++f) r[f] = __fma_rn(-l, al[f][p], r[f]);
-          }
-        }
-        for (int p = 32; p < n; ++p) {
-          const double l = (i > p && i < n) ? ar[p] : 0.0;
-#pragma unroll
-          for (int f = 0; f < KF; ++f)
-            r[f] = __fma_rn(-l, __shfl_sync(0xffffffffu, r[f], p - 32), r[f]);
+          for (int f = 0; f < KF; ++f) r[f] = __fma_rn(-l, al[f][p], r[f]);
         }
       }
-      __syncthreads();
     }
   }
 
-  // U alpha = y: each warp its own rows from the last, the second warp's
-  // results through shared memory.
+  // U alpha = y: each warp its own rows from the last, what earlier warps need
+  // of them through shared memory.
   {
     const double *ar = As + (i < n ? i : 0) * LD;
     const double dg = i < n ? ar[i] : 1.0;
