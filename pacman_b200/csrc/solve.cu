@@ -433,6 +433,7 @@ static void run_list(Plan &p, PatchArgs a, int mode, const std::vector<int> &pat
     }
     if (keep) {
       keep->ranges = ranges;
+      keep->rest = rest;
       keep->small_fac.alloc(sizeof(double) * std::max<size_t>(tot, 2), st);
     }
   } else {
@@ -594,7 +595,9 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   // 5.8e-15 -> 4.4e-15, C4 2.5e-13 -> 2.8e-13.  A patch that is not positive
   // definite in FP64 is solved again by the LU below.
   const int mode = precision == PACMAN_B200_FP64 ? kLU : kChol;
-  const int nbig = big_threshold(p, mode);
+  // Kept factors: the line that they were made with, whatever it is now.
+  const int nbig = cached ? cached->nbig : big_threshold(p, mode);
+  if (keep) keep->nbig = nbig;
   std::vector<int> small, big;
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;  // no target: the patch contributes nothing
@@ -621,6 +624,7 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
     // to wait for), the large ones run their sweeps on the group streams.
     if (beside) PB_CUDA(cudaStreamWaitEvent(ss, rep.tail_event, 0));
     run_small_cached(*cached, a, ss);
+    run_list(p, a, mode, cached->rest, rep, ss, nullptr, true);
     solve_big_cached(p, *p.fcache, basis, vals_dev, F, local_dev, p.status.as<int>(), rep, ex);
     for (const SmallRange &r : cached->ranges) rep.factors_reused += r.count;
   } else {

@@ -6,6 +6,7 @@ import pytest
 
 import oracle
 import pacman_b200 as pacman
+from pacman_b200 import workloads as W
 from tests.conftest import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -56,3 +57,32 @@ def test_whole_cloud_patches(n, fields):
 def test_uniform_clouds(dim, count, fields):
     rng = np.random.default_rng(dim)
     _check(dim, rng.random((count, dim)), rng.random((4000, dim)), 0x12, 50, 0.1, fields)
+
+
+@pytest.mark.parametrize("made,used", [("128", "128"), ("128", None), (None, "128"), ("8", "128")])
+def test_size_line_of_the_environment(made, used, monkeypatch):
+    # PACMAN_B200_BIG_N = 128 leaves patches of 97 to 128 sources to a kernel that
+    # keeps nothing; the line may also differ between the two executes.
+    def line(value):
+        if value is None:
+            monkeypatch.delenv("PACMAN_B200_BIG_N", raising=False)
+        else:
+            monkeypatch.setenv("PACMAN_B200_BIG_N", value)
+    case = W.make("grid_blobs_1m", scale=0.01)
+    S, T = case["src"], case["tgt"]
+    plan = pacman.rbf.Plan(3, S, T, precision="mixed")
+    n = np.diff(plan.patch_lists("source")[0])
+    m = np.diff(plan.patch_lists("target")[0])
+    assert ((n > 96) & (n <= 128) & (m > 0)).any() and ((n > 128) & (m > 0)).any()
+    line(made)
+    plan.execute(0x12, _fields(S, 1, 0), keep_factors=True)
+    line(used)
+    for fields, seed in ((1, 1), (2, 2)):
+        v = _fields(S, fields, seed)
+        st = {}
+        out = plan.execute(0x12, v, keep_factors=True, stats=st)
+        assert st["factors_reused"] > 0
+        for f in range(fields):
+            ref = oracle.interpolate(3, 0x12, S, np.ascontiguousarray(v[:, f]), T)
+            assert rel_l2(out[:, f], ref) <= TOL_MIXED
+    plan.close()
