@@ -553,6 +553,7 @@ void solve_group(const pacman_b200_problem *qs, const std::vector<int> &ids,
       g.n_host.insert(g.n_host.end(), p.n_host.begin(), p.n_host.end());
       g.m_host.insert(g.m_host.end(), p.m_host.begin(), p.m_host.end());
     }
+    g.part_end.push_back(int(k0 + p.K));
     n0 += p.n;
     m0 += p.m;
     k0 += p.K;

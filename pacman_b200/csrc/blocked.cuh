@@ -386,7 +386,7 @@ struct FactorCache {
   DevMem small_list;               // patch ids of the small launches
   DevMem small_fac;                // their L and U factors
   std::vector<SmallRange> ranges;
-  int nbig = 0;                    // the patch size above which the engine took them
+  std::vector<int> lines;          // per patch, the size above which the engine took it
   std::vector<int> rest;           // between both kernels' sizes: nothing kept, solved every execute
   std::vector<int> redo_small, redo_big;  // re-solved by the FP64 LU every execute
   int64_t patches = 0;

@@ -142,6 +142,7 @@ struct Plan {
   DevMem soff, sidx, toff, tidx;  // int64 offsets, int32 ids
   int64_t snnz = 0, tnnz = 0;
   std::vector<int> n_host, m_host;  // per patch sizes
+  std::vector<int> part_end;        // merged plan of a batch: end of each problem's patches
   DevGrid cgrid;                    // grid of centres (weights)
   DevMem torder;                    // targets in the order of the search grid's cells
   DevMem scratch;                   // solver workspace

@@ -514,26 +514,35 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
 void solve_big_cached(Plan &p, FactorCache &c, int basis, const double *vals, int F,
                       double *local, int *status, SolveReport &rep, const BigExtra &extra);
 
-// Patches above this size use the blocked engine (blocked.cu): for the mixed
-// path the tuned value, at most kSmallMax, but kSmallWide where no patch of the
-// plan is larger (the register kernel then takes them all, which saves the
-// engine's set-up and launches: 500k uniform points 3.85 -> 3.68 ms; where the
-// engine runs anyway it takes the patches above 64 along).  Patches without
-// targets count too: a shard of a plan then solves its patches as the whole
-// plan does.  128 for the FP64 and adjoint paths, whose shared-memory kernel is
+// Per patch, the size above which it goes to the blocked engine (blocked.cu):
+// for the mixed path the tuned value, at most kSmallMax, but kSmallWide where no
+// patch of its problem is larger (the register kernel then takes them all, which
+// saves the engine's set-up and launches: 500k uniform points 3.85 -> 3.68 ms;
+// where the engine runs anyway it takes the patches above 64 along).  Patches
+// without targets count too, and the other problems of a batch do not: a shard
+// and a batch then solve a patch as a call with the whole problem alone does.
+// 128 for the FP64 and adjoint paths, whose shared-memory kernel is
 // as fast up to there and takes one launch (250k refined points, 685 patches of
 // 65 to 128 sources: 46.7 ms a call with either line; 150k uniform points,
 // 154 such patches, gradients: 7.77 against 7.97 ms with 64).
-// PACMAN_B200_BIG_N overrides both.
-static int big_threshold(const Plan &p, int mode) {
+// PACMAN_B200_BIG_N overrides all.
+static std::vector<int> size_lines(const Plan &p, int mode) {
+  const auto all = [&](int line) { return std::vector<int>(size_t(p.K), line); };
   const char *e = std::getenv("PACMAN_B200_BIG_N");
-  if (e) return std::max(1, std::atoi(e));
-  if (mode != kChol) return 128;
+  if (e) return all(std::max(1, std::atoi(e)));
+  if (mode != kChol) return all(128);
   const int tuned = tuning_for_current_device().big_n_chol;
-  if (tuned < kSmallMax) return std::max(1, tuned);
-  for (int k = 0; k < p.K; ++k)
-    if (p.n_host[k] > kSmallWide) return kSmallMax;
-  return kSmallWide;
+  if (tuned < kSmallMax) return all(std::max(1, tuned));
+  std::vector<int> lines = all(kSmallWide);
+  const auto n = p.n_host.begin();
+  int k = 0;
+  for (size_t u = 0; k < p.K; ++u) {
+    const int end = u < p.part_end.size() ? p.part_end[u] : p.K;
+    if (end > k && *std::max_element(n + k, n + end) > kSmallWide)
+      std::fill(lines.begin() + k, lines.begin() + end, kSmallMax);
+    k = end;
+  }
+  return lines;
 }
 
 static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F, int precision,
@@ -596,12 +605,12 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
   // definite in FP64 is solved again by the LU below.
   const int mode = precision == PACMAN_B200_FP64 ? kLU : kChol;
   // Kept factors: the line that they were made with, whatever it is now.
-  const int nbig = cached ? cached->nbig : big_threshold(p, mode);
-  if (keep) keep->nbig = nbig;
+  const std::vector<int> nbig = cached ? cached->lines : size_lines(p, mode);
+  if (keep) keep->lines = nbig;
   std::vector<int> small, big;
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;  // no target: the patch contributes nothing
-    (p.n_host[k] > nbig ? big : small).push_back(k);
+    (p.n_host[k] > nbig[k] ? big : small).push_back(k);
   }
   cudaEvent_t ev0, ev1;
   PB_CUDA(cudaEventCreate(&ev0));
@@ -656,11 +665,11 @@ static void solve_patches_impl(Plan &p, int basis, const double *vals_dev, int F
     if (p.m_host[k] == 0) continue;
     if (stat[k] & kStatusDropped) rep.dropped++;
     // Every patch that the LU has not solved already (k_patch_solve takes
-    // kSmallWide < n <= nbig of the FP64 path).
-    const bool other = mode == kChol || p.n_host[k] <= kSmallWide || p.n_host[k] > nbig;
+    // kSmallWide < n <= nbig[k] of the FP64 path).
+    const bool other = mode == kChol || p.n_host[k] <= kSmallWide || p.n_host[k] > nbig[k];
     if ((other && (stat[k] & (kStatusBreakdown | kStatusNonFinite | kStatusTimeout))) ||
         (cached && redo_mark[k]))
-      (p.n_host[k] > nbig ? redo_big : redo_small).push_back(k);
+      (p.n_host[k] > nbig[k] ? redo_big : redo_small).push_back(k);
   }
   if (keep) {
     keep->redo_small = redo_small;
@@ -724,11 +733,11 @@ void solve_adjoint(Plan &p, int basis, int F, const double *h, double *g_out, So
   a.basis = basis;
   a.h = h;
   a.g_out = g_out;
-  const int nbig = big_threshold(p, kAdj);
+  const std::vector<int> nbig = size_lines(p, kAdj);
   std::vector<int> small, big;
   for (int k = 0; k < K; ++k) {
     if (p.m_host[k] == 0) continue;  // h = 0 there: g = 0 (the caller zeroes g)
-    (p.n_host[k] > nbig ? big : small).push_back(k);
+    (p.n_host[k] > nbig[k] ? big : small).push_back(k);
   }
   run_list(p, a, kAdj, small, rep, p.stream);
   BigExtra ex;
