@@ -21,7 +21,7 @@
 //    formulas) whose rotations are applied to u = V^T e_0 and v = V^T b, so
 //    neither V nor A^+ is formed; value = sum over |l_k| > 1e-13 max|l| of
 //    u_k v_k / l_k.
-// 500,000 refined sources -> 500,000 uniform targets: 1.6 + 6.3 ms, against 32.8
+// 500,000 refined sources -> 500,000 uniform targets: 1.6 + 6.1 ms, against 32.8
 // ms for one kernel in the caller's target order, whose search (always 5^3
 // cells or more, a warp's targets scattered over the cloud) kept 12 of 32
 // lanes busy at 8 warps per SM.  The search runs at twice the warps now; the
@@ -35,6 +35,7 @@
 #include <climits>
 #include <cmath>
 
+#include "jacobi.cuh"
 #include "plan.hpp"
 #include "search.cuh"
 
@@ -49,11 +50,6 @@ struct Mls {
   static constexpr int K = DIM == 1 ? 3 : (DIM == 2 ? 6 : 10);
   static constexpr int NP = K * (K + 1) / 2;
 };
-
-// Packed upper-triangle position of (i, j) in an M x M symmetric matrix.
-__host__ __device__ constexpr int sym_at(int i, int j, int M) {
-  return i <= j ? i * M - i * (i - 1) / 2 + (j - i) : j * M - j * (j - 1) / 2 + (i - j);
-}
 
 template <int DIM>
 __device__ __forceinline__ void mls_basis(const double *x, double *p) {
@@ -78,81 +74,6 @@ __device__ __forceinline__ void mls_basis(const double *x, double *p) {
     p[8] = x[1] * x[2];
     p[9] = x[2] * x[2];
   }
-}
-
-// A thread's column of a [K][128] array in shared memory.
-struct MlsColumn {
-  double *p;
-  __device__ __forceinline__ double &operator[](int i) const { return p[128 * i]; }
-};
-
-// Correctly rounded a / b without the compiler's branches, for operands and
-// quotients far from the ends of the exponent range (others, and zero, take
-// the division): r ~ 1 / b, q = a r, then q + r (a - b q) (Markstein, IBM J.
-// Res. Dev. 34(1), 1990).  The rotations' chains are divisions and roots, and
-// with these several of them overlap (k_mls_fit 7.2 -> 6.3 ms at 500,000 targets).
-__device__ __forceinline__ double div_mid(double a, double b) { return quot(a, b, recip(b)); }
-__device__ __forceinline__ double div_any(double a, double b) {
-  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
-  const bool mid = ea > 200 && ea < 1846 && eb > 200 && eb < 1846 && abs(ea - eb) < 900;
-  return mid ? div_mid(a, b) : a / b;
-}
-// Correctly rounded square root for x in [1, 1e40]: two Goldschmidt steps and
-// the residual correction (the same reference).
-__device__ __forceinline__ double root_mid(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double g = x * y, h = 0.5 * y;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const double e = __fma_rn(-g, h, 0.5);
-    g = __fma_rn(g, e, g);
-    h = __fma_rn(h, e, h);
-  }
-  return __fma_rn(__fma_rn(-g, g, x), h, g);
-}
-
-// The rotation annihilating A(P, Q), applied to A, u and v.
-template <int M, int P, int Q>
-__device__ __forceinline__ void mls_rotate(double *a, MlsColumn u, MlsColumn v) {
-  constexpr int pq = sym_at(P, Q, M), pp = sym_at(P, P, M), qq = sym_at(Q, Q, M);
-  const double apq = a[pq];
-  if (apq == 0.0) return;
-  const double app = a[pp], aqq = a[qq];
-  const double g = 100.0 * fabs(apq);
-  if (fabs(app) + g == fabs(app) && fabs(aqq) + g == fabs(aqq)) {
-    a[pq] = 0.0;  // below the rounding of both diagonal entries
-    return;
-  }
-  const double h = aqq - app;
-  double t;
-  if (fabs(h) + g == fabs(h)) {
-    t = div_any(apq, h);
-  } else {
-    const double theta = div_any(0.5 * h, apq);  // at most 1e18: |h| + 100 |apq| > |h|
-    t = div_mid(1.0, fabs(theta) + root_mid(1.0 + theta * theta));
-    if (theta < 0.0) t = -t;
-  }
-  const double c = div_mid(1.0, root_mid(1.0 + t * t));
-  const double s = t * c;
-  const double tau = div_any(s, 1.0 + c);
-  a[pp] = app - t * apq;
-  a[qq] = aqq + t * apq;
-  a[pq] = 0.0;
-#pragma unroll
-  for (int r = 0; r < M; ++r) {
-    if (r == P || r == Q) continue;
-    const int rp = sym_at(r, P, M), rq = sym_at(r, Q, M);
-    const double arp = a[rp], arq = a[rq];
-    a[rp] = arp - s * (arq + tau * arp);
-    a[rq] = arq + s * (arp - tau * arq);
-  }
-  const double up = u[P], uq = u[Q];
-  u[P] = up - s * (uq + tau * up);
-  u[Q] = uq + s * (up - tau * uq);
-  const double vp = v[P], vq = v[Q];
-  v[P] = vp - s * (vq + tau * vp);
-  v[Q] = vq + s * (vp - tau * vq);
 }
 
 // One cyclic sweep over the pairs (P, Q), P < Q, row by row.
