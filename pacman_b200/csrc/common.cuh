@@ -6,6 +6,7 @@
 // never relies on compiler contraction.
 #pragma once
 
+#include <cfloat>
 #include <cstdint>
 #include <type_traits>
 #include <cuda_runtime.h>
@@ -97,7 +98,8 @@ __device__ __forceinline__ T wendland(int basis, T r, T rinv) {
 // sqrt(x) for x >= 0 without branches: the hardware's 1 / sqrt(x) and one
 // Goldschmidt step for g ~ sqrt(x), h ~ 1 / (2 sqrt(x)), then the residual
 // correction g + (x - g g) h (Markstein, IBM J. Res. Dev. 34(1), 1990).  Zero
-// and what the approximation flushes give zero, overflowed squares pass.
+// and the subnormal squares, which the approximation flushes, give zero, an
+// overflowed square stays infinite.
 __device__ __forceinline__ double root(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -106,8 +108,8 @@ __device__ __forceinline__ double root(double x) {
   g = __fma_rn(g, e, g);
   h = __fma_rn(h, e, h);
   g = __fma_rn(__fma_rn(-g, g, x), h, g);
-  g = x < 1e-290 ? 0.0 : g;
-  return x > 1e290 ? x : g;
+  g = x < DBL_MIN ? 0.0 : g;
+  return x > DBL_MAX ? x : g;
 }
 
 // phi at squared distance d2 (common.cuh: wendland with its mask, r >= 0).

@@ -168,6 +168,10 @@ def test_others_are_within_one_ulp(run):
         a = a * np.ldexp(1.0, np.clip(np.frexp(d)[1], -900, 900))
         assert _ulps(run(QUOT, a, d), a / d) <= 1
         assert np.array_equal(run(QUOT, d, d), np.ones_like(d))
-    x = _random(rng, 1 << 21, -963, 963)
+    # Every normal number; the residual of the smallest is subnormal.
+    x = np.r_[_random(rng, 1 << 21, -960, 1024), np.finfo(float).max]
     assert _ulps(run(ROOT, x), np.sqrt(x)) <= 1
-    assert np.array_equal(run(ROOT, np.zeros(4)), np.zeros(4))
+    x = np.r_[_random(rng, 1 << 21, -1022, -960), np.finfo(float).tiny]
+    assert _ulps(run(ROOT, x), np.sqrt(x)) <= 2
+    x = np.array([0.0, 5e-324, np.nextafter(np.finfo(float).tiny, 0.0), np.inf, np.nan])
+    assert np.array_equal(run(ROOT, x), np.array([0.0, 0.0, 0.0, np.inf, np.nan]), equal_nan=True)
