@@ -195,10 +195,11 @@ struct GridView {
   const double4 *sorted;
 };
 
+// Cell index of x along one axis, always in [0, nc): 0 for a NaN, which as an
+// integer would be INT_MIN.
 __device__ __forceinline__ int cell_coord(double x, double lo, double inv_h, int nc) {
   const double f = floor(__dmul_rn(__dsub_rn(x, lo), inv_h));
-  int c = (f < 0.0) ? 0 : (f > double(nc - 1) ? nc - 1 : int(f));
-  return c;
+  return !(f >= 0.0) ? 0 : (f > double(nc - 1) ? nc - 1 : int(f));
 }
 
 // Calls fn(point) for every point of g.sorted in the 3^3 cells around q.

@@ -107,27 +107,29 @@ __global__ void __launch_bounds__(128)
       bd[k] = DBL_MAX;
       bi[k] = INT_MAX;
     }
-    scan_shells<DIM>(
-        g, sorted, h, y,
-        [&](const double4 &x) {
-          const int id = int(x.w);
-          const double d2 = sqdist3(y.x, y.y, y.z, x.x, x.y, x.z);
-          if (!(d2 < bd[K - 1] || (d2 == bd[K - 1] && id < bi[K - 1]))) return;
-          bd[K - 1] = d2;
-          bi[K - 1] = id;
+    // A target with a NaN coordinate has no neighbours: its value is zero.
+    if (!has_nan(y))
+      scan_shells<DIM>(
+          g, sorted, h, y,
+          [&](const double4 &x) {
+            const int id = int(x.w);
+            const double d2 = sqdist3(y.x, y.y, y.z, x.x, x.y, x.z);
+            if (!(d2 < bd[K - 1] || (d2 == bd[K - 1] && id < bi[K - 1]))) return;
+            bd[K - 1] = d2;
+            bi[K - 1] = id;
 #pragma unroll
-          for (int k = K - 1; k > 0; --k) {
-            if (bd[k] < bd[k - 1] || (bd[k] == bd[k - 1] && bi[k] < bi[k - 1])) {
-              const double td = bd[k];
-              bd[k] = bd[k - 1];
-              bd[k - 1] = td;
-              const int ti = bi[k];
-              bi[k] = bi[k - 1];
-              bi[k - 1] = ti;
+            for (int k = K - 1; k > 0; --k) {
+              if (bd[k] < bd[k - 1] || (bd[k] == bd[k - 1] && bi[k] < bi[k - 1])) {
+                const double td = bd[k];
+                bd[k] = bd[k - 1];
+                bd[k - 1] = td;
+                const int ti = bi[k];
+                bi[k] = bi[k - 1];
+                bi[k - 1] = ti;
+              }
             }
-          }
-        },
-        [&] { return bi[K - 1] == INT_MAX ? INFINITY : bd[K - 1]; });
+          },
+          [&] { return bi[K - 1] == INT_MAX ? INFINITY : bd[K - 1]; });
 #pragma unroll
     for (int k = 0; k < K; ++k) nbr[int64_t(k) * M + t] = bi[k];
   }

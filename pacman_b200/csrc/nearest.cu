@@ -29,6 +29,10 @@ __global__ void k_fe_nearest(int64_t M, GridView g, const double4 *__restrict__ 
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < M;
        t += int64_t(gridDim.x) * blockDim.x) {
     const double4 y = tgt[t];
+    if (has_nan(y)) {  // nearest to nothing: zero, as without sources
+      out[int(y.w)] = 0.0;
+      continue;
+    }
     double best = INFINITY;
     int bi = -1;
     scan_shells<DIM>(

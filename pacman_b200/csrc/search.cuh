@@ -24,9 +24,14 @@ __device__ __forceinline__ double scanned_reach(const GridView &g, const double 
   return reach;
 }
 
+__device__ __forceinline__ bool has_nan(const double4 &q) {
+  return isnan(q.x) || isnan(q.y) || isnan(q.z);
+}
+
 // Calls visit(point) for the cell-sorted sources shell by shell; after each
 // shell worst() is the squared distance that a further source would have to
-// beat (infinity while fewer than wanted are known).
+// beat (infinity while fewer than wanted are known).  Not for a query with a NaN
+// coordinate (has_nan), which would visit every cell and find nothing.
 template <int DIM, typename Visit, typename Worst>
 __device__ __forceinline__ void scan_shells(const GridView &g, const double4 *__restrict__ sorted,
                                             double h, const double4 &q, Visit &&visit,
