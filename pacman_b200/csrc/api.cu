@@ -413,6 +413,16 @@ int check_problem(const pacman_b200_problem &q, int32_t i) {
   return 0;
 }
 
+// Work queued on st from here on runs after what `before` holds now.
+void order_after(cudaStream_t st, cudaStream_t before) {
+  cudaEvent_t e;
+  PB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  cudaError_t rc = cudaEventRecord(e, before);
+  if (rc == cudaSuccess) rc = cudaStreamWaitEvent(st, e, 0);
+  cudaEventDestroy(e);
+  PB_CUDA(rc);
+}
+
 struct PlanHandle {
   pacman_b200_plan *h = nullptr;
   PlanHandle() = default;
@@ -424,19 +434,25 @@ struct PlanHandle {
 };
 
 // Host threads that build the per-problem geometry of a batch, one stream
-// each.  The plans keep those streams for their stream-ordered frees, so the
-// streams live until release(), after the plans are gone.
+// each.  Those streams wait for the batch's stream st (device inputs may be on
+// their way there) and st then waits for them: a plan's lists are still being
+// filled when its thread is done with it.  The plans keep the streams for their
+// stream-ordered frees, so the streams live until release(), after the plans are
+// gone.
 struct GeometryWorkers {
   std::vector<cudaStream_t> streams;
   int device = 0;
   int run(const pacman_b200_problem *qs, int32_t count, const pacman_b200_options &o, int dev,
-          std::vector<PlanHandle> &plans) {
+          std::vector<PlanHandle> &plans, cudaStream_t st) {
     int nt = 8;
     if (const char *e = std::getenv("PACMAN_B200_BATCH_THREADS")) nt = std::atoi(e);
     nt = std::max(1, std::min<int>(nt, count));
     streams.assign(size_t(nt), nullptr);
     device = dev;
-    for (auto &s : streams) s = take_stream(dev);
+    for (auto &s : streams) {
+      s = take_stream(dev);
+      order_after(s, st);
+    }
     std::atomic<int> next{0};
     std::atomic<bool> stop{false};
     std::vector<int> rcs(size_t(count), 0);
@@ -462,6 +478,7 @@ struct GeometryWorkers {
     for (auto &t : th) t.join();
     for (int32_t i = 0; i < count; ++i)
       if (rcs[size_t(i)]) return fail(rcs[size_t(i)], "problem " + std::to_string(i) + ": " + msgs[size_t(i)]);
+    for (cudaStream_t s : streams) order_after(st, s);
     return 0;
   }
   void release() {
@@ -629,7 +646,7 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     // overlap those waits and the small launches of different problems.
     GeometryWorkers gw;  // declared first: its streams outlive the plans
     std::vector<PlanHandle> plans(static_cast<size_t>(count));
-    int rc = gw.run(qs, count, o, ds.dev, plans);
+    int rc = gw.run(qs, count, o, ds.dev, plans, st);
     if (rc) {
       plans.clear();
       gw.release();
