@@ -145,6 +145,13 @@ bool is_device_ptr(const void *ptr, int device) {
   return at.type == cudaMemoryTypeDevice && at.device == device;
 }
 
+// On a stream of the library's own: waits for the default stream if any of the
+// caller's arrays is device memory.
+template <typename... Ptr>
+void await_inputs(cudaStream_t own, int device, Ptr... ptrs) {
+  if ((is_device_ptr(ptrs, device) || ...)) await_default_stream(own);
+}
+
 // Device view of a caller array: the pointer itself, or a staged copy.
 struct InBuf {
   DevMem mem;
@@ -226,6 +233,7 @@ int create_plan(int32_t dim, const double *src, int64_t n, const double *tgt, in
     } else {
       p.stream = take_stream(ds.dev);
       p.own_stream = true;
+      await_inputs(p.stream, ds.dev, src, tgt);
     }
     if (n > 0) {
       InBuf s, t;
@@ -411,16 +419,6 @@ int check_problem(const pacman_b200_problem &q, int32_t i) {
   if ((q.target_points == nullptr || q.target_values == nullptr) && q.n_target > 0)
     return fail(PACMAN_B200_ERR_INVALID, at + "target arrays are null but n_target > 0");
   return 0;
-}
-
-// Work queued on st from here on runs after what `before` holds now.
-void order_after(cudaStream_t st, cudaStream_t before) {
-  cudaEvent_t e;
-  PB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  cudaError_t rc = cudaEventRecord(e, before);
-  if (rc == cudaSuccess) rc = cudaStreamWaitEvent(st, e, 0);
-  cudaEventDestroy(e);
-  PB_CUDA(rc);
 }
 
 struct PlanHandle {
@@ -633,6 +631,14 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     if (!o.stream) {
       own = take_stream(ds.dev);
       o.stream = own;
+      for (int32_t i = 0; i < count; ++i)
+        if (is_device_ptr(qs[i].source_points, ds.dev) ||
+            is_device_ptr(qs[i].source_values, ds.dev) ||
+            is_device_ptr(qs[i].target_points, ds.dev) ||
+            is_device_ptr(qs[i].target_values, ds.dev)) {
+          await_default_stream(own);
+          break;
+        }
     }
     cudaStream_t st = static_cast<cudaStream_t>(o.stream);
     cudaEvent_t e0, e1, e2;
@@ -952,6 +958,7 @@ int pacman_b200_fe_interpolate(int32_t dim, int32_t method, const double *src, i
       own = take_stream(ds.dev);
       st = own;
       own_device = ds.dev;
+      await_inputs(own, ds.dev, src, vals, tgt, out, status);
     }
     {
       InBuf s, v, t;
@@ -1017,6 +1024,7 @@ int pacman_b200_mls_interpolate(int32_t dim, const double *src, int64_t n, const
       own = take_stream(ds.dev);
       st = own;
       own_device = ds.dev;
+      await_inputs(own, ds.dev, src, vals, tgt, out);
     }
     {
       InBuf s, v, t;

@@ -110,12 +110,16 @@ struct AuxStreams {
   Set *set_ = nullptr;
 };
 
-// A stream of the library's own for a call without one, ordered after the
-// work already queued on the legacy default stream (device inputs may still
-// be on their way there).  Kept idle like AuxStreams; give_stream waits for
-// what is queued on it first.
+// A stream of the library's own for a call without one.  Kept idle like
+// AuxStreams; give_stream waits for what is queued on it first.
 cudaStream_t take_stream(int device);
 void give_stream(cudaStream_t s, int device);
+// Work queued on st from here on runs after what `before` holds now.
+void order_after(cudaStream_t st, cudaStream_t before);
+// The same for the legacy default stream, for a call on a stream of the
+// library's own that was given device memory (which may still be on its way
+// there).  Calls on host memory have nothing to wait for.
+void await_default_stream(cudaStream_t s);
 
 // Factorisations kept by an execute with PACMAN_B200_KEEP_FACTORS (defined
 // in blocked.cuh; destroyed through destroy_factor_cache).

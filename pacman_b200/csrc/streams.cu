@@ -87,17 +87,25 @@ cudaStream_t take_stream(int device) {
     }
   }
   if (!s) PB_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  return s;
+}
+
+void order_after(cudaStream_t st, cudaStream_t before) {
+  cudaEvent_t e;
+  PB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  cudaError_t rc = cudaEventRecord(e, before);
+  if (rc == cudaSuccess) rc = cudaStreamWaitEvent(st, e, 0);
+  cudaEventDestroy(e);
+  PB_CUDA(rc);
+}
+
+void await_default_stream(cudaStream_t s) {
   // Not while a capture is under way that the legacy stream would break.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaEvent_t e = nullptr;
   if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) == cudaSuccess &&
-      cap == cudaStreamCaptureStatusNone &&
-      cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
-    if (cudaEventRecord(e, cudaStreamLegacy) == cudaSuccess) cudaStreamWaitEvent(s, e, 0);
-    cudaEventDestroy(e);
-  }
+      cap == cudaStreamCaptureStatusNone)
+    order_after(s, cudaStreamLegacy);
   cudaGetLastError();
-  return s;
 }
 
 void give_stream(cudaStream_t s, int device) {
