@@ -72,7 +72,8 @@ typedef struct pacman_b200_options {
   double support_radius;     /* 0.1: interpolator.hxx:41 (absolute basis support) */
   int32_t precision;         /* PACMAN_B200_FP64 or PACMAN_B200_MIXED */
   int32_t device;            /* CUDA device ordinal, -1 = the current device */
-  void *stream;              /* cudaStream_t to run on, NULL = a library-owned stream */
+  void *stream;              /* cudaStream_t to run on, NULL = a library-owned stream, which
+                                waits for the default stream in calls on device memory */
 } pacman_b200_options;
 
 typedef struct pacman_b200_stats {

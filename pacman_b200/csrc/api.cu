@@ -265,6 +265,7 @@ int execute_plan(pacman_b200_plan *h, int32_t basis, const double *vals, int32_t
     DeviceScope ds(p.device);
     HostArena::get().reset();
     cudaStream_t st = p.stream;
+    if (p.own_stream) await_inputs(st, p.device, vals, out);
     cudaEvent_t e0, e1, e2;
     PB_CUDA(cudaEventCreate(&e0));
     PB_CUDA(cudaEventCreate(&e1));
@@ -799,6 +800,7 @@ int pacman_b200_plan_adjoint(pacman_b200_plan *plan, const double *grad_out, dou
     DeviceScope ds(p.device);
     HostArena::get().reset();
     cudaStream_t st = p.stream;
+    if (p.own_stream) await_inputs(st, p.device, grad_out, grad_values, grad_targets);
     const int F = p.saved_F;
     InBuf g;
     g.stage(grad_out, size_t(p.m) * F, p.device, st);

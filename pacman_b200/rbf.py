@@ -221,6 +221,17 @@ def _empty_like_kind(kind, shape, ref):
     return a.ctypes.data, a
 
 
+def _await_current_stream(kind, device):
+    """A plan runs on a stream of its own, which waits for the default stream
+    where it is given device memory; what torch has queued on another stream is
+    waited for here."""
+    if kind == "cuda":
+        import torch
+        stream = torch.cuda.current_stream(device)
+        if stream != torch.cuda.default_stream(device):
+            stream.synchronize()
+
+
 class Plan:
     """Reusable transfer plan: geometry built once, ``execute`` per field set.
 
@@ -240,6 +251,7 @@ class Plan:
         self.n, self.m = sp_shape[0], tp_shape[0]
         if kind == "cuda" and device is None:
             device = self._sp.device.index
+        _await_current_stream(kind, device)
         opts = _options(nodes_per_cluster, relative_overlap, support_radius, precision, device,
                         None)
         h = ctypes.c_void_p()
@@ -334,6 +346,7 @@ class Plan:
             raise ValueError("source values must have one row per source point")
         F = 1 if len(shape) == 1 else shape[1]
         out_ptr, out = _empty_like_kind(kind, (self.m,) if len(shape) == 1 else (self.m, F), keep)
+        _await_current_stream(kind, keep.device if kind == "cuda" else None)
         st = _lib.Stats()
         flags = (_lib.SAVE_FOR_ADJOINT if save_for_adjoint else 0) | (
             _lib.TIME_KERNELS if time_kernels else 0) | (_lib.KEEP_FACTORS if keep_factors else 0)
@@ -355,6 +368,7 @@ class Plan:
         vshape = (self.n,) if self._vector else (self.n, F)
         gv_ptr, gv = _empty_like_kind(kind, vshape, keep) if values else (None, None)
         gt_ptr, gt = _empty_like_kind(kind, (self.m, self.dim), keep) if targets else (None, None)
+        _await_current_stream(kind, keep.device if kind == "cuda" else None)
         rc = self._lib.pacman_b200_plan_adjoint(self._h, ptr, gv_ptr, gt_ptr)
         _lib.raise_for(rc, "pacman.rbf.Plan.adjoint")
         return gv, gt

@@ -1,5 +1,6 @@
-"""Calls on the library's own stream and the work queued on the default stream:
-calls on host arrays do not wait for it."""
+"""Calls on the library's own stream and the work queued on the caller's: calls on
+host arrays do not wait for the default stream, calls on device tensors run
+after what torch has queued on its current stream."""
 import numpy as np
 import pytest
 
@@ -44,3 +45,35 @@ def test_host_arrays_do_not_wait(call):
     torch.cuda.synchronize()
     assert not waited
     assert np.array_equal(got, want)
+
+
+def _gpu(*arrays):
+    return [torch.tensor(a, device="cuda") for a in arrays]
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_plan_waits_for_device_tensors(side):
+    grad = RNG.standard_normal(len(T))
+    plan = pacman_b200.rbf.Plan(3, S, T)
+    want = plan.execute(0x11, V, save_for_adjoint=True)
+    want_v, want_t = plan.adjoint(grad)
+    final = _gpu(S, T, V, grad)
+    sources, targets, values, upstream = early = _gpu(
+        RNG.random(S.shape), RNG.random(T.shape), np.zeros(len(S)), np.zeros(len(T)))
+    stream = torch.cuda.Stream() if side else torch.cuda.default_stream()
+    torch.cuda.synchronize()
+
+    def late(*which):
+        torch.cuda._sleep(50_000_000)  # some 25 ms
+        for i in which:
+            early[i].copy_(final[i])
+    with torch.cuda.stream(stream):
+        late(0, 1)
+        plan = pacman_b200.rbf.Plan(3, sources, targets)
+        late(2)
+        out = plan.execute(0x11, values, save_for_adjoint=True)
+        late(3)
+        gv, gt = plan.adjoint(upstream)
+        out, gv, gt = (x.cpu().numpy() for x in (out, gv, gt))
+    assert np.array_equal(out, want)
+    assert np.array_equal(gv, want_v) and np.array_equal(gt, want_t)
