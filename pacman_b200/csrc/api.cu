@@ -245,7 +245,8 @@ int create_plan(int32_t dim, const double *src, int64_t n, const double *tgt, in
       p.syncs_geometry = host_sync_counter() - h0;
     }
   } catch (const Error &e) {
-    delete h;
+    settle(p);
+    pacman_b200_plan_destroy(h);
     return fail(e.code, e.msg);
   }
   *out = h;
@@ -349,6 +350,7 @@ int execute_plan(pacman_b200_plan *h, int32_t basis, const double *vals, int32_t
     cudaEventDestroy(e1);
     cudaEventDestroy(e2);
   } catch (const Error &e) {
+    settle(p);
     return fail(e.code, e.msg);
   }
   return 0;
@@ -653,6 +655,11 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     // overlap those waits and the small launches of different problems.
     GeometryWorkers gw;  // declared first: its streams outlive the plans
     std::vector<PlanHandle> plans(static_cast<size_t>(count));
+    // Destroyed first: what st still does with the plans' buffers is over then.
+    struct Settle {
+      cudaStream_t st;
+      ~Settle() { cudaStreamSynchronize(st); }
+    } settled{st};
     int rc = gw.run(qs, count, o, ds.dev, plans, st);
     if (rc) {
       plans.clear();
@@ -821,6 +828,7 @@ int pacman_b200_plan_adjoint(pacman_b200_plan *plan, const double *grad_out, dou
     if (ht) PB_CUDA(cudaMemcpyAsync(grad_targets, dt, sizeof(double) * p.m * p.dim, cudaMemcpyDeviceToHost, st));
     PB_CUDA(host_sync(st));
   } catch (const Error &e) {
+    settle(p);
     return fail(e.code, e.msg);
   }
   return 0;
@@ -989,6 +997,7 @@ int pacman_b200_fe_interpolate(int32_t dim, int32_t method, const double *src, i
     give_stream(own, own_device);
     own = nullptr;
   } catch (const Error &e) {
+    if (o.stream) cudaStreamSynchronize(static_cast<cudaStream_t>(o.stream));
     give_stream(own, own_device);
     return fail(e.code, e.msg);
   }
@@ -1049,6 +1058,7 @@ int pacman_b200_mls_interpolate(int32_t dim, const double *src, int64_t n, const
     give_stream(own, own_device);
     own = nullptr;
   } catch (const Error &e) {
+    if (o.stream) cudaStreamSynchronize(static_cast<cudaStream_t>(o.stream));
     give_stream(own, own_device);
     return fail(e.code, e.msg);
   }

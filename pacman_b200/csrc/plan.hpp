@@ -101,6 +101,9 @@ struct AuxStreams {
   cudaStream_t *s = nullptr;
   cudaEvent_t *ev = nullptr;
   void make();                      // for the current device
+  void wait() const {               // for what is queued on them
+    for (int i = 0; s && i <= kN; ++i) cudaStreamSynchronize(s[i]);
+  }
   AuxStreams() = default;
   AuxStreams(const AuxStreams &) = delete;
   AuxStreams &operator=(const AuxStreams &) = delete;
@@ -181,11 +184,19 @@ struct Plan {
   std::unique_ptr<FactorCache, FactorCacheDeleter> fcache;  // kept factorisations, or null
 };
 
+// Waits for whatever a failed call has left queued, so that its buffers (freed on
+// one stream, used on others) and the pinned staging can go to others.
+inline void settle(const Plan &p) {
+  p.aux.wait();
+  if (p.stream) cudaStreamSynchronize(p.stream);
+  cudaGetLastError();
+}
+
 // Pinned host staging for the small host-to-device uploads of one call.  A
 // copy from pageable memory first synchronises its stream, which would stall
 // the host behind every queued kernel; copies from this arena do not.  The
 // arena is reset at the start of each call (the previous call synchronised
-// before returning), blocks outgrown in the middle of a call are released at
+// before returning, also where it failed), blocks outgrown in the middle of a call are released at
 // the next reset.
 class HostArena {
  public:

@@ -706,6 +706,7 @@ void solve_patches(Plan &p, int basis, const double *vals_dev, int F, int precis
   try {
     solve_patches_impl(p, basis, vals_dev, F, precision, local_dev, rep, save, keep_factors);
   } catch (...) {
+    settle(p);
     if (keep_factors) p.fcache.reset();  // a half-built cache is never reused
     throw;
   }
