@@ -751,12 +751,20 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
     a.dpart = nullptr;
     DevMem ddiag;
     if (oz && tot_sl > 0) {
-      dsl.alloc(size_t(tot_sl), st);
-      a.slices = dsl.as<uint8_t>();
-      // The int8 steps' next diagonal tile: D' (TB x TB per slot), written by
-      // the step's diagonal item and factored by k_diag_next.
-      ddiag.alloc(sizeof(double) * TB * TB * size_t(ns), st);
-      a.dpart = ddiag.as<double>();
+      // A wave of one patch may be larger than the budget.  Where its slices
+      // (as much memory again as W) do not fit beside W, it is factored with
+      // FP64 updates, which need none.
+      try {
+        dsl.alloc(size_t(tot_sl), st);
+        // The int8 steps' next diagonal tile: D' (TB x TB per slot), written by
+        // the step's diagonal item and factored by k_diag_next.
+        ddiag.alloc(sizeof(double) * TB * TB * size_t(ns), st);
+        a.slices = dsl.as<uint8_t>();
+        a.dpart = ddiag.as<double>();
+      } catch (const Error &) {
+        if (ns > 1) throw;
+        dsl.release();
+      }
     }
     const size_t n_inv = lu ? size_t(2) * TB * TB * ns : size_t(tot_inv);
     const size_t n_beta = size_t(4) * kMaxF * ns;
