@@ -750,7 +750,7 @@ void solve_big(Plan &p, int basis, const double *vals, int F, BigSolver solver,
     a.slices = nullptr;
     a.dpart = nullptr;
     DevMem ddiag;
-    if (oz && tot_sl > 0) {
+    if (oz && tot_sl > 0 && slots.front().T <= kOzMaxT) {
       // A wave of one patch may be larger than the budget.  Where its slices
       // (as much memory again as W) do not fit beside W, it is factored with
       // FP64 updates, which need none.

@@ -355,6 +355,14 @@ struct CholPlan {
 };
 CholPlan chol_prefix(const std::vector<BigSlot> &slots);
 void chol_set_smem_attributes();
+// Tile rows up to which the int8 steps' int32 sums cannot overflow: K = 86,912
+// columns at most.  Digits below the first are at most 64 in magnitude, so the
+// six pairs of level 9 add at most 24,576 per column; of level 8's seven pairs
+// the five without a first digit add 20,480, and the two with one at most 64 256
+// sqrt(K) each altogether (a row of L has norm sigma or less, and a first digit
+// is 0 or at most twice the number it rounds, so a row's first digits have norm
+// 256 or less).  Larger patches take FP64 updates.
+constexpr int kOzMaxT = 1359;
 // Bytes of int8 slice tiles of a slot with T tile rows (strictly lower tiles,
 // plain and in row pairs).
 size_t oz_slot_bytes(int T);

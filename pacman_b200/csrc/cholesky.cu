@@ -967,7 +967,7 @@ __device__ __forceinline__ void ws_mma_half(uint32_t tmem, uint32_t sA, uint32_t
 // An epilogue warp reads TMEM lanes 32 qd .. + 31 (rows of the pair) and
 // columns 16 h .. + 15 of every column group: the sums of levels 2..9 of its
 // rows.  The levels are merged in int64 first: a level's sum is below 2^31
-// (at most 36,700 per column of K: 58,000 columns), so the top three shifted
+// (kOzMaxT), so the top three shifted
 // by 7 bits each stay below 2^53 and convert exactly, and the lower five
 // (below 2^60 in units of 128^-9) round to within 2^-57; then two FP64 terms
 // (in units of sigma^2), of which sig2 x their sum is subtracted from sC
