@@ -494,7 +494,7 @@ __device__ __forceinline__ int cell_of(const GridSpec &g, const double4 &p) {
 // about 9 for each.
 __global__ void k_cell_count(const double4 *__restrict__ p0, int64_t n0, GridSpec g0,
                              const double4 *__restrict__ p1, int64_t n1, GridSpec g1,
-                             int *__restrict__ count, int *__restrict__ rank) {
+                             unsigned *__restrict__ count, int *__restrict__ rank) {
   const int lane = threadIdx.x & 31;
   for (int64_t b = blockIdx.x * (int64_t)blockDim.x; b < n0 + n1;
        b += (int64_t)gridDim.x * blockDim.x) {  // block-uniform: whole warps vote below
@@ -511,10 +511,10 @@ __global__ void k_cell_count(const double4 *__restrict__ p0, int64_t n0, GridSpe
     int r = 0;
     if (m) {
       const int leader = __ffs(m) - 1;
-      if (lane == leader) r = atomicAdd(&count[c], __popc(m));
+      if (lane == leader) r = int(atomicAdd(&count[c], unsigned(__popc(m))));
       r = __shfl_sync(0xffffffffu, r, leader) + __popc(m & ((1u << lane) - 1u));
     }
-    if (live) rank[i] = out ? r : atomicAdd(&count[c], 1);
+    if (live) rank[i] = out ? r : int(atomicAdd(&count[c], 1u));
   }
 }
 
@@ -522,7 +522,7 @@ __global__ void k_cell_count(const double4 *__restrict__ p0, int64_t n0, GridSpe
 // exact).
 __global__ void k_cell_place(const double4 *__restrict__ p0, int64_t n0, GridSpec g0,
                              const double4 *__restrict__ p1, int64_t n1, GridSpec g1,
-                             const int *__restrict__ start, const int *__restrict__ rank,
+                             const unsigned *__restrict__ start, const int *__restrict__ rank,
                              double4 *__restrict__ sorted) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n0 + n1;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -530,7 +530,7 @@ __global__ void k_cell_place(const double4 *__restrict__ p0, int64_t n0, GridSpe
     double4 p = first ? p0[i] : p1[i - n0];
     const int c = first ? cell_of(g0, p) : g0.ncells + 1 + cell_of(g1, p);
     p.w = double(first ? i : i - n0);
-    sorted[start[c] + rank[i]] = p;
+    sorted[start[c] + unsigned(rank[i])] = p;
   }
 }
 
@@ -540,7 +540,7 @@ __global__ void k_ids(const double4 *__restrict__ pts, int64_t n, int *__restric
     out[i] = int(pts[i].w);
 }
 
-GridView view_of(const GridSpec &g, const int *start) {
+GridView view_of(const GridSpec &g, const unsigned *start) {
   GridView v{};
   for (int d = 0; d < 3; ++d) {
     v.lo[d] = g.lo[d];
@@ -548,7 +548,7 @@ GridView view_of(const GridSpec &g, const int *start) {
   }
   v.inv_h = g.inv_h;
   v.ncells = g.ncells;
-  v.start = start;
+  v.start = reinterpret_cast<const int *>(start);
   return v;
 }
 
@@ -564,24 +564,25 @@ struct Slab {
 };
 
 // Sorts set 0 (and set 1) into the cells of g0 (and g1), each followed by its
-// points outside the domain: set 1 starts at sorted[n0].  With a null slab the
+// points outside the domain: set 1 starts at sorted[n0].  Each set has less than
+// 2^31 points; positions in both together are unsigned.  With a null slab the
 // call only counts the memory it needs.
 void sort_into_cells(Slab &slab, const double4 *p0, int64_t n0, const GridSpec &g0,
                      const double4 *p1, int64_t n1, const GridSpec &g1, GridView &v0, GridView &v1,
                      const double4 *&sorted, cudaStream_t st) {
   const size_t cells = size_t(g0.ncells) + 1 + size_t(n1 > 0 ? g1.ncells + 1 : 0);
   const size_t npts = size_t(std::max<int64_t>(n0 + n1, 1));
-  if (cells + 1 > 0x7fffffffull || npts > 0x7fffffffull)
-    throw Error{PACMAN_B200_ERR_LIMIT, "more than 2^31 - 1 points or cells in one search grid"};
-  int *count = slab.take<int>(cells + 1);
-  int *start = slab.take<int>(cells + 1);
+  if (cells + 1 > 0x7fffffffull)
+    throw Error{PACMAN_B200_ERR_LIMIT, "more than 2^31 - 1 cells in one search grid"};
+  unsigned *count = slab.take<unsigned>(cells + 1);
+  unsigned *start = slab.take<unsigned>(cells + 1);
   int *rank = slab.take<int>(npts);
   double4 *out = slab.take<double4>(npts);
   size_t tb = 0;
   PB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, count, start, int(cells + 1), st));
   void *tmp = slab.take<char>(tb);
   if (!slab.cur) return;
-  PB_CUDA(cudaMemsetAsync(count, 0, sizeof(int) * (cells + 1), st));
+  PB_CUDA(cudaMemsetAsync(count, 0, sizeof(unsigned) * (cells + 1), st));
   k_cell_count<<<grid_for(n0 + n1), kThreads, 0, st>>>(p0, n0, g0, p1, n1, g1, count, rank);
   PB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, count, start, int(cells + 1), st));
   k_cell_place<<<grid_for(n0 + n1), kThreads, 0, st>>>(p0, n0, g0, p1, n1, g1, start, rank, out);
@@ -660,7 +661,7 @@ void build_grid(DevGrid &out, const double4 *pts, int64_t n, int dim, const doub
     PB_CUDA(cudaMemsetAsync(out.start.p, 0, sizeof(int) * (size_t(g.ncells) + 1), st));
   }
   PB_CUDA(cudaGetLastError());
-  out.view = view_of(g, out.start.as<int>());
+  out.view = view_of(g, out.start.as<unsigned>());
   out.view.sorted = out.sorted.as<double4>();
 }
 
@@ -693,18 +694,17 @@ __device__ __forceinline__ void warp_neighbors(const GridView &g, const double4 
   const int z0 = max(cz - 1, 0), z1 = min(cz + 1, g.nc[2] - 1);
   const int ny = y1 - y0 + 1, runs = (x1 - x0 + 1) * ny;
   // Lane r < runs (at most 9) holds the r-th run of cells [s, e).
-  int rs = 0, re = 0;
+  unsigned rs = 0, re = 0;
   if (lane < runs) {
     const int base = ((x0 + lane / ny) * g.nc[1] + y0 + lane % ny) * g.nc[2];
-    rs = g.start[base + z0];
-    re = g.start[base + z1 + 1];
+    rs = unsigned(g.start[base + z0]);
+    re = unsigned(g.start[base + z1 + 1]);
   }
   for (int r = 0; r < runs; ++r) {
-    const int s = __shfl_sync(0xffffffffu, rs, r), e = __shfl_sync(0xffffffffu, re, r);
-    for (int i0 = s; i0 < e; i0 += 32) {
-      const int i = i0 + lane;
-      const bool ok = i < e;
-      if (!fn(pts[ok ? i : s], ok)) return;
+    const unsigned s = __shfl_sync(0xffffffffu, rs, r), e = __shfl_sync(0xffffffffu, re, r);
+    for (unsigned u = lane; u - lane < e - s; u += 32) {
+      const bool ok = u < e - s;
+      if (!fn(pts[ok ? s + u : s], ok)) return;
     }
   }
 }

@@ -254,13 +254,16 @@ void mls_interpolate(int dim, const double *src_dev, int64_t n, const double *va
     PB_CUDA(cudaMemsetAsync(out_dev, 0, sizeof(double) * size_t(m), st));
     return;
   }
-  PointSearch ps;
-  // Cells 1.5 times as wide as for one source each: the ten nearest of a
-  // uniform cloud then mostly lie in the 3^3 cells around the target.
-  build_point_search(ps, dim, src_dev, n, tgt_dev, m, 1.5, st);
-  if (dim == 1) launch_mls<1>(ps, m, vals_dev, n, out_dev, st);
-  else if (dim == 2) launch_mls<2>(ps, m, vals_dev, n, out_dev, st);
-  else launch_mls<3>(ps, m, vals_dev, n, out_dev, st);
+  for (int64_t t0 = 0; t0 < m; t0 += kSearchTargets) {
+    const int64_t M = std::min(m - t0, kSearchTargets);
+    PointSearch ps;
+    // Cells 1.5 times as wide as for one source each: the ten nearest of a
+    // uniform cloud then mostly lie in the 3^3 cells around the target.
+    build_point_search(ps, dim, src_dev, n, tgt_dev + t0 * dim, M, 1.5, st);
+    if (dim == 1) launch_mls<1>(ps, M, vals_dev, n, out_dev + t0, st);
+    else if (dim == 2) launch_mls<2>(ps, M, vals_dev, n, out_dev + t0, st);
+    else launch_mls<3>(ps, M, vals_dev, n, out_dev + t0, st);
+  }
   PB_CUDA(host_sync(st));
 }
 

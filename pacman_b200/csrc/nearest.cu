@@ -59,18 +59,21 @@ void fe_nearest(int dim, const double *src_dev, int64_t n, const double *vals_de
     PB_CUDA(cudaMemsetAsync(out_dev, 0, sizeof(double) * size_t(m), st));
     return;
   }
-  PointSearch ps;
-  build_point_search(ps, dim, src_dev, n, tgt_dev, m, 1.0, st);
-  const double h = 1.0 / ps.grid.inv_h;
-  const int blocks = int(std::max<int64_t>(1, std::min<int64_t>((m + 127) / 128, 148 * 64)));
-  auto go = [&](auto kernel) {
-    kernel<<<blocks, 128, 0, st>>>(m, ps.grid, ps.sorted, h, vals_dev, out_dev);
-  };
-  if (dim == 1) go(k_fe_nearest<1>);
-  else if (dim == 2) go(k_fe_nearest<2>);
-  else go(k_fe_nearest<3>);
-  note_launch();
-  PB_CUDA(cudaGetLastError());
+  for (int64_t t0 = 0; t0 < m; t0 += kSearchTargets) {
+    const int64_t M = std::min(m - t0, kSearchTargets);
+    PointSearch ps;
+    build_point_search(ps, dim, src_dev, n, tgt_dev + t0 * dim, M, 1.0, st);
+    const double h = 1.0 / ps.grid.inv_h;
+    const int blocks = int(std::max<int64_t>(1, std::min<int64_t>((M + 127) / 128, 148 * 64)));
+    auto go = [&](auto kernel) {
+      kernel<<<blocks, 128, 0, st>>>(M, ps.grid, ps.sorted, h, vals_dev, out_dev + t0);
+    };
+    if (dim == 1) go(k_fe_nearest<1>);
+    else if (dim == 2) go(k_fe_nearest<2>);
+    else go(k_fe_nearest<3>);
+    note_launch();
+    PB_CUDA(cudaGetLastError());
+  }
   PB_CUDA(host_sync(st));
 }
 

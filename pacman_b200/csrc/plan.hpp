@@ -262,6 +262,9 @@ struct PointSearch {
   GridView grid{};               // start only
   const double4 *sorted = nullptr;
 };
+// Targets of one such search (callers take more in turns: their packed and
+// sorted copies take 68 bytes each).
+constexpr int64_t kSearchTargets = int64_t(1) << 28;
 void build_point_search(PointSearch &ps, int dim, const double *src_dev, int64_t n,
                         const double *tgt_dev, int64_t m, double scale, cudaStream_t st);
 // Finite-element NEAREST_NEAREST transfer (nearest.cu).
