@@ -2032,7 +2032,8 @@ void chol_launch_steps(const BigArgs &a, const BigSlot *ds, const std::vector<Bi
       const int items = cp.pre[cp.ioff[j] + c];
       // Programmatic dependent launch: the step's copies and MMAs overlap
       // the tail of the previous k_diag_next (see griddepcontrol.wait in the
-      // kernel); without kernel timing, where events separate the launches.
+      // kernel); not behind an FP64 step, whose slices the copies read, and
+      // not with kernel timing, where events separate the launches.
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(std::min(items, sms));
       cfg.blockDim = dim3(kWsThreads);
@@ -2040,7 +2041,7 @@ void chol_launch_steps(const BigArgs &a, const BigSlot *ds, const std::vector<Bi
       cfg.stream = st;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = rep.time_kernels ? 0 : 1;
+      attr[0].val.programmaticStreamSerializationAllowed = rep.time_kernels || j == oz_from ? 0 : 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       PB_CUDA(cudaLaunchKernelEx(&cfg, k_col_step_ws, a, ds, static_cast<const int *>(dpre + cp.ioff[j]), c, j));
