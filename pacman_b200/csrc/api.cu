@@ -289,11 +289,13 @@ int execute_plan(pacman_b200_plan *h, int32_t basis, const double *vals, int32_t
       } else {
         InBuf v;
         v.stage(vals, size_t(p.n) * F, p.device, st);
+        p.local_count = 0;
         p.local.alloc(sizeof(double) * size_t(std::max<int64_t>(p.tnnz, 1)) * F, st);
         rep.time_kernels = (flags & PACMAN_B200_TIME_KERNELS) != 0;
         solve_patches(p, basis, v.ptr, F, p.opts.precision, p.local.as<double>(), rep,
                       (flags & PACMAN_B200_SAVE_FOR_ADJOINT) != 0,
                       (flags & PACMAN_B200_KEEP_FACTORS) != 0);
+        p.local_count = p.tnnz * F;
         PB_CUDA(cudaEventRecord(e1, st));
         pu_gather(p, p.local.as<double>(), F, o);
       }
@@ -916,7 +918,9 @@ int pacman_b200_plan_local_values(const pacman_b200_plan *plan, double *local) {
   if (!p.local.p) return fail(PACMAN_B200_ERR_INVALID, "plan has not been executed");
   try {
     DeviceScope ds(p.device);
-    PB_CUDA(cudaMemcpyAsync(local, p.local.p, p.local.bytes, cudaMemcpyDefault, p.stream));
+    if (p.local_count > 0)
+      PB_CUDA(cudaMemcpyAsync(local, p.local.p, sizeof(double) * size_t(p.local_count),
+                              cudaMemcpyDefault, p.stream));
     PB_CUDA(host_sync(p.stream));
   } catch (const Error &e) {
     return fail(e.code, e.msg);

@@ -154,6 +154,7 @@ struct Plan {
   DevMem torder;                    // targets in the order of the search grid's cells
   DevMem scratch;                   // solver workspace
   DevMem local;                     // per (patch, target) local values
+  int64_t local_count = 0;          // how many, of the last execute (the block may be larger)
   DevMem status;                    // per patch status words
   std::vector<int> patch_status;    // status words of the last execute (host copy)
   double ms_geometry = -1.0;         // device time of the geometry (read lazily)
