@@ -137,7 +137,12 @@ void shard_plan(Plan &p, int rank, int world) {
   cudaStream_t st = p.stream;
   const int64_t M = p.m;
   const int K = p.K;
-  p.fcache.reset();  // kept factors were laid out for the unsharded target lists
+  // Kept factors, local values and the state saved for the adjoint were laid out
+  // for the unsharded target lists.
+  p.fcache.reset();
+  p.local.release();
+  p.local_count = 0;
+  p.saved_basis = -1;
   p.shard_rank = rank;
   p.shard_world = world;
   if (M == 0) {
