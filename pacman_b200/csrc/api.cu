@@ -657,15 +657,19 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     // overlap those waits and the small launches of different problems.
     GeometryWorkers gw;  // declared first: its streams outlive the plans
     std::vector<PlanHandle> plans(static_cast<size_t>(count));
-    // Destroyed first: what st still does with the plans' buffers is over then.
+    // Where a call fails: destroyed before the plans, so that what st still does
+    // with their buffers is over (the other ways out give st back before that).
     struct Settle {
       cudaStream_t st;
-      ~Settle() { cudaStreamSynchronize(st); }
-    } settled{st};
+      ~Settle() {
+        if (st) cudaStreamSynchronize(st);
+      }
+    } settle_on_error{st};
     int rc = gw.run(qs, count, o, ds.dev, plans, st);
     if (rc) {
       plans.clear();
       gw.release();
+      settle_on_error.st = nullptr;
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       cudaEventDestroy(e2);
@@ -747,6 +751,7 @@ int run_batch(const pacman_b200_problem *qs, int32_t count, const pacman_b200_op
     cudaEventDestroy(e2);
     plans.clear();
     gw.release();
+    settle_on_error.st = nullptr;
     give_stream(own, ds.dev);
     own = nullptr;
   } catch (const Error &e) {
