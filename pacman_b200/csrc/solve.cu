@@ -332,26 +332,26 @@ static size_t smem_bytes(int n, int F, bool with_A) {
   return d * sizeof(double);
 }
 
+// Dynamic shared memory that every launch of k_patch_solve is allowed, whatever
+// it asks for: the limit belongs to the kernel, not to the launch, and other
+// threads' launches come between.
+constexpr size_t kSolveSmem = 220 * 1024;
+
+template <int MODE>
+static void launch_mode(const PatchArgs &a, const int *plist, int np, int use_global, size_t smem,
+                        cudaStream_t st) {
+  PB_CUDA(cudaFuncSetAttribute(k_patch_solve<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(std::max(smem, kSolveSmem))));
+  k_patch_solve<MODE><<<np, kSolveThreads, smem, st>>>(a, plist, np, use_global);
+  note_launch();
+  PB_CUDA(cudaGetLastError());
+}
 static void launch(int mode, const PatchArgs &a, const int *plist, int np, int use_global,
                    size_t smem, cudaStream_t st) {
   if (np == 0) return;
-  if (mode == kLU) {
-    PB_CUDA(cudaFuncSetAttribute(k_patch_solve<kLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem)));
-    k_patch_solve<kLU><<<np, kSolveThreads, smem, st>>>(a, plist, np, use_global);
-    note_launch();
-  } else if (mode == kAdj) {
-    PB_CUDA(cudaFuncSetAttribute(k_patch_solve<kAdj>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    k_patch_solve<kAdj><<<np, kSolveThreads, smem, st>>>(a, plist, np, use_global);
-    note_launch();
-  } else {
-    PB_CUDA(cudaFuncSetAttribute(k_patch_solve<kChol>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    k_patch_solve<kChol><<<np, kSolveThreads, smem, st>>>(a, plist, np, use_global);
-    note_launch();
-  }
-  PB_CUDA(cudaGetLastError());
+  if (mode == kLU) launch_mode<kLU>(a, plist, np, use_global, smem, st);
+  else if (mode == kAdj) launch_mode<kAdj>(a, plist, np, use_global, smem, st);
+  else launch_mode<kChol>(a, plist, np, use_global, smem, st);
 }
 
 // Polynomial results of `count` register-kernel patches (launch_small_poly).
