@@ -560,13 +560,13 @@ static int64_t count_strips(const BigSlot &q, int s) {
 }
 
 static void set_smem_attributes() {
-  static bool done = false;
-  if (done) return;
-  const int s3 = 3 * TB * LDS * sizeof(double), s2 = 2 * TB * LDS * sizeof(double);
-  PB_CUDA(cudaFuncSetAttribute(k_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
-  PB_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
-  PB_CUDA(cudaFuncSetAttribute(k_update_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
-  done = true;
+  static OncePerDevice once;
+  once([] {
+    const int s3 = 3 * TB * LDS * sizeof(double), s2 = 2 * TB * LDS * sizeof(double);
+    PB_CUDA(cudaFuncSetAttribute(k_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
+    PB_CUDA(cudaFuncSetAttribute(k_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
+    PB_CUDA(cudaFuncSetAttribute(k_update_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, s3));
+  });
 }
 
 // Solves the listed patches (each with m > 0) with the blocked engine.  The

@@ -1960,9 +1960,7 @@ CholPlan chol_prefix(const std::vector<BigSlot> &slots) {
   return cp;
 }
 
-void chol_set_smem_attributes() {
-  static bool done = false;
-  if (done) return;
+static void set_attributes() {
   PB_CUDA(cudaFuncSetAttribute(k_col_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                int(kColSmem)));
   PB_CUDA(cudaFuncSetAttribute(k_col_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1993,7 +1991,11 @@ void chol_set_smem_attributes() {
     PB_SWEEP_ATTR(k_chol_fwd, kMaxF);
 #undef PB_SWEEP_ATTR
   }
-  done = true;
+}
+
+void chol_set_smem_attributes() {
+  static OncePerDevice once;
+  once(set_attributes);
 }
 
 void chol_launch_steps(const BigArgs &a, const BigSlot *ds, const std::vector<BigSlot> &hs,

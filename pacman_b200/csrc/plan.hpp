@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -231,6 +232,24 @@ struct Tuning {
   std::string source = "built-in defaults";
 };
 const Tuning &tuning_for_current_device();
+// Runs fn once per device (the current one): kernels' attributes are set for the
+// device that is current.  A thread that comes meanwhile waits.
+class OncePerDevice {
+ public:
+  template <typename Fn> void operator()(Fn &&fn) {
+    int dev = 0;
+    PB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu_);
+    if (dev < 64 && (done_ >> dev & 1)) return;
+    fn();
+    if (dev < 64) done_ |= uint64_t(1) << dev;
+  }
+
+ private:
+  std::mutex mu_;
+  uint64_t done_ = 0;
+};
+
 // The environment variable if set, else the tuned value.
 int tuned_int(const char *env, int value);
 
